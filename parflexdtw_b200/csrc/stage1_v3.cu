@@ -7,15 +7,14 @@
 // 64k+2i+1 (B) and at local step tau computes A = (64k+2i, tau-2i) and
 // B = (64k+2i+1, tau-2i-1): row rho = r mod 64 sits at column tau - rho, and
 // r + c = 64k + tau is the same for every cell of a warp-step.  The
-// predecessors of A are lane i-1's B two steps ago ((1,1)), lane i-1's B
-// three steps ago ((1,2), relayed: what this lane received one step earlier)
-// and lane i-1's A three steps ago ((2,1)); those of B are this lane's own A
-// two and three steps ago and again lane i-1's B three steps ago.  Two
-// shuffles of (D, P) per step feed both cells, which are independent of each
-// other.  mdist = (r + c) - |P| is formed in FP64 (exact: both integers).
+// predecessors of A are lane i-1's B two steps ago ((1,1)) and three steps ago
+// ((1,2): what this lane had one step earlier) and lane i-1's A three steps
+// ago ((2,1)); those of B are this lane's own A two and three steps ago and
+// again lane i-1's B three steps ago.  Lanes pass (D, P) of both rows through
+// shared memory, one entry per lane; lane 31's entry is a slot of its strip's
+// ring and lane 0 reads the previous strip's ring (see Rings).  mdist =
+// (r + c) - |P| is formed in FP64 (exact: both integers).
 //
-// Lane 0 takes rows 64k-2 and 64k-1 (the previous strip's lane 31) from a
-// per-warp shared-memory ring indexed by (strip start + column) mod RB.
 // Strips start `lag` (>= 80) steps apart.  Inside a tile warps do not use CTA
 // barriers: each publishes the global step it has completed (release store by
 // lane 31, the ring writer) and, before a block, waits (acquire, bounded)
@@ -28,17 +27,21 @@
 // (cost slab, output addresses, shape) from a device queue with one atomic
 // per tile, so the tiles of one alignment or of a whole batch of alignments
 // of uneven sizes run in one launch.  Queues are ordered largest tile first.
-// A CTA barrier separates consecutive tiles of a CTA (rings and progress
-// words are reset there).
+// A CTA barrier separates consecutive tiles of a CTA (progress words are
+// reset there).
 //
-// Selection.  Every cell first takes a branch-free, division-free comparison
-// of the three candidates (cross products with a 2^-48 relative margin, see
-// qless_exact); cells too close to call, cells with a predecessor on row 0 /
-// column 0 or outside the tile, and non-finite values go -- one uniform
-// branch per warp-step -- to the exact per-lane routine, which falls back to
-// IEEE division.  Only blocks touching a tile boundary ("edge" blocks) pay
-// for the bounds tests and the edge-row stores.  The cost queue runs two
-// steps ahead.
+// Selection.  Every cell takes a branch-free, division-free comparison of the
+// three candidates (cross products with a 2^-46 relative margin, see
+// decide_quot); cells too close to call and non-finite values go to the exact
+// routine, which falls back to IEEE division.  Blocks inside the tile run a
+// loop that holds nothing else; see run_block.  The cost queue runs two steps
+// ahead.
+//
+// Measured (592 tiles of 2000 x 2000, 4 warps per tile, B200): 6.91 ms = 343
+// Gcells/s, against 9.47 ms = 250 Gcells/s with shuffles, per-lane ring
+// selects, one loop for all blocks and the exact routine inside it.  A fast
+// step costs 52 thread instructions per cell (79 before), 19 of them on the
+// half-rate FP64 pipe; a careful one 112.
 #include <algorithm>
 #include <cooperative_groups.h>
 #include <cuda/atomic>
@@ -103,11 +106,13 @@ __device__ __forceinline__ bool qless_exact(float b, float nd, float a, float md
 }
 
 // Exact selection of one cell with r, c >= 1 (generic steps, any position).
+// Start encodings are the internal ones (see Wave): a boundary predecessor's
+// mdist is r + c, as the reference stores P = 0 there (FlexDTW.py:346-356).
 template <bool STD, bool ALLIN, typename T>
 __device__ __forceinline__ void select_exact(const Geo& g, T w_last, int r, int c, T rc, T cval,
                                           T x1D, int x1P, T x2D, int x2P, T x3D, int x3P, T& oD,
                                           int& oP, int& code) {
-    int bs = -1, bk = 0, bP = 0;
+    int bs = -1, bP = 0;
     T bA = 0, bM = 1;
 #pragma unroll
     for (int s = 0; s < 3; ++s) {
@@ -117,12 +122,12 @@ __device__ __forceinline__ void select_exact(const Geo& g, T w_last, int r, int 
         if (!inb) continue;
         const T pD = kd == 0 ? x1D : (kd == 1 ? x2D : x3D);
         const int pP = kd == 0 ? x1P : (kd == 1 ? x2P : x3P);
+        const bool rim = !ALLIN && (r == (kd == 2 ? 2 : 1) || c == (kd == 1 ? 2 : 1));
         const T a = addr(pD, mulr(cval, (T)g.w[s]));
-        const T md = addr(rc, -fabs((T)pP));
+        const T md = rim ? rc : addr(rc, -fabs((T)pP));
         const bool take = bs < 0 ? a < (T)CUDART_INF : qless_exact(a, md, bA, bM);
         if (take) {
             bs = s;
-            bk = kd;
             bA = a;
             bM = md;
             bP = pP;
@@ -136,131 +141,151 @@ __device__ __forceinline__ void select_exact(const Geo& g, T w_last, int r, int 
     } else {
         oD = bA;
         code = bs;
-        const int pr = r - (bk == 2 ? 2 : 1);
-        const int pcn = c - (bk == 1 ? 2 : 1);
-        oP = pr == 0 ? pcn : (pcn == 0 ? -pr : bP);
+        oP = bP;
     }
 }
 
-// Steps (1,1), (1,2), (2,1): branch-free selection of one cell with r, c >= 1.
+// Division-free decision of "the new candidate's quotient is strictly below
+// the incumbent's", RN(a_new / m_new) < RN(a_inc / m_inc) with positive
+// integer-valued m, for the FP64 form.  Returns whether the cross products
+// decide it (else the caller divides); `win` is the answer when they do.
+//   U = RN(a_new * m_inc), d = RN(a_inc * m_new - U) (one FMA) and the
+//   threshold t = RN(|U| * 2^-46 + 2^-900) (one FMA).  With V the exact
+//   a_inc * m_new, d's error is below 2^-53 |U| + 2^-53 |d| (plus 2^-1074
+//   where a value is subnormal).
+//   * |V| <= 3 |U|: |d| > t > 2^-46 |U| exceeds that error by a factor of 32,
+//     so it fixes the sign of the exact V - a_new m_inc and leaves a relative
+//     gap > 2^-49 between the exact quotients: their roundings cannot meet.
+//   * |V| > 3 |U|: the exact difference has V's sign and |V| / 2 or more of
+//     magnitude, the same conclusion.
+//   |d| > t needs max(|U|, |V|) > 2^-901: no quotient is subnormal.  An
+//   infinite U makes t infinite and a NaN product makes d NaN: neither
+//   decides.  An infinite a_inc against a finite U decides as the reference
+//   does (+inf never becomes the incumbent, -inf is never beaten).
+__device__ __forceinline__ bool decide_quot(double a_new, double m_new, double a_inc,
+                                            double m_inc, bool& win) {
+    const double U = __dmul_rn(a_new, m_inc);
+    const double d = __fma_rn(a_inc, m_new, -U);
+    const double t = __fma_rn(fabs(U), 0x1p-46, 0x1p-900);
+    win = d > 0.0;
+    return fabs(d) > t;
+}
+// FP32 form: the cross products of FP32 values and integers below 2^24 are
+// exact in FP64 (see the FP32 qless_exact): d <= 0 decides "not below", a
+// relative margin of 2^-21 decides "below".  Infinite values never decide.
+__device__ __forceinline__ bool decide_quot(float a_new, float m_new, float a_inc, float m_inc,
+                                            bool& win) {
+    const double U = __dmul_rn((double)a_new, (double)m_inc);
+    const double V = __dmul_rn((double)a_inc, (double)m_new);
+    const double d = __dadd_rn(V, -U);
+    win = d > __dmul_rn(__dadd_rn(fabs(U), fabs(V)), 0x1p-21);
+    return (win || d <= 0.0) && fabs(d) < CUDART_INF;
+}
+
+// Steps (1,1), (1,2), (2,1) at one cell, mdists given: branch-free selection.
 // Returns false when a comparison is too close to call or a value is not
-// finite; the caller then recomputes the cell with select_exact.  EDGE adds
-// the in-bounds tests of (1,2) (c >= 2) and (2,1) (r >= 2) and the start
-// encoding of a predecessor on row 0 / column 0 (FlexDTW.py:365-370).
-template <bool EDGE>
-__device__ __forceinline__ bool select_fast_std(const Geo& g, int r, int c, double rc,
-                                                double cval, double x1D, int x1P, double x2D,
-                                                int x2P, double x3D, int x3P, double& oD,
-                                                int& oP, int& code) {
-    const double a0 = __dadd_rn(x1D, __dmul_rn(cval, g.w[0]));
-    const double a1 = __dadd_rn(x2D, __dmul_rn(cval, g.w[1]));
-    const double a2 = __dadd_rn(x3D, __dmul_rn(cval, g.w[2]));
-    const double m0 = __dadd_rn(rc, -fabs((double)x1P));
-    const double m1 = __dadd_rn(rc, -fabs((double)x2P));
-    const double m2 = __dadd_rn(rc, -fabs((double)x3P));
-    const bool in1 = !EDGE || c >= 2, in2 = !EDGE || r >= 2;
-    const double U1 = __dmul_rn(a1, m0), V1 = __dmul_rn(a0, m1);
-    const double d1 = __dadd_rn(V1, -U1);
-    const double g1 = __dadd_rn(fabs(U1), fabs(V1));
-    const double t1 = __dmul_rn(g1, 0x1p-48);
-    const bool win1 = in1 && d1 > t1;
-    const bool ok1 = !in1 || (g1 >= 0x1p-950 && (d1 > t1 || -d1 > t1));
-    const double bA = win1 ? a1 : a0, bM = win1 ? m1 : m0;
-    const double U2 = __dmul_rn(a2, bM), V2 = __dmul_rn(bA, m2);
-    const double d2 = __dadd_rn(V2, -U2);
-    const double g2 = __dadd_rn(fabs(U2), fabs(V2));
-    const double t2 = __dmul_rn(g2, 0x1p-48);
-    const bool win2 = in2 && d2 > t2;
-    const bool ok2 = !in2 || (g2 >= 0x1p-950 && (d2 > t2 || -d2 > t2));
-    oD = win2 ? a2 : bA;
-    const int inh = win2 ? x3P : (win1 ? x2P : x1P);
-    code = win2 ? 2 : (win1 ? 1 : 0);
-    if (EDGE) {
-        const int pr = r - (win2 ? 2 : 1);
-        const int pcn = c - (win1 && !win2 ? 2 : 1);
-        oP = pr == 0 ? pcn : (pcn == 0 ? -pr : inh);
-    } else {
-        oP = inh;
+// finite; the caller then recomputes the cell with select_exact.  RIM: in1 /
+// in2 say whether the (1,2) / (2,1) predecessor exists (else all do).
+template <bool RIM, typename T>
+__device__ __forceinline__ bool select_std(T cval, T w0, T w1, T w2, T x1D, int x1P, T m0, T x2D,
+                                           int x2P, T m1, bool in1, T x3D, int x3P, T m2, bool in2,
+                                           T& oD, int& oP, int& code) {
+    const T a0 = addr(x1D, mulr(cval, w0));
+    const T a1 = addr(x2D, mulr(cval, w1));
+    const T a2 = addr(x3D, mulr(cval, w2));
+    bool win1, win2;
+    bool ok1 = decide_quot(a1, m1, a0, m0, win1);
+    if (RIM) {
+        win1 = win1 && in1;
+        ok1 = in1 ? ok1 : a0 < (T)CUDART_INF;
     }
-    return a0 < CUDART_INF && ok1 && ok2;
+    const T bA = win1 ? a1 : a0, bM = win1 ? m1 : m0;
+    bool ok2 = decide_quot(a2, m2, bA, bM, win2);
+    if (RIM) {
+        win2 = win2 && in2;
+        ok2 = in2 ? ok2 : bA < (T)CUDART_INF;
+    }
+    oD = win2 ? a2 : bA;
+    oP = win2 ? x3P : (win1 ? x2P : x1P);
+    code = win2 ? 2 : (win1 ? 1 : 0);
+    return ok1 && ok2;
 }
 
-// FP32 form of select_fast_std: FP32 path costs, exact FP64 cross products
-// (see the FP32 qless_exact) for the two comparisons.
-template <bool EDGE>
-__device__ __forceinline__ bool select_fast_std(const Geo& g, int r, int c, float rc, float cval,
-                                                float x1D, int x1P, float x2D, int x2P,
-                                                float x3D, int x3P, float& oD, int& oP,
-                                                int& code) {
-    const float a0 = __fadd_rn(x1D, __fmul_rn(cval, (float)g.w[0]));
-    const float a1 = __fadd_rn(x2D, __fmul_rn(cval, (float)g.w[1]));
-    const float a2 = __fadd_rn(x3D, __fmul_rn(cval, (float)g.w[2]));
-    const float m0 = __fadd_rn(rc, -fabsf((float)x1P));
-    const float m1 = __fadd_rn(rc, -fabsf((float)x2P));
-    const float m2 = __fadd_rn(rc, -fabsf((float)x3P));
-    const bool in1 = !EDGE || c >= 2, in2 = !EDGE || r >= 2;
-    const double U1 = __dmul_rn((double)a1, (double)m0), V1 = __dmul_rn((double)a0, (double)m1);
-    const double d1 = __dadd_rn(V1, -U1);
-    const double t1 = __dmul_rn(__dadd_rn(fabs(U1), fabs(V1)), 0x1p-21);
-    const bool win1 = in1 && d1 > t1;
-    const bool ok1 = !in1 || d1 > t1 || d1 <= 0.0;
-    const float bA = win1 ? a1 : a0, bM = win1 ? m1 : m0;
-    const double U2 = __dmul_rn((double)a2, (double)bM), V2 = __dmul_rn((double)bA, (double)m2);
-    const double d2 = __dadd_rn(V2, -U2);
-    const double t2 = __dmul_rn(__dadd_rn(fabs(U2), fabs(V2)), 0x1p-21);
-    const bool win2 = in2 && d2 > t2;
-    const bool ok2 = !in2 || d2 > t2 || d2 <= 0.0;
-    oD = win2 ? a2 : bA;
-    const int inh = win2 ? x3P : (win1 ? x2P : x1P);
-    code = win2 ? 2 : (win1 ? 1 : 0);
-    if (EDGE) {
-        const int pr = r - (win2 ? 2 : 1);
-        const int pcn = c - (win1 && !win2 ? 2 : 1);
-        oP = pr == 0 ? pcn : (pcn == 0 ? -pr : inh);
-    } else {
-        oP = inh;
-    }
-    return a0 < CUDART_INF_F && a1 < CUDART_INF_F && a2 < CUDART_INF_F && ok1 && ok2;
-}
-
+// A warp's wavefront state between steps.  At the start of step tau: A's
+// outputs 1..3 steps ago, B's output one step ago, the predecessors of this
+// step's A cell -- x1 (1,1), x2 (1,2), x3 (2,1) -- already received, and the
+// mdists of A's and B's (1,2) predecessors.  Start encodings are internal: a
+// cell on row 0 carries its column, one on column 0 minus its row, so that a
+// successor inherits its predecessor's encoding everywhere.
 template <typename T>
 struct Wave {
-    T aD1, aD2, aD3, bD1, bD2, xpD;  // own A outputs 1..3 steps ago, own B 1..2 ago,
-    int aP1, aP2, aP3, bP1, bP2, xpP;  // lane i-1's B received one step ago
+    T aD1, aD2, aD3, bD1, x1D, x2D, x3D, m1A, m1B;
+    int aP1, aP2, aP3, bP1, x1P, x2P, x3P;
     typename Vec2<T>::type q[2];     // cost queue, step tau in slot tau & 1
 };
 
-// Per-warp rings of a strip's last two rows, [NW][RB] slots.  Slot s of a
-// ring holds row 64k+63 ("B") at the strip's local step s+63 and row 64k+62
-// ("A") at step s+62, the pair the next strip's lane 0 reads at once: D as
-// one {B, A} vector and the start encodings as one {B, A} int2, so a read is
-// two shared-memory loads and a write two stores (lane 31 writes A one step
-// late, together with B).
+// Per-warp rings of a strip's last two rows, [NW][RB] slots, RB a multiple
+// of kBlk, and per-warp exchange entries, [NW][kXch].  At the start of its
+// step T (counted from the tile's start) every lane stores the pair {B one
+// step ago, A two steps ago} and loads its neighbour lane i-1's, which the
+// next step uses as x1 and x3.  Lanes 0..30 store into their exchange entry;
+// lane 31 stores into ring slot (T - 64) mod RB, which then holds rows 64k+63
+// and 64k+62 of column j = tau - 64; lane 0 loads ring slot (T' - lag) mod RB
+// of the previous strip, its column tau'.  So one address per lane takes the
+// place of shuffles, of the ring's own loads and stores and of the selects
+// between the two.  Both ring windows of a block start on a multiple of
+// kBlk: no address inside a block wraps.  D is one {B, A} vector, the start
+// encodings one {B, A} int2.
 template <typename T>
 struct Rings {
-    typename Vec2<T>::type* D;  // {D of row 64k+63, D of row 64k+62}
-    int2* P;                    // {P of row 64k+63, P of row 64k+62}
+    typename Vec2<T>::type *D, *xD;
+    int2 *P, *xP;
 };
+constexpr int kXch = 34;  // 32 lanes, shifted by one entry in odd steps, and one spare
 template <typename T>
 __host__ __device__ constexpr int ring_slot_bytes() {
     return (int)(sizeof(typename Vec2<T>::type) + sizeof(int2));
 }
-
-// rg: the CTA's rings.  A warp reads its producer's ring at rbase and
-// writes its own at wbase, both with rg's layout: rg.D itself, or in a
-// cluster the generic address of the other CTA's rings.  A slot is accessed
-// at base + its byte offset in rg, so that the address derives from the base
-// alone.  bw (when non-null) receives the block's backpointer word instead of
-// the store to td.Bw.
-template <typename X, typename T>
-__device__ __forceinline__ X ring_at(const char* rbase, const Rings<T>& rg, const X* p) {
-    return *reinterpret_cast<const X*>(
-        rbase + (reinterpret_cast<const char*>(p) - reinterpret_cast<const char*>(rg.D)));
+// Shared memory of nw warps' rings and exchange entries, and n progress words.
+template <typename T>
+__host__ __device__ constexpr size_t ring_bytes(int nw, int rb, int n) {
+    return (size_t)nw * (rb + kXch) * ring_slot_bytes<T>() + n * sizeof(int);
 }
-template <typename X, typename T>
-__device__ __forceinline__ void ring_put(char* wbase, const Rings<T>& rg, const X* p, X v) {
-    *reinterpret_cast<X*>(wbase + (reinterpret_cast<const char*>(p) -
-                                   reinterpret_cast<const char*>(rg.D))) = v;
+template <typename T>
+__device__ __forceinline__ Rings<T> ring_layout(unsigned char* smem, int nw, int rb) {
+    using V2 = typename Vec2<T>::type;
+    Rings<T> r;
+    r.D = reinterpret_cast<V2*>(smem);
+    r.xD = r.D + nw * rb;
+    r.P = reinterpret_cast<int2*>(r.xD + nw * kXch);
+    r.xP = r.P + nw * rb;
+    return r;
+}
+__device__ __forceinline__ void st_pair(uint32_t aD, uint32_t aP, double b, double a, int pb,
+                                        int pa) {
+    asm volatile("st.shared.v2.f64 [%0], {%1, %2};\nst.shared.v2.s32 [%3], {%4, %5};" ::"r"(aD),
+                 "d"(b), "d"(a), "r"(aP), "r"(pb), "r"(pa)
+                 : "memory");
+}
+__device__ __forceinline__ void st_pair(uint32_t aD, uint32_t aP, float b, float a, int pb,
+                                        int pa) {
+    asm volatile("st.shared.v2.f32 [%0], {%1, %2};\nst.shared.v2.s32 [%3], {%4, %5};" ::"r"(aD),
+                 "f"(b), "f"(a), "r"(aP), "r"(pb), "r"(pa)
+                 : "memory");
+}
+__device__ __forceinline__ void ld_pair(uint32_t aD, uint32_t aP, double& b, double& a, int& pb,
+                                        int& pa) {
+    asm volatile("ld.shared.v2.f64 {%0, %1}, [%4];\nld.shared.v2.s32 {%2, %3}, [%5];"
+                 : "=d"(b), "=d"(a), "=r"(pb), "=r"(pa)
+                 : "r"(aD), "r"(aP)
+                 : "memory");
+}
+__device__ __forceinline__ void ld_pair(uint32_t aD, uint32_t aP, float& b, float& a, int& pb,
+                                        int& pa) {
+    asm volatile("ld.shared.v2.f32 {%0, %1}, [%4];\nld.shared.v2.s32 {%2, %3}, [%5];"
+                 : "=f"(b), "=f"(a), "=r"(pb), "=r"(pa)
+                 : "r"(aD), "r"(aP)
+                 : "memory");
 }
 template <typename T>
 __device__ __forceinline__ typename Vec2<T>::type make_v2(T x, T y) {
@@ -270,361 +295,305 @@ __device__ __forceinline__ typename Vec2<T>::type make_v2(T x, T y) {
     return v;
 }
 
-// PUSH: the ring is written at wbase (generic address, a cluster peer's
-// shared memory possibly); otherwise straight into this CTA's rings.
-template <bool EDGE, bool STD, bool PUSH, typename T>
-__device__ __forceinline__ void run_block(const Geo& g, Wave<T>& st, const Rings<T>& rg,
-                                          const char* rbase, char* wbase,
-                                          const typename Vec2<T>::type* __restrict__ Cs,
-                                          int span, int tau0, int k, int R, int W, int lane,
-                                          int prev_base, int mine_base, int rmask, int Tb,
-                                          int lag, const TileDesc& td, int nP,
-                                          uint2* bw = nullptr) {
-    using V2 = typename Vec2<T>::type;
-    const unsigned F = 0xffffffffu;
-    const T w_last = (T)(g.S == 1 ? g.w[0] : (g.S == 2 ? g.w[1] : g.w[2]));
-    const int rA = 64 * k + 2 * lane, rB = rA + 1;
-    uint32_t bitsA = 0, bitsB = 0;
-    const T rc0 = (T)(64 * k + tau0);
-#pragma unroll 1
-    for (int tq = 0; tq < kBlk; tq += 2) {
-#pragma unroll
-        for (int u = 0; u < 2; ++u) {
-            const int t = tq + u;
-            const int tau = tau0 + t;
-            const T rc = addr(rc0, (T)t);
-            const V2 cc = st.q[u & 1];
-            if (tau + 2 < span) st.q[u & 1] = __ldcs(Cs + (int64_t)(tau + 2) * 32);
-            T x1D = __shfl_up_sync(F, st.bD2, 1);
-            int x1P = __shfl_up_sync(F, st.bP2, 1);
-            T x3D = __shfl_up_sync(F, st.aD3, 1);
-            int x3P = __shfl_up_sync(F, st.aP3, 1);
-            {
-                // every lane reads the same slot (a broadcast); lane 0 keeps it
-                const int rs = prev_base + ((Tb + t - lag - 1) & rmask);
-                const V2 rD = ring_at(rbase, rg, rg.D + rs);
-                const int2 rP = ring_at(rbase, rg, rg.P + rs);
-                if (lane == 0) {
-                    x1D = rD.x;
-                    x1P = rP.x;
-                    x3D = rD.y;
-                    x3P = rP.y;
-                }
-            }
-            const T x2D = st.xpD;
-            const int x2P = st.xpP;
-            const int cA = tau - 2 * lane, cB = cA - 1;
-            T oAD, oBD;
-            int oAP, oBP, codeA, codeB;
-            bool actA = true, actB = true;
-            bool okA, okB;
-            if (STD) {
-                okA = select_fast_std<EDGE>(g, rA, cA, rc, cc.x, x1D, x1P, x2D, x2P, x3D, x3P, oAD,
-                                            oAP, codeA);
-                okB = select_fast_std<EDGE>(g, rB, cB, rc, cc.y, st.aD2, st.aP2, st.aD3, st.aP3,
-                                            x2D, x2P, oBD, oBP, codeB);
-            } else {
-                okA = okB = false;
-            }
-            if (EDGE) {
-                actA = rA < R && cA >= 0 && cA < W;
-                actB = rB < R && cB >= 0 && cB < W;
-                // boundary cells are set below; absent cells are zeroed
-                okA = !actA || rA == 0 || cA == 0 || okA;
-                okB = !actB || cB == 0 || okB;
-            }
-            if (__any_sync(F, !(okA && okB))) {
-                if (!okA) {
-                    if (rA == 0 || cA == 0) {
-                        oAD = cc.x; oAP = 0; codeA = 0;
-                    } else {
-                        select_exact<STD, !EDGE>(g, w_last, rA, cA, rc, cc.x, x1D, x1P, x2D, x2P,
-                                                 x3D, x3P, oAD, oAP, codeA);
-                    }
-                }
-                if (!okB) {
-                    if (cB == 0) {
-                        oBD = cc.y; oBP = 0; codeB = 0;
-                    } else {
-                        select_exact<STD, !EDGE>(g, w_last, rB, cB, rc, cc.y, st.aD2, st.aP2,
-                                                 st.aD3, st.aP3, x2D, x2P, oBD, oBP, codeB);
-                    }
-                }
-            }
-            if (EDGE) {
-                double* eD = td.eD;
-                int32_t* eP = td.eP;
-                if (actA && (rA == 0 || cA == 0)) { oAD = cc.x; oAP = 0; codeA = 0; }
-                if (actB && cB == 0) { oBD = cc.y; oBP = 0; codeB = 0; }
-                if (!actA) { oAD = 0; oAP = 0; codeA = 0; }
-                if (!actB) { oBD = 0; oBP = 0; codeB = 0; }
-                // edges are FP64 for stage 2 (exact widening in the FP32 form)
-                if (actA && rA == R - 1) { eD[cA] = (double)oAD; eP[cA] = oAP; }
-                if (actB && rB == R - 1) { eD[cB] = (double)oBD; eP[cB] = oBP; }
-                if (actA && cA == W - 1) { eD[td.L + rA] = (double)oAD; eP[td.L + rA] = oAP; }
-                if (actB && cB == W - 1) { eD[td.L + rB] = (double)oBD; eP[td.L + rB] = oBP; }
-            }
-            if (lane == 31 && actB) {
-                // B of this step and A of the previous one (the same column,
-                // active whenever B is): slot (step - 63)
-                const int ws = mine_base + ((Tb + t - 63) & rmask);
-                if (PUSH) {
-                    ring_put(wbase, rg, rg.D + ws, make_v2<T>(oBD, st.aD1));
-                    ring_put(wbase, rg, rg.P + ws, make_int2(oBP, st.aP1));
-                } else {
-                    rg.D[ws] = make_v2<T>(oBD, st.aD1);
-                    rg.P[ws] = make_int2(oBP, st.aP1);
-                }
-            }
-            bitsA |= (uint32_t)codeA << (2 * t);
-            bitsB |= (uint32_t)codeB << (2 * t);
-            st.aD3 = st.aD2; st.aP3 = st.aP2;
-            st.aD2 = st.aD1; st.aP2 = st.aP1;
-            st.aD1 = oAD;    st.aP1 = oAP;
-            st.bD2 = st.bD1; st.bP2 = st.bP1;
-            st.bD1 = oBD;    st.bP1 = oBP;
-            st.xpD = x1D;    st.xpP = x1P;
-        }
-    }
-    if (bw) {
-        *bw = make_uint2(bitsA, bitsB);
-    } else if (rA < R) {
-        uint2* Bt = reinterpret_cast<uint2*>(td.Bw);
-        Bt[((int64_t)k * nP + (tau0 >> 4)) * 32 + lane] = make_uint2(bitsA, bitsB);
-    }
-}
-
-// Division-free decision of "the new candidate's quotient is strictly below
-// the incumbent's", RN(a_new / m_new) < RN(a_inc / m_inc) with positive
-// integer-valued m, for the FP64 form.  Returns whether the cross products
-// decide it (else the caller divides); `win` is the answer when they do.
-//   U = RN(a_new * m_inc), V = RN(a_inc * m_new), d = RN(V - U) and the
-//   threshold t = RN(|U| * 2^-46 + 2^-900) (one FMA).  d's error is below
-//   2^-52 (|U| + |V|) (plus 2^-1073 where a product is subnormal).
-//   * |V| <= 3 |U|: t >= 2^-48 (|U| + |V|) + 2^-900 exceeds that error by a
-//     factor of 16, so |d| > t fixes the sign of the exact a_inc m_new -
-//     a_new m_inc and leaves a relative gap > 2^-49 between the exact
-//     quotients: their roundings cannot meet.
-//   * |V| > 3 |U|: the exact difference has V's sign and |V| / 2 or more of
-//     magnitude, the same conclusion.
-//   |d| > t needs max(|U|, |V|) > 2^-901: no quotient is subnormal.  A NaN
-//   or infinite product never decides (every comparison with it is false or
-//   t is infinite).
-__device__ __forceinline__ bool decide_quot(double a_new, double m_new, double a_inc,
-                                            double m_inc, bool& win) {
-    const double U = __dmul_rn(a_new, m_inc);
-    const double V = __dmul_rn(a_inc, m_new);
-    const double d = __dadd_rn(V, -U);
-    const double t = __fma_rn(fabs(U), 0x1p-46, 0x1p-900);
-    win = d > t;
-    return win || -d > t;
-}
-// FP32 form: the cross products of FP32 values and integers below 2^24 are
-// exact in FP64 (see the FP32 qless_exact): d <= 0 decides "not below", a
-// relative margin of 2^-21 decides "below".
-__device__ __forceinline__ bool decide_quot(float a_new, float m_new, float a_inc, float m_inc,
-                                            bool& win) {
-    const double U = __dmul_rn((double)a_new, (double)m_inc);
-    const double V = __dmul_rn((double)a_inc, (double)m_new);
-    const double d = __dadd_rn(V, -U);
-    win = d > __dmul_rn(__dadd_rn(fabs(U), fabs(V)), 0x1p-21);
-    return win || d <= 0.0;
-}
-__device__ __forceinline__ bool finite_first(double a0, double, double) { return a0 < CUDART_INF; }
-__device__ __forceinline__ bool finite_first(float a0, float a1, float a2) {
-    return a0 < CUDART_INF_F && a1 < CUDART_INF_F && a2 < CUDART_INF_F;
-}
-
-// Steps (1,1), (1,2), (2,1) at a cell with every predecessor inside the tile
-// and r, c >= 2, mdists given: the selection of select_fast_std<false>.
+// What a block needs besides the wave state.
 template <typename T>
-__device__ __forceinline__ bool select_std_m(T cval, T w0, T w1, T w2, T x1D, int x1P, T m0,
-                                             T x2D, int x2P, T m1, T x3D, int x3P, T m2, T& oD,
-                                             int& oP, int& code) {
-    const T a0 = addr(x1D, mulr(cval, w0));
-    const T a1 = addr(x2D, mulr(cval, w1));
-    const T a2 = addr(x3D, mulr(cval, w2));
-    bool win1, win2;
-    const bool ok1 = decide_quot(a1, m1, a0, m0, win1);
-    const T bA = win1 ? a1 : a0, bM = win1 ? m1 : m0;
-    const bool ok2 = decide_quot(a2, m2, bA, bM, win2);
-    oD = win2 ? a2 : bA;
-    oP = win2 ? x3P : (win1 ? x2P : x1P);
-    code = win2 ? 2 : (win1 ? 1 : 0);
-    return finite_first(a0, a1, a2) && ok1 && ok2;
-}
-
-// Exact selection of the fast block's undecided cells (rare), by value.
-template <typename T>
-struct SelOut {
-    T d;
-    int p, code;
+struct Block {
+    const typename Vec2<T>::type* Cs;  // the strip's cost, at this lane
+    uint32_t w, r;                     // this lane's store and load addresses (P; the
+    uint32_t kd;                       // D address is that times 2 (FP32 form: 1), + kd)
+    typename Vec2<T>::type* pD;        // PUSH: the ring slot in a cluster peer's
+    int2* pP;                          // shared memory, or null
+    uint32_t incW, incR;               // and their moves per two steps (ring lanes)
+    int span, tau0, k, R, W, lane, nP;
 };
+
+// Edge values of a cell on the tile's last row / last column; FP64 for stage
+// 2 (exact widening in the FP32 form), P = 0 on row 0 and column 0.
 template <typename T>
-__device__ __forceinline__ SelOut<T> select_exact_std_call(T w0, T w1, T w2, int r, int c, T rc,
-                                                        T cval, T x1D, int x1P, T x2D, int x2P,
-                                                        T x3D, int x3P) {
-    Geo g;
-    g.S = 3;
-    g.kind[0] = 0;
-    g.kind[1] = 1;
-    g.kind[2] = 2;
-    g.w[0] = (double)w0;
-    g.w[1] = (double)w1;
-    g.w[2] = (double)w2;
-    SelOut<T> o;
-    select_exact<true, true>(g, w2, r, c, rc, cval, x1D, x1P, x2D, x2P, x3D, x3P, o.d, o.p,
-                             o.code);
-    return o;
+__device__ __forceinline__ void store_edges(const TileDesc& td, int r, int c, int R, int W, T D,
+                                            int P) {
+    const int p = (r == 0 || c == 0) ? 0 : P;
+    if (r == R - 1) {
+        td.eD[c] = (double)D;
+        td.eP[c] = p;
+    }
+    if (c == W - 1) {
+        td.eD[td.L + r] = (double)D;
+        td.eP[td.L + r] = p;
+    }
 }
 
-// A block of 16 steps of the standard step set in which every cell of the
-// strip is inside the tile with r, c >= 2 and off the tile's last row and
-// column (the caller's "interior" test).  Same results as
-// run_block<false, true, PUSH, T>, with fewer instructions per step:
-//  * no bounds tests, no edge stores, and no guard on the cost loads (the
-//    block ends at least 17 steps before the strip's span);
-//  * mdist of a predecessor that the previous step also used is that step's
-//    mdist + 1 (r + c grows by one per step), and B's (2,1) predecessor is
-//    A's (1,2) one, so a step converts three start encodings, not six;
-//  * ring slots are read and written as {B, A} pairs (two shared-memory
-//    loads per step, two stores by lane 31);
-//  * the FP64 decision margin is one FMA (decide_quot).
-// The loop is unrolled two steps deep only: steps t and t+1 are independent
-// (each reads outputs of two steps back), and a small loop body stays in the
-// instruction cache (a 16-step unroll, or a second copy of the body, each
-// measured slower).
-//
-// MASK (a run-time flag, so that one copy of the loop body serves both: a
-// second inlined copy measured slower): the same path for a block of strip
-// k >= 1 at tau0 >= 80 (every cell at r >= 64, c >= 18, so every
-// predecessor of a cell inside the tile is inside too) that reaches the
-// tile's last column or its last row, or lies partly outside the tile (the
-// right end of a strip, the last strip): cells outside the tile (r >= R or
-// c >= W) are set to 0 and never call for the exact routine, cells on the
-// last row / column store their edge values, and the cost loads stop at the
-// strip's span.  Same results as run_block<true, true, PUSH, T>.
+// The step's outputs enter the wave.
+template <typename T>
+__device__ __forceinline__ void advance(Wave<T>& st, T oAD, int oAP, T oBD, int oBP, T x1n,
+                                        int p1n, T x3n, int p3n) {
+    st.aD3 = st.aD2; st.aP3 = st.aP2;
+    st.aD2 = st.aD1; st.aP2 = st.aP1;
+    st.aD1 = oAD;    st.aP1 = oAP;
+    st.bD1 = oBD;    st.bP1 = oBP;
+    st.x2D = st.x1D; st.x2P = st.x1P;
+    st.x1D = x1n;    st.x1P = p1n;
+    st.x3D = x3n;    st.x3P = p3n;
+}
+
+// Shared address of the D pair that belongs to the P pair at p.
+template <typename T>
+__device__ __forceinline__ uint32_t d_address(uint32_t p, uint32_t kd) {
+    return p * (2 * (uint32_t)sizeof(T) / (uint32_t)sizeof(int2)) + kd;
+}
+
+// One step of the fast loop: standard steps, every cell of the strip inside
+// the tile with r >= 64, c >= 18 and off its last row and column.  Returns
+// false, with the wave unchanged, when some lane's cell needs the exact
+// routine.  u: the step's parity.
 template <bool PUSH, typename T>
-__device__ __forceinline__ void run_block_std(const Geo& g, Wave<T>& st, const Rings<T>& rg,
-                                              char* wbase,
-                                              const typename Vec2<T>::type* __restrict__ Cs,
-                                              int tau0, int k, int lane, int prev_base,
-                                              int mine_base, int rmask, int Tb, int lag,
-                                              const TileDesc& td, int nP, uint2* bw,
-                                              const bool MASK, int R, int W, int span) {
-    using V2 = typename Vec2<T>::type;
+__device__ __forceinline__ bool fast_step(Wave<T>& st, const int u, T rc, T w0, T w1, T w2,
+                                          uint32_t w, uint32_t r, uint32_t kd,
+                                          typename Vec2<T>::type* pD, int2* pP, int lane,
+                                          uint32_t& bitsA, uint32_t& bitsB) {
+    constexpr int SD = 2 * (int)sizeof(T), SP = (int)sizeof(int2);
+    const typename Vec2<T>::type cc = st.q[u];
+    T x1n, x3n;
+    int p1n, p3n;
+    st_pair(d_address<T>(w, kd) + u * SD, w + u * SP, st.bD1, st.aD2, st.bP1, st.aP2);
+    if (PUSH && pD && lane == 31) {
+        pD[u] = make_v2<T>(st.bD1, st.aD2);
+        pP[u] = make_int2(st.bP1, st.aP2);
+    }
+    __syncwarp();
+    ld_pair(d_address<T>(r, kd) + u * SD, r + u * SP, x1n, x3n, p1n, p3n);
+    const T m0A = addr(rc, -fabs((T)st.x1P));
+    const T m2A = addr(rc, -fabs((T)st.x3P));
+    const T m0B = addr(rc, -fabs((T)st.aP2));
+    T oAD, oBD;
+    int oAP, oBP, codeA, codeB;
+    const bool okA = select_std<false, T>(cc.x, w0, w1, w2, st.x1D, st.x1P, m0A, st.x2D, st.x2P,
+                                          st.m1A, true, st.x3D, st.x3P, m2A, true, oAD, oAP,
+                                          codeA);
+    const bool okB = select_std<false, T>(cc.y, w0, w1, w2, st.aD2, st.aP2, m0B, st.aD3, st.aP3,
+                                          st.m1B, true, st.x2D, st.x2P, st.m1A, true, oBD, oBP,
+                                          codeB);
+    if (!__all_sync(0xffffffffu, okA && okB)) return false;
+    bitsA = bitsA * 4 + codeA;  // the first step ends up highest
+    bitsB = bitsB * 4 + codeB;
+    st.m1A = addr(m0A, (T)1);
+    st.m1B = addr(m0B, (T)1);
+    advance(st, oAD, oAP, oBD, oBP, x1n, p1n, x3n, p3n);
+    return true;
+}
+
+// One step of the careful loop (see run_block).  rim: cells on row 0 / column
+// 0 or next to them may occur; mask: cells past the last row / column or on
+// it.  Outputs of cells outside the tile are arbitrary (nothing inside reads
+// them) but for their code, 0.
+template <bool STD, bool PUSH, typename T>
+__device__ __forceinline__ void careful_step(const Geo& g, Wave<T>& st, const Block<T>& b,
+                                             const TileDesc& td, const int u, int t,
+                                             const bool rim, const bool mask, T rc,
+                                             const typename Vec2<T>::type cc, uint32_t& bitsA,
+                                             uint32_t& bitsB) {
+    constexpr int SD = 2 * (int)sizeof(T), SP = (int)sizeof(int2);
     const unsigned F = 0xffffffffu;
     const T w0 = (T)g.w[0], w1 = (T)g.w[1], w2 = (T)g.w[2];
-    const int rA = 64 * k + 2 * lane, rB = rA + 1;
-    const T rc0 = (T)(64 * k + tau0);
-    // mdist of A's and B's (1,2) predecessors at the next step
-    T m1A_next = addr(rc0, -fabs((T)st.xpP));
-    T m1B_next = addr(rc0, -fabs((T)st.aP3));
-    uint32_t bitsA = 0, bitsB = 0;
-    const V2* cp = Cs + (int64_t)(tau0 + 2) * 32;  // the cost two steps ahead
-    const V2* rD = rg.D + prev_base;
-    const int2* rP = rg.P + prev_base;
-    const int rs0 = Tb - lag - 1;
+    const int lane = b.lane;
+    const int rA = 64 * b.k + 2 * lane, rB = rA + 1;
+    const int cA = b.tau0 + t - 2 * lane, cB = cA - 1;
+    T x1n, x3n;
+    int p1n, p3n;
+    st_pair(d_address<T>(b.w, b.kd) + u * SD, b.w + u * SP, st.bD1, st.aD2, st.bP1, st.aP2);
+    if (PUSH && b.pD && lane == 31) {
+        b.pD[u] = make_v2<T>(st.bD1, st.aD2);
+        b.pP[u] = make_int2(st.bP1, st.aP2);
+    }
+    __syncwarp();
+    ld_pair(d_address<T>(b.r, b.kd) + u * SD, b.r + u * SP, x1n, x3n, p1n, p3n);
+    T m0A = addr(rc, -fabs((T)st.x1P));
+    T m2A = addr(rc, -fabs((T)st.x3P));
+    T m0B = addr(rc, -fabs((T)st.aP2));
+    if (rim) {
+        // predecessors on row 0 / column 0 (for (1,2) the sum carried over
+        // from the previous step already is r + c)
+        if (cA == 1) m0A = rc;
+        if (cA == 1 || rA == 2) m2A = rc;
+        if (cB == 1 || rB == 1) m0B = rc;
+    }
+    T oAD, oBD;
+    int oAP, oBP, codeA, codeB;
+    bool okA = false, okB = false;
+    if (STD) {
+        okA = select_std<true, T>(cc.x, w0, w1, w2, st.x1D, st.x1P, m0A, st.x2D, st.x2P, st.m1A,
+                                  cA >= 2, st.x3D, st.x3P, m2A, true, oAD, oAP, codeA);
+        okB = select_std<true, T>(cc.y, w0, w1, w2, st.aD2, st.aP2, m0B, st.aD3, st.aP3, st.m1B,
+                                  cB >= 2, st.x2D, st.x2P, st.m1A, rB >= 2, oBD, oBP, codeB);
+    }
+    const bool actA = rA < b.R && cA >= 0 && cA < b.W;
+    const bool actB = rB < b.R && cB >= 0 && cB < b.W;
+    const bool rimA = rA == 0 || cA == 0, rimB = cB == 0;
+    okA = okA || !actA || rimA;
+    okB = okB || !actB || rimB;
+    if (__any_sync(F, !(okA && okB))) {
+        const T w_last = (T)(g.S == 1 ? g.w[0] : (g.S == 2 ? g.w[1] : g.w[2]));
+        if (!okA)
+            select_exact<STD, false>(g, w_last, rA, cA, rc, cc.x, st.x1D, st.x1P, st.x2D, st.x2P,
+                                     st.x3D, st.x3P, oAD, oAP, codeA);
+        if (!okB)
+            select_exact<STD, false>(g, w_last, rB, cB, rc, cc.y, st.aD2, st.aP2, st.aD3, st.aP3,
+                                     st.x2D, st.x2P, oBD, oBP, codeB);
+    }
+    if (rim) {
+        if (rimA) { oAD = cc.x; oAP = rA == 0 ? cA : -rA; codeA = 0; }
+        if (rimB) { oBD = cc.y; oBP = -rB; codeB = 0; }
+    }
+    if (mask) {
+        if (actA) store_edges(td, rA, cA, b.R, b.W, oAD, oAP);
+        if (actB) store_edges(td, rB, cB, b.R, b.W, oBD, oBP);
+    }
+    bitsA = bitsA * 4 + (actA ? codeA : 0);
+    bitsB = bitsB * 4 + (actB ? codeB : 0);
+    st.m1A = addr(m0A, (T)1);
+    st.m1B = addr(m0B, (T)1);
+    advance(st, oAD, oAP, oBD, oBP, x1n, p1n, x3n, p3n);
+}
+
+// The careful loop: steps t .. 15 of a block.
+template <bool STD, bool PUSH, typename T>
+__device__ __forceinline__ void careful_steps(const Geo& g, Wave<T>& st, Block<T>& b,
+                                              const TileDesc& td, int t, const bool rim,
+                                              const bool mask, T rc,
+                                              const typename Vec2<T>::type* cp, int ahead,
+                                              uint32_t& bitsA, uint32_t& bitsB) {
+    using V2 = typename Vec2<T>::type;
+    // the cost queue in step order
+    V2 q0 = st.q[0], q1 = st.q[1];
+    if (t & 1) {
+        const V2 s = q0;
+        q0 = q1;
+        q1 = s;
+        cp += 32;
+    }
 #pragma unroll 1
-    for (int tq = 0; tq < kBlk; tq += 2) {
-        const T rcq = addr(rc0, (T)tq);
-#pragma unroll
-        for (int u = 0; u < 2; ++u) {
-            const int t = tq + u;
-            const T rc = addr(rcq, (T)u);
-            const V2 cc = st.q[u & 1];
-            if (!MASK || tau0 + t + 2 < span) st.q[u & 1] = __ldcs(cp + (int64_t)t * 32);
-            const int rs = (rs0 + t) & rmask;
-            const V2 ringD = rD[rs];  // every lane reads the same slot; lane 0 keeps it
-            const int2 ringP = rP[rs];
-            T x1D = __shfl_up_sync(F, st.bD2, 1);
-            int x1P = __shfl_up_sync(F, st.bP2, 1);
-            T x3D = __shfl_up_sync(F, st.aD3, 1);
-            int x3P = __shfl_up_sync(F, st.aP3, 1);
-            x1D = lane == 0 ? ringD.x : x1D;
-            x1P = lane == 0 ? ringP.x : x1P;
-            x3D = lane == 0 ? ringD.y : x3D;
-            x3P = lane == 0 ? ringP.y : x3P;
-            const T x2D = st.xpD;
-            const int x2P = st.xpP;
-            const T m0A = addr(rc, -fabs((T)x1P));
-            const T m1A = m1A_next;
-            const T m2A = addr(rc, -fabs((T)x3P));
-            const T m0B = addr(rc, -fabs((T)st.aP2));
-            const T m1B = m1B_next;
-            m1A_next = addr(m0A, (T)1);
-            m1B_next = addr(m0B, (T)1);
-            T oAD, oBD;
-            int oAP, oBP, codeA, codeB;
-            bool okA = select_std_m<T>(cc.x, w0, w1, w2, x1D, x1P, m0A, x2D, x2P, m1A, x3D,
-                                       x3P, m2A, oAD, oAP, codeA);
-            bool okB = select_std_m<T>(cc.y, w0, w1, w2, st.aD2, st.aP2, m0B, st.aD3, st.aP3,
-                                       m1B, x2D, x2P, m1A, oBD, oBP, codeB);
-            bool actA = true, actB = true;
-            if (MASK) {
-                const int cA = tau0 + t - 2 * lane;
-                actA = rA < R && cA < W;
-                actB = rB < R && cA - 1 < W;
-                okA = okA || !actA;
-                okB = okB || !actB;
+    for (; t < kBlk; ++t) {
+        const V2 cc = q0;
+        q0 = q1;
+        if (t < ahead) q1 = __ldcs(cp);
+        cp += 32;
+        careful_step<STD, PUSH, T>(g, st, b, td, t & 1, t, rim, mask, rc, cc, bitsA, bitsB);
+        rc = addr(rc, (T)1);
+        if (t & 1) {
+            b.w += b.incW;
+            b.r += b.incR;
+            if (PUSH && b.pD) {
+                b.pD += 2;
+                b.pP += 2;
             }
-            if (__any_sync(F, !(okA && okB))) {
-                const int cA = tau0 + t - 2 * lane;
-                if (!okA) {
-                    const SelOut<T> o = select_exact_std_call<T>(w0, w1, w2, rA, cA, rc, cc.x,
-                                                                 x1D, x1P, x2D, x2P, x3D, x3P);
-                    oAD = o.d;
-                    oAP = o.p;
-                    codeA = o.code;
-                }
-                if (!okB) {
-                    const SelOut<T> o = select_exact_std_call<T>(w0, w1, w2, rB, cA - 1, rc,
-                                                                 cc.y, st.aD2, st.aP2, st.aD3,
-                                                                 st.aP3, x2D, x2P);
-                    oBD = o.d;
-                    oBP = o.p;
-                    codeB = o.code;
-                }
-            }
-            if (MASK) {
-                const int cA = tau0 + t - 2 * lane, cB = cA - 1;
-                if (!actA) { oAD = 0; oAP = 0; codeA = 0; }
-                if (!actB) { oBD = 0; oBP = 0; codeB = 0; }
-                // edges are FP64 for stage 2 (exact widening in the FP32 form)
-                double* eD = td.eD;
-                int32_t* eP = td.eP;
-                if (actA && rA == R - 1) { eD[cA] = (double)oAD; eP[cA] = oAP; }
-                if (actB && rB == R - 1) { eD[cB] = (double)oBD; eP[cB] = oBP; }
-                if (actA && cA == W - 1) { eD[td.L + rA] = (double)oAD; eP[td.L + rA] = oAP; }
-                if (actB && cB == W - 1) { eD[td.L + rB] = (double)oBD; eP[td.L + rB] = oBP; }
-            }
-            if (lane == 31 && actB) {
-                // B of this step and A of the previous one: slot (step - 63)
-                const int ws = mine_base + ((Tb + t - 63) & rmask);
-                if (PUSH) {
-                    ring_put(wbase, rg, rg.D + ws, make_v2<T>(oBD, st.aD1));
-                    ring_put(wbase, rg, rg.P + ws, make_int2(oBP, st.aP1));
-                } else {
-                    rg.D[ws] = make_v2<T>(oBD, st.aD1);
-                    rg.P[ws] = make_int2(oBP, st.aP1);
-                }
-            }
-            bitsA |= (uint32_t)codeA << (2 * t);
-            bitsB |= (uint32_t)codeB << (2 * t);
-            st.aD3 = st.aD2; st.aP3 = st.aP2;
-            st.aD2 = st.aD1; st.aP2 = st.aP1;
-            st.aD1 = oAD;    st.aP1 = oAP;
-            st.bD2 = st.bD1; st.bP2 = st.bP1;
-            st.bD1 = oBD;    st.bP1 = oBP;
-            st.xpD = x1D;    st.xpP = x1P;
         }
     }
+    st.q[0] = q0;  // kBlk is even: the next block's step 0
+    st.q[1] = q1;
+}
+
+// One block of 16 steps of a strip, in two loops.
+//
+// The fast loop (standard steps, neither `rim` nor `mask`: every cell of the
+// block inside the tile with r >= 64, c >= 18 and off its last row and column)
+// has no bounds tests, no divisions and one branch per step, out of the loop
+// when some cell is too close to call.  The careful loop does the rest: the
+// remaining steps of such a block, and whole blocks of strip 0 or of the first
+// five of a strip (`rim`), or that reach the tile's last row or column or past
+// them (`mask`).  There cells on row 0 / column 0, predecessors on them (mdist
+// r + c) or missing are handled by selects around the same selection, and
+// undecided cells -- with other step sets than the standard one, all cells --
+// take the exact routine.
+//
+// What bounds it: warp instructions issued, then the FP64 pipe (half rate), so
+// the step is written for few of both.  mdist of a predecessor that the
+// previous step also used is that step's mdist + 1 (r + c grows by one per
+// step) and B's (2,1) predecessor is A's (1,2) one, so a step converts three
+// start encodings; lanes exchange their rows through shared memory (see
+// Rings).  The fast loop is unrolled two steps deep only and holds no rare
+// code: its size decides how well it is fetched.
+template <bool STD, bool PUSH, typename T>
+__device__ __forceinline__ void run_block(const Geo& g, Wave<T>& st, Block<T>& b,
+                                          const TileDesc& td, const bool rim, const bool mask,
+                                          uint2* bw) {
+    using V2 = typename Vec2<T>::type;
+    const T w0 = (T)g.w[0], w1 = (T)g.w[1], w2 = (T)g.w[2];
+    const int lane = b.lane;
+    uint32_t bitsA = 0, bitsB = 0;
+    T rc = (T)(64 * b.k + b.tau0);
+    const V2* cp = b.Cs + (int64_t)(b.tau0 + 2) * 32;  // the cost two steps ahead
+    const int ahead = b.span - 2 - b.tau0;
+    int t = 0;
+    if (STD && !rim && !mask) {
+        bool good = true;
+#pragma unroll 1
+        for (; t < kBlk; t += 2) {
+            good = fast_step<PUSH, T>(st, 0, rc, w0, w1, w2, b.w, b.r, b.kd, b.pD, b.pP, lane,
+                                      bitsA, bitsB);
+            if (!good) break;
+            st.q[0] = __ldcs(cp);
+            rc = addr(rc, (T)1);
+            good = fast_step<PUSH, T>(st, 1, rc, w0, w1, w2, b.w, b.r, b.kd, b.pD, b.pP, lane,
+                                      bitsA, bitsB);
+            if (!good) {
+                ++t;
+                break;
+            }
+            st.q[1] = __ldcs(cp + 32);
+            rc = addr(rc, (T)1);
+            cp += 64;
+            b.w += b.incW;
+            b.r += b.incR;
+            if (PUSH && b.pD) {
+                b.pD += 2;
+                b.pP += 2;
+            }
+        }
+    }
+    if (t < kBlk)
+        careful_steps<STD, PUSH, T>(g, st, b, td, t, rim, mask, rc, cp, ahead, bitsA, bitsB);
+    // step t's code belongs in bits 2t, 2t+1: reverse the sixteen pairs
+    bitsA = __brev(bitsA);
+    bitsB = __brev(bitsB);
+    bitsA = ((bitsA >> 1) & 0x55555555u) | ((bitsA & 0x55555555u) << 1);
+    bitsB = ((bitsB >> 1) & 0x55555555u) | ((bitsB & 0x55555555u) << 1);
     if (bw) {
         *bw = make_uint2(bitsA, bitsB);
-    } else if (!MASK || rA < R) {
+    } else if (64 * b.k + 2 * lane < b.R) {
         uint2* Bt = reinterpret_cast<uint2*>(td.Bw);
-        Bt[((int64_t)k * nP + (tau0 >> 4)) * 32 + lane] = make_uint2(bitsA, bitsB);
+        Bt[((int64_t)b.k * b.nP + (b.tau0 >> 4)) * 32 + lane] = make_uint2(bitsA, bitsB);
     }
+}
+
+template <typename T>
+__device__ __forceinline__ void zero_wave(Wave<T>& st) {
+    st.aD1 = st.aD2 = st.aD3 = st.bD1 = st.x1D = st.x2D = st.x3D = st.m1A = st.m1B = 0;
+    st.aP1 = st.aP2 = st.aP3 = st.bP1 = st.x1P = st.x2P = st.x3P = 0;
+#pragma unroll
+    for (int q = 0; q < 2; ++q) st.q[q].x = st.q[q].y = 0;
+}
+
+// Ring slots at which a block at step Tb starts to read (off = lag) or write
+// (off = 64); Tb = 0 here, stepped by kBlk with the blocks.
+__device__ __forceinline__ int ring_start(int off, int RB) { return (RB - off % RB) % RB; }
+__device__ __forceinline__ int ring_next(int s, int RB) { return s + kBlk == RB ? 0 : s + kBlk; }
+
+// Lane addresses of a block: exchange entries, but lane 31 stores into the
+// ring slot `wslot` (< 0: nobody reads the strip, its entry instead; then a
+// ring another strip still reads is not overwritten) and lane 0 loads slot
+// `rslot` (< 0: strip 0, which has no producer).
+template <typename T>
+__device__ __forceinline__ void lane_addresses(Block<T>& b, const Rings<T>& rg, int warp,
+                                               int wslot, int rslot) {
+    const bool w = b.lane == 31 && wslot >= 0, r = b.lane == 0 && rslot >= 0;
+    const int x = warp * kXch + b.lane;
+    const int y = b.lane == 0 ? x : x - 1;
+    b.w = (uint32_t)__cvta_generic_to_shared(w ? rg.P + wslot : rg.xP + x);
+    b.r = (uint32_t)__cvta_generic_to_shared(r ? rg.P + rslot : rg.xP + y);
+    b.kd = (uint32_t)__cvta_generic_to_shared(rg.D) -
+           d_address<T>((uint32_t)__cvta_generic_to_shared(rg.P), 0u);
+    b.incW = w ? 2 * (int)sizeof(int2) : 0;
+    b.incR = r ? 2 * (int)sizeof(int2) : 0;
 }
 
 // Bounded wait until progress word *p reaches target; gives up early when
@@ -639,19 +608,20 @@ __device__ __forceinline__ bool wait_progress(int* p, int target, const volatile
     return false;
 }
 
-// Ring length: the largest power of two whose rings fit the shared-memory
-// limit, capped at the first power of two >= lag + 64 (enough slack that the
-// pairwise waits rarely block); at least lag - 29 (one block of slack).
-// `vbytes` is the size of a DP value (8 for FP64, 4 for FP32).
+// Ring length: as many slots (a multiple of kBlk) as fit the shared-memory
+// limit, at most lag + 128 (enough slack that the pairwise waits rarely
+// block).  0: lag is too large for the memory; the largest accepted one is
+// 29 above the largest power of two of slots that fits (so the tile lengths
+// a caller may ask for do not depend on the rounding here), which leaves at
+// least the lag - 16 slots the waits need.  `vbytes` is the size of a DP
+// value (8 for FP64, 4 for FP32).
 __host__ __device__ inline int ring_len(int lag, int nw, int smem_limit, int vbytes) {
-    int cap = 16;
-    while (cap * 2 <= lag + 64) cap *= 2;
-    if (cap < lag + 64) cap *= 2;
-    int fit = 16;
     const int per = nw * (2 * vbytes + (int)sizeof(int2));
-    while ((fit * 2) * per + nw * (int)sizeof(int) <= smem_limit) fit *= 2;
-    const int rb = cap < fit ? cap : fit;
-    return rb >= lag - 29 ? rb : 0;
+    int pow2 = 16;
+    while ((pow2 * 2) * per + nw * (int)sizeof(int) <= smem_limit) pow2 *= 2;
+    if (lag - 29 > pow2) return 0;
+    const int fit = ((smem_limit - (nw + 2) * (int)sizeof(int)) / per - kXch) / kBlk * kBlk;
+    return lag + 128 < fit ? lag + 128 : fit;
 }
 
 // ---------------------------------------------------------------------------
@@ -769,14 +739,14 @@ __global__ void __launch_bounds__(NW * 32, 16 / NW)
                 int32_t* __restrict__ status, const int RB, const CostGen gen) {
     using V2 = typename Vec2<T>::type;
     extern __shared__ __align__(16) unsigned char smem_raw[];
-    Rings<T> rg;
-    rg.D = reinterpret_cast<V2*>(smem_raw);
-    rg.P = reinterpret_cast<int2*>(rg.D + NW * RB);
-    int* prog = reinterpret_cast<int*>(rg.P + NW * RB);
+    const Rings<T> rg = ring_layout<T>(smem_raw, NW, RB);
+    int* prog = reinterpret_cast<int*>(rg.xP + NW * kXch);
     __shared__ TileDesc td;
     __shared__ Sched2 s_sc;  // schedule of the current tile (read from smem, not held in registers)
     __shared__ int s_item, s_abort, s_ttot;
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    // (the warp index through a shuffle, so that what derives from it is known
+    // to be uniform in the warp and stays out of the vector registers)
+    const int lane = threadIdx.x & 31, warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0);
     const int prevw = (warp + NW - 1) % NW, nextw = (warp + 1) % NW;
     const int ntiles = ntiles_dev ? min(*ntiles_dev, ntiles_max) : ntiles_max;
     if (GEN && (int)blockIdx.x >= gen.nslots) return;  // no cost slot (the launch prevents it)
@@ -825,11 +795,8 @@ __global__ void __launch_bounds__(NW * 32, 16 / NW)
                 : reinterpret_cast<const V2*>(td.Csk);
 
         Wave<T> st;
-        st.aD1 = st.aD2 = st.aD3 = st.bD1 = st.bD2 = st.xpD = 0;
-        st.aP1 = st.aP2 = st.aP3 = st.bP1 = st.bP2 = st.xpP = 0;
-#pragma unroll
-        for (int q = 0; q < 2; ++q) st.q[q].x = st.q[q].y = 0;
-
+        zero_wave(st);
+        int rs = ring_start(lag, RB), ws = ring_start(64, RB);
         for (int Tb = 0; Tb < Ttot; Tb += kBlk) {
             int k = -1;
             if (Tb >= warp * lag) {
@@ -841,7 +808,7 @@ __global__ void __launch_bounds__(NW * 32, 16 / NW)
                 int failed = 0;
                 if (lane == 0) {
                     // producer (strip k-1) has written every ring slot this block reads
-                    if (k >= 1 && !wait_progress(prog + prevw, Tb - lag + 78, &s_abort)) failed = 1;
+                    if (k >= 1 && !wait_progress(prog + prevw, Tb - lag + 80, &s_abort)) failed = 1;
                     // consumer (strip k+1) has read every slot this block overwrites
                     if (!failed && k + 1 < sc.nS &&
                         !wait_progress(prog + nextw, Tb + lag - RB - 45, &s_abort))
@@ -852,31 +819,31 @@ __global__ void __launch_bounds__(NW * 32, 16 / NW)
                     }
                 }
                 if (__shfl_sync(0xffffffffu, failed, 0)) break;  // to the tile barrier
-                const int tau0 = Tb - k * lag;
-                const V2* Cs = Ct + (int64_t)k * sc.span * 32 + lane;
-                if (lane == 0 && tau0 + 2 * kBlk <= sc.span)
-                    prefetch_next_block(Ct + (int64_t)k * sc.span * 32, tau0 + kBlk);
-                if (tau0 == 0) {
-#pragma unroll
-                    for (int q = 0; q < 2; ++q) st.q[q] = __ldcs(Cs + q * 32);
+                Block<T> b;
+                b.tau0 = Tb - k * lag;
+                b.span = sc.span;
+                b.k = k;
+                b.R = R;
+                b.W = W;
+                b.lane = lane;
+                b.nP = sc.nP;
+                b.Cs = Ct + (int64_t)k * sc.span * 32 + lane;
+                lane_addresses(b, rg, warp, k + 1 < sc.nS ? warp * RB + ws : -1,
+                               k >= 1 ? prevw * RB + rs : -1);
+                b.pD = nullptr;
+                b.pP = nullptr;
+                if (lane == 0 && b.tau0 + 2 * kBlk <= sc.span)
+                    prefetch_next_block(Ct + (int64_t)k * sc.span * 32, b.tau0 + kBlk);
+                if (b.tau0 == 0) {
+                    st.q[0] = __ldcs(b.Cs);
+                    st.q[1] = __ldcs(b.Cs + 32);
                 }
-                const bool lean = k >= 1 && tau0 >= 80;
-                const bool interior = lean && k <= sc.nS - 2 && tau0 + 17 <= W;
-                if (STD && lean) {
-                    run_block_std<false, T>(g, st, rg, reinterpret_cast<char*>(rg.D), Cs, tau0,
-                                            k, lane, prevw * RB, warp * RB, RB - 1, Tb, lag, td,
-                                            sc.nP, nullptr, !interior, R, W, sc.span);
-                } else if (!STD && interior) {
-                    run_block<false, STD, false>(g, st, rg, reinterpret_cast<const char*>(rg.D),
-                                                 reinterpret_cast<char*>(rg.D), Cs, sc.span, tau0,
-                                                 k, R, W, lane, prevw * RB, warp * RB, RB - 1, Tb,
-                                                 lag, td, sc.nP);
-                } else
-                    run_block<true, STD, false>(g, st, rg, reinterpret_cast<const char*>(rg.D),
-                                         reinterpret_cast<char*>(rg.D), Cs,
-                                         sc.span, tau0, k, R, W, lane,
-                                         prevw * RB, warp * RB, RB - 1, Tb, lag, td, sc.nP);
+                // the block reaches the last row or column, or past them
+                const bool mask = k > sc.nS - 2 || b.tau0 + 17 > W;
+                run_block<STD, false, T>(g, st, b, td, k == 0 || b.tau0 < 80, mask, nullptr);
             }
+            rs = ring_next(rs, RB);
+            ws = ring_next(ws, RB);
             __syncwarp();
             if (lane == 31) my_prog.store(Tb + kBlk, cuda::memory_order_release);
         }
@@ -930,17 +897,15 @@ __global__ void __launch_bounds__(kClW * 32, 1)
     cg::cluster_group cl = cg::this_cluster();
     const int rank = (int)cl.block_rank();
     extern __shared__ __align__(16) unsigned char smem_raw[];
-    Rings<T> rg;  // this CTA's rings
-    rg.D = reinterpret_cast<V2*>(smem_raw);
-    rg.P = reinterpret_cast<int2*>(rg.D + kClW * RB);
+    const Rings<T> rg = ring_layout<T>(smem_raw, kClW, RB);  // this CTA's rings
     // progress words: [w] warp w's; [kClW] the other CTA's last warp's (this
     // CTA's warp 0 waits on it); [kClW + 1] the other CTA's warp 0's (this
     // CTA's last warp waits on it) -- written by the other CTA, polled here
-    int* prog = reinterpret_cast<int*>(rg.P + kClW * RB);
+    int* prog = reinterpret_cast<int*>(rg.xP + kClW * kXch);
     __shared__ TileDesc td;
     __shared__ Sched2 s_sc;
     __shared__ int s_item, s_abort, s_ttot;
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int lane = threadIdx.x & 31, warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0);
     const int vw = rank * kClW + warp;
     const int pv = (vw + NWT - 1) % NWT, nv = (vw + 1) % NWT;
     // the producer's rings (generic address, this CTA's or the peer's)
@@ -948,8 +913,8 @@ __global__ void __launch_bounds__(kClW * 32, 1)
     // dependency chain) and reads its producer's ring from its own CTA: ring
     // region w of a CTA is written by warp w of the CTA that feeds it (its own
     // warp w, or for w = kClW - 1 the other CTA's last warp)
-    const char* rbase = reinterpret_cast<const char*>(rg.D);
-    char* wbase = reinterpret_cast<char*>(cl.map_shared_rank(rg.D, nv / kClW));
+    V2* wD = cl.map_shared_rank(rg.D, nv / kClW);
+    int2* wP = cl.map_shared_rank(rg.P, nv / kClW);
     // cluster scope only where the neighbour is in the other CTA
     const bool prev_remote = pv / kClW != rank, next_remote = nv / kClW != rank;
     const bool read_remotely = warp == 0 || warp == kClW - 1;  // my progress word
@@ -989,11 +954,8 @@ __global__ void __launch_bounds__(kClW * 32, 1)
         const V2* Ct = reinterpret_cast<const V2*>(td.Csk);
 
         Wave<T> st;
-        st.aD1 = st.aD2 = st.aD3 = st.bD1 = st.bD2 = st.xpD = 0;
-        st.aP1 = st.aP2 = st.aP3 = st.bP1 = st.bP2 = st.xpP = 0;
-#pragma unroll
-        for (int q = 0; q < 2; ++q) st.q[q].x = st.q[q].y = 0;
-
+        zero_wave(st);
+        int rs = ring_start(lag, RB), ws = ring_start(64, RB);
         for (int Tb = 0; Tb < Ttot; Tb += kBlk) {
             int k = -1;
             uint2 bw = make_uint2(0u, 0u);
@@ -1008,8 +970,8 @@ __global__ void __launch_bounds__(kClW * 32, 1)
                     // producer (strip k-1) has written every ring slot this block reads
                     if (k >= 1 &&
                         !(prev_remote
-                              ? wait_progress_cl(prog + kClW, Tb - lag + 78, &s_abort)
-                              : wait_progress(prog + pv % kClW, Tb - lag + 78, &s_abort)))
+                              ? wait_progress_cl(prog + kClW, Tb - lag + 80, &s_abort)
+                              : wait_progress(prog + pv % kClW, Tb - lag + 80, &s_abort)))
                         failed = 1;
                     // consumer (strip k+1) has read every slot this block overwrites
                     if (!failed && k + 1 < sc.nS &&
@@ -1023,30 +985,32 @@ __global__ void __launch_bounds__(kClW * 32, 1)
                     }
                 }
                 if (__shfl_sync(0xffffffffu, failed, 0)) break;  // to the tile's end barrier
-                const int tau0 = Tb - k * lag;
-                const V2* Cs = Ct + (int64_t)k * sc.span * 32 + lane;
-                if (lane == 0 && tau0 + 2 * kBlk <= sc.span)
-                    prefetch_next_block(Ct + (int64_t)k * sc.span * 32, tau0 + kBlk);
-                if (tau0 == 0) {
-#pragma unroll
-                    for (int q = 0; q < 2; ++q) st.q[q] = __ldcs(Cs + q * 32);
+                Block<T> b;
+                b.tau0 = Tb - k * lag;
+                b.Cs = Ct + (int64_t)k * sc.span * 32 + lane;
+                b.span = sc.span;
+                b.k = k;
+                b.R = R;
+                b.W = W;
+                b.lane = lane;
+                b.nP = sc.nP;
+                const bool feeds = k + 1 < sc.nS;
+                lane_addresses(b, rg, warp, feeds && !next_remote ? warp * RB + ws : -1,
+                               k >= 1 ? (pv % kClW) * RB + rs : -1);
+                b.pD = feeds && next_remote ? wD + warp * RB + ws : nullptr;
+                b.pP = feeds && next_remote ? wP + warp * RB + ws : nullptr;
+                if (lane == 0 && b.tau0 + 2 * kBlk <= sc.span)
+                    prefetch_next_block(Ct + (int64_t)k * sc.span * 32, b.tau0 + kBlk);
+                if (b.tau0 == 0) {
+                    st.q[0] = __ldcs(b.Cs);
+                    st.q[1] = __ldcs(b.Cs + 32);
                 }
-                const bool lean = k >= 1 && tau0 >= 80;
-                const bool interior = lean && k <= sc.nS - 2 && tau0 + 17 <= W;
-                if (STD && lean)
-                    run_block_std<true, T>(g, st, rg, wbase, Cs, tau0, k, lane,
-                                           (pv % kClW) * RB, warp * RB, RB - 1, Tb, lag, td,
-                                           sc.nP, &bw, !interior, R, W, sc.span);
-                else if (!STD && interior)
-                    run_block<false, STD, true>(g, st, rg, rbase, wbase, Cs, sc.span, tau0, k, R,
-                                                W, lane, (pv % kClW) * RB, warp * RB, RB - 1, Tb,
-                                                lag, td, sc.nP, &bw);
-                else
-                    run_block<true, STD, true>(g, st, rg, rbase, wbase, Cs, sc.span, tau0, k, R, W,
-                                         lane,
-                                         (pv % kClW) * RB, warp * RB, RB - 1, Tb, lag, td,
-                                         sc.nP, &bw);
+                // the block reaches the last row or column, or past them
+                const bool mask = k > sc.nS - 2 || b.tau0 + 17 > W;
+                run_block<STD, true, T>(g, st, b, td, k == 0 || b.tau0 < 80, mask, &bw);
             }
+            rs = ring_next(rs, RB);
+            ws = ring_next(ws, RB);
             __syncwarp();
             // publish first: the backpointer store below is nobody's dependency
             if (lane == 31) {
@@ -1093,7 +1057,7 @@ static size_t smem_bytes(int32_t L, int nw, int smem_limit, int vbytes) {
     const Sched2 s = make_sched2(L, L, nw);
     const int rb = ring_len(s.lag, nw, smem_limit, vbytes);
     if (rb == 0) return (size_t)1 << 30;  // does not fit
-    return (size_t)nw * rb * (2 * vbytes + sizeof(int2)) + nw * sizeof(int);
+    return vbytes == 8 ? ring_bytes<double>(nw, rb, nw) : ring_bytes<float>(nw, rb, nw);
 }
 
 int stage1_queue_warps(int ntiles, int32_t L, int num_sms) {
@@ -1163,8 +1127,7 @@ static cudaError_t launch_cl_t(const TileDesc* descs, int ntiles, int* head, con
     const Sched2 s = make_sched2(g.L, g.L, kClW * kClN);
     const int rb = ring_len(s.lag, kClW, limit, (int)sizeof(T));
     if (rb == 0) return cudaErrorInvalidValue;
-    const size_t smem =
-        (size_t)kClW * rb * ring_slot_bytes<T>() + (kClW + 2) * sizeof(int);
+    const size_t smem = ring_bytes<T>(kClW, rb, kClW + 2);
     auto kern = k_stage1_cl<STD, T>;
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                          (int)smem);
@@ -1199,8 +1162,7 @@ static int cl_max_t(const Geo& g) {
     const Sched2 s = make_sched2(g.L, g.L, kClW * kClN);
     const int rb = ring_len(s.lag, kClW, limit, (int)sizeof(T));
     if (rb == 0) return 0;
-    const size_t smem =
-        (size_t)kClW * rb * ring_slot_bytes<T>() + (kClW + 2) * sizeof(int);
+    const size_t smem = ring_bytes<T>(kClW, rb, kClW + 2);
     auto kern = k_stage1_cl<STD, T>;
     if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) !=
         cudaSuccess)
