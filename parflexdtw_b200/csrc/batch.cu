@@ -396,9 +396,9 @@ extern "C" int pfx_batch_create(int32_t n, const int64_t* N, const int64_t* M, c
         b->max_wave_tiles = std::max(b->max_wave_tiles, t);
     }
     b->nw = nw ? nw
-               : stage1_queue_warps((int)std::min<int64_t>(b->max_wave_tiles, 1 << 30), maxL,
+               : stage1_queue_warps(b->max_wave_tiles, maxL,
                                     num_sms_cur());
-    if (b->nw == 0 || stage1_queue_warps(1, maxL, 1) == 0) {
+    if (b->nw == 0 || !stage1_queue_fits(maxL, 16)) {
         batch_free(b);
         return errf(PFX_ERR_TOO_LARGE, "L=%d: the stage-1 rings do not fit in shared memory", maxL);
     }

@@ -165,8 +165,9 @@ int pfx::plan_init(pfx_plan* p, int64_t N, int64_t M, int32_t L, const int64_t* 
     cudaGetDevice(&p->device);
     const Geo& g = p->g;
     const int64_t nt = (int64_t)g.n1 * g.n2;
-    p->nw = nw ? nw : stage1_queue_warps((int)std::min<int64_t>(nt, 1 << 30), L, num_sms_cur());
-    if (p->nw == 0 || stage1_queue_warps(1, L, 1) == 0)
+    p->nw = nw ? nw : stage1_queue_warps(nt, L, num_sms_cur());
+    p->nw_default = p->nw;
+    if (p->nw == 0 || !stage1_queue_fits(L, 16))
         return fail(PFX_ERR_TOO_LARGE, "L=%d: the stage-1 rings do not fit in shared memory", L);
     p->skew_stride = skew_slab_elems(L);
     p->n4 = nt * 2 * g.L;
@@ -299,10 +300,11 @@ extern "C" int pfx_plan_create_ex(int64_t N, int64_t M, int32_t L, const int64_t
 extern "C" int pfx_plan_set_warps(pfx_plan* p, int32_t nw) {
     if (!p) return fail(PFX_ERR_ARG, "null plan");
     if (nw != 4 && nw != 8 && nw != 16) return fail(PFX_ERR_ARG, "nw=%d: 4, 8 or 16", nw);
-    if (stage1_queue_warps(1, p->g.L, 1) == 0 ||
-        (nw != 16 && stage1_queue_warps(1 << 30, p->g.L, 1) > nw))
+    if (!stage1_queue_fits(p->g.L, nw))
         return fail(PFX_ERR_TOO_LARGE, "L=%d: rings of %d warps do not fit", p->g.L, nw);
     p->nw = nw;
+    p->nw_set = nw != p->nw_default;
+    p->s1_planned = 0;
     return PFX_OK;
 }
 
@@ -531,36 +533,39 @@ extern "C" int pfx_stage1(pfx_plan* p, const double* C, int64_t ldc, void* strea
                                p->s1.status, p->nw, p->fp32 != 0, s));
     } else {
         const int nt = p->g.n1 * p->g.n2;
-        const int sms = num_sms_cur();
-        const int maxc = (p->nw == 16 && p->arena_mode == 0 && nt < sms)
-                             ? stage1_cluster_max(p->g, p->fp32 != 0)
-                             : 0;
-        if (maxc > 0) {
-            // fewer tiles than SMs: the largest tiles (the queue is ordered
-            // largest first) take two SMs each, as many as leave one SM for
-            // every other tile and as many clusters as can run at once; the
-            // other tiles run at the same time on a second stream
-            int nbig = nt < sms - nt ? nt : sms - nt;
-            if (nbig > maxc) nbig = maxc;
-            if (!p->aux) {
+        // (decided once per plan: it asks the driver what fits)
+        if (!p->s1_planned) {
+            p->s1_plan = p->arena_mode == 0 && (!p->nw_set || p->nw == 16)
+                             ? stage1_plan(p->g, nt, p->fp32 != 0, num_sms_cur())
+                             : S1Plan{0, p->nw, 0};
+            if (p->s1_plan.cn == 0) p->s1_plan.cw = p->nw;
+            p->s1_planned = 1;
+        }
+        const S1Plan& sp = p->s1_plan;
+        if (sp.cn > 0) {
+            // few tiles: the largest (the queue is ordered largest first) on
+            // clusters, the others at the same time on a second stream
+            if (nt > sp.big && !p->aux) {
                 CK(cudaStreamCreateWithFlags(&p->aux, cudaStreamNonBlocking));
                 CK(cudaEventCreateWithFlags(&p->ev_fork, cudaEventDisableTiming));
                 CK(cudaEventCreateWithFlags(&p->ev_join, cudaEventDisableTiming));
             }
-            CK(cudaMemsetAsync(p->head2, 0, sizeof(int), s));
-            CK(cudaEventRecord(p->ev_fork, s));
-            // the clusters first, so that they find pairs of free SMs
-            CK(launch_stage1_cluster(p->descs, nbig, p->head, p->g, p->s1.status,
-                                     p->fp32 != 0, s));
-            if (nt > nbig) {
+            if (nt > sp.big) {
+                CK(cudaMemsetAsync(p->head2, 0, sizeof(int), s));
+                CK(cudaEventRecord(p->ev_fork, s));
+            }
+            // the clusters first, so that they find neighbouring free SMs
+            CK(launch_stage1_cluster(sp.cn, sp.cw, p->descs, sp.big, p->head, p->g,
+                                     p->s1.status, p->fp32 != 0, s));
+            if (nt > sp.big) {
                 CK(cudaStreamWaitEvent(p->aux, p->ev_fork, 0));
-                CK(launch_stage1_queue(p->descs + nbig, nt - nbig, nullptr, p->head2, p->g,
+                CK(launch_stage1_queue(p->descs + sp.big, nt - sp.big, nullptr, p->head2, p->g,
                                        p->s1.status, 16, p->fp32 != 0, p->aux));
                 CK(cudaEventRecord(p->ev_join, p->aux));
                 CK(cudaStreamWaitEvent(s, p->ev_join, 0));
             }
         } else {
-            CK(launch_stage1_queue(p->descs, nt, nullptr, p->head, p->g, p->s1.status, p->nw,
+            CK(launch_stage1_queue(p->descs, nt, nullptr, p->head, p->g, p->s1.status, sp.cw,
                                    p->fp32 != 0, s));
         }
     }

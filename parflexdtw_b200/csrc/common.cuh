@@ -227,14 +227,28 @@ cudaError_t launch_mask_slots(const uint8_t* mask, int n, int32_t* slot, cudaStr
 // Keeps the descriptors whose tile is set in `mask`, in order; *count = kept.
 cudaError_t launch_compact_descs(const TileDesc* in, int n, const uint8_t* mask, TileDesc* out,
                                  int* count, cudaStream_t st);
-// Stage 1 of descs[0, ntiles) on clusters of two 16-warp CTAs (32 warps per
-// tile), claimed through *head; for alignments with fewer tiles than SMs.
-cudaError_t launch_stage1_cluster(const TileDesc* descs, int ntiles, int* head, const Geo& g,
-                                  int32_t* status, bool fp32, cudaStream_t st);
+// Stage 1 of descs[0, ntiles) on clusters of cn CTAs of cw (4, 8, 12 or 16)
+// warps each, claimed through *head; for alignments with few tiles.
+cudaError_t launch_stage1_cluster(int cn, int cw, const TileDesc* descs, int ntiles, int* head,
+                                  const Geo& g, int32_t* status, bool fp32, cudaStream_t st);
 // Clusters of that kernel that can run at once on this device (0: none).
-int stage1_cluster_max(const Geo& g, bool fp32);
-// Smallest valid warps-per-tile choice heuristic for `ntiles` tiles of length L.
-int stage1_queue_warps(int ntiles, int32_t L, int num_sms);
+int stage1_cluster_max(int cn, int cw, const Geo& g, bool fp32);
+// Whether the queue kernel's rings fit at tile length L with nw warps per
+// tile; its modelled time for ntiles tiles; the nw of the least (0: none fits).
+bool stage1_queue_fits(int32_t L, int nw);
+double stage1_queue_ns(int64_t ntiles, int32_t L, int nw, int num_sms);
+int stage1_queue_warps(int64_t ntiles, int32_t L, int num_sms);
+// Modelled pipeline steps of an R x W tile on nw warps, and the time of a
+// step with `ctas` CTAs of nw warps on an SM.
+double stage1_model_steps(int32_t R, int32_t W, int nw);
+double stage1_step_ns(int nw, int ctas);
+// How to run the ntiles tiles of one alignment: the first `big` (the largest)
+// on clusters of cn CTAs of cw warps, the rest on single CTAs of 16 warps in
+// a second stream; cn = 0: all through the queue kernel, cw warps per tile.
+struct S1Plan {
+    int cn, cw, big;
+};
+S1Plan stage1_plan(const Geo& g, int ntiles, bool fp32, int num_sms);
 // Cost-building launchers take an optional slot map: tile t's slab is slab
 // slot[t] of Csk, and tiles with slot[t] < 0 are skipped (null: slab = t).
 // The feature launchers also take an optional list of the nlist tiles to

@@ -73,7 +73,7 @@ def check(C, warps, oracle_mod, steps=STD, weights=(2.0, 3.0, 3.0), precision="f
     assert np.array_equal(B, Bo)
 
 
-# warps 0: the plan's own choice for one tile, a cluster of two 16-warp CTAs
+# warps 0: the plan's own choice (for one tile, a cluster of CTAs)
 @pytest.mark.parametrize("warps", [0, 4, 8])
 @pytest.mark.parametrize("R,W", [(2, 2), (3, 200), (200, 3), (64, 97), (65, 96), (127, 129),
                                  (128, 128), (193, 241), (320, 65), (700, 655)])
@@ -101,7 +101,8 @@ def test_step_sets(steps, weights, kind, oracle_mod):
     check(cost(kind, 150, 219, 9), 4, oracle_mod, steps, weights)
 
 
-@pytest.mark.parametrize("L,warps", [(257, 4), (320, 8), (1000, 4), (2000, 4), (2000, 16)])
+@pytest.mark.parametrize("L,warps", [(257, 4), (320, 8), (1000, 0), (1000, 4), (2000, 0),
+                                     (2000, 4), (2000, 16), (2600, 0)])
 def test_long_tiles_share_rings(L, warps, oracle_mod):
     """Several rounds of strips per warp, last strips full or not: no strip
     overwrites ring slots another one still reads."""
