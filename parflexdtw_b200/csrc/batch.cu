@@ -12,6 +12,7 @@
 #include <string.h>
 
 #include <algorithm>
+#include <cmath>
 #include <vector>
 
 #include "plan.cuh"
@@ -20,7 +21,7 @@ using namespace pfx;
 
 namespace {
 
-constexpr int kSide = 32;     // streams stage 2 of a wave is spread over
+constexpr int kSide = 4;      // streams the waves' stage 2 is spread over
 constexpr int kCostSide = 3;  // extra streams a wave's per-pair cost work is spread over
 
 struct PairOut {
@@ -152,6 +153,17 @@ __global__ void k_path_to_rows(const PathRef* __restrict__ pr, const int64_t* __
     }
 }
 
+// Paths one after the other: pair p's points go to out[2 o_p ..) as they are.
+__global__ void k_path_pack(const PathRef* __restrict__ pr, const int64_t* __restrict__ offs,
+                            const int64_t* __restrict__ lens, int64_t* __restrict__ out) {
+    const longlong2* wp = reinterpret_cast<const longlong2*>(pr[blockIdx.y].wp);
+    longlong2* o = reinterpret_cast<longlong2*>(out) + offs[blockIdx.y];
+    const int64_t K = lens[blockIdx.y];
+    for (int64_t k = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; k < K;
+         k += (int64_t)gridDim.x * blockDim.x)
+        o[k] = wp[k];
+}
+
 int errf(int status, const char* fmt, ...) {
     char buf[512];
     va_list ap;
@@ -222,6 +234,8 @@ struct pfx_batch {
     bool ran = false;  // a run since pfx_batch_set_masks
     // path checks and row-layout copies (allocated on first use)
     PathRef* pref = nullptr;
+    S2Pair* s2tab = nullptr;  // every pair's stage 2, in wave order (NaN beta: stale)
+    double s2tab_beta = 0.0;
     int32_t* rows = nullptr;  // lo | hi block-row scratch
     size_t rows_cap = 0;
     int64_t* prow = nullptr;  // device staging of row-layout paths, + offsets and lengths
@@ -246,6 +260,10 @@ static void batch_free(pfx_batch* b) {
     if (b->cfork_ev) cudaEventDestroy(b->cfork_ev);
     for (cudaEvent_t e : b->phase_ev) cudaEventDestroy(e);
     if (b->cap) cudaStreamDestroy(b->cap);
+    for (pfx_plan& p : b->plans) {  // staging of pfx_result / pfx_copy_path
+        if (p.res_host) cudaFreeHost(p.res_host);
+        if (p.path_host) cudaFreeHost(p.path_host);
+    }
     if (b->arena) cudaFree(b->arena);
     if (b->slabs) cudaFree(b->slabs);
     if (b->stage) cudaFreeHost(b->stage);
@@ -253,6 +271,7 @@ static void batch_free(pfx_batch* b) {
     if (b->fbsegs) cudaFree(b->fbsegs);
     if (b->gpairs) cudaFree(b->gpairs);
     if (b->pref) cudaFree(b->pref);
+    if (b->s2tab) cudaFree(b->s2tab);
     if (b->rows) cudaFree(b->rows);
     if (b->prow) cudaFree(b->prow);
     cudaSetDevice(cur);
@@ -737,6 +756,7 @@ extern "C" int pfx_batch_set_masks(pfx_batch* b, const uint8_t* masks, int32_t o
     b->max_wave_tiles = 0;
     for (int64_t x : wt) b->max_wave_tiles = std::max(b->max_wave_tiles, x);
     b->masked = 1;
+    b->s2tab_beta = NAN;  // the waves changed
     if (b->exec) {
         cudaGraphExecDestroy(b->exec);
         b->exec = nullptr;
@@ -876,7 +896,7 @@ extern "C" int pfx_batch_plan(pfx_batch* b, int32_t i, pfx_plan** plan) {
 
 // The launch sequence of one batch run, on stream s (captured or direct;
 // `timed` records the phase events, direct runs only).
-static int batch_enqueue(pfx_batch* b, double beta, cudaStream_t s, bool timed) {
+static int batch_enqueue(pfx_batch* b, cudaStream_t s, bool timed) {
     const int waves = (int)b->wave_first.size() - 1;
     BCK(cudaMemsetAsync(b->heads, 0, (size_t)waves * sizeof(int), s));
     if (timed && b->phase_ev.empty()) {
@@ -887,7 +907,6 @@ static int batch_enqueue(pfx_batch* b, double beta, cudaStream_t s, bool timed) 
     auto mark = [&](int w, int k) -> cudaError_t {
         return timed ? cudaEventRecord(b->phase_ev[(size_t)w * 4 + k], s) : cudaSuccess;
     };
-    int st;
     int used_side = 0;  // side streams forked so far (joined at the end)
     // a wave's per-pair launches (cost, edge gathers) spread over s and up to
     // kCostSide more streams, forked from s and joined back into it, so that
@@ -974,16 +993,24 @@ static int batch_enqueue(pfx_batch* b, double beta, cudaStream_t s, bool timed) 
         BCK(cost_join(nc));
         BCK(mark(w, 3));
         BCK(cudaEventRecord(b->fork_ev, s));
-        const int nside = std::min(kSide, q1 - q0);
-        used_side = std::max(used_side, nside);
-        for (int k = 0; k < nside; ++k) BCK(cudaStreamWaitEvent(b->side[k], b->fork_ev, 0));
+        // the rest of the wave's stage 2: a launch per step for all its pairs
+        const cudaStream_t ss = b->side[w % kSide];
+        used_side = std::max(used_side, w % kSide + 1);
+        BCK(cudaStreamWaitEvent(ss, b->fork_ev, 0));
+        S2Pair one;
+        memset(&one, 0, sizeof(one));
         for (int q = q0; q < q1; ++q) {
-            pfx_plan* p = &b->plans[b->wave_pairs[q]];
-            cudaStream_t ss = b->side[(q - q0) % nside];
-            BCK(launch_stage2_prop(p->g, p->s2, ss));
-            if ((st = pfx_stage2_scan(p, beta, ss))) return st;
-            if ((st = pfx_stage2_stitch(p, 1, 0, 0, 0, 0, ss))) return st;
+            const Geo& g = b->plans[b->wave_pairs[q]].g;
+            one.g.n1 = std::max(one.g.n1, g.n1);
+            one.g.n2 = std::max(one.g.n2, g.n2);
+            one.g.L = std::max(one.g.L, g.L);
+            one.g.N = std::max(one.g.N, g.N);
+            one.g.M = std::max(one.g.M, g.M);
         }
+        const S2Pair* tab = b->s2tab + q0;
+        BCK(launch_stage2_prop(one, tab, q1 - q0, ss));
+        BCK(launch_sync_scan(one, tab, q1 - q0, ss));
+        BCK(launch_stitch(one, tab, q1 - q0, ss, 1, 0, 0, 0, 0));
     }
     for (int k = 0; k < used_side; ++k) {
         BCK(cudaEventRecord(b->join_ev[k], b->side[k]));
@@ -1001,7 +1028,21 @@ extern "C" int pfx_batch_run(pfx_batch* b, double beta, int32_t use_graph, void*
         b->done = b->mask_host;
         b->ran = true;
     }
-    if (!use_graph) return batch_enqueue(b, beta, s, true);
+    if (!b->s2tab || b->s2tab_beta != beta) {
+        // every pair's stage 2 in wave order (waves and beta are fixed until
+        // the next pfx_batch_set_masks or another beta)
+        BCK(cudaStreamSynchronize(s));  // an earlier run may still read the table
+        if (!b->s2tab) BCK(cudaMalloc(&b->s2tab, (size_t)b->n * sizeof(S2Pair)));
+        std::vector<S2Pair> tab((size_t)b->n);
+        for (int q = 0; q < b->n; ++q) {
+            const pfx_plan& p = b->plans[b->wave_pairs[q]];
+            tab[q] = S2Pair{p.g, p.s2, buffer_global(p.g.N, p.g.M, beta)};
+        }
+        BCK(cudaMemcpy(b->s2tab, tab.data(), tab.size() * sizeof(S2Pair),
+                       cudaMemcpyHostToDevice));
+        b->s2tab_beta = beta;
+    }
+    if (!use_graph) return batch_enqueue(b, s, true);
     if (!b->exec || b->graph_beta != beta) {
         if (b->exec) {
             cudaGraphExecDestroy(b->exec);
@@ -1012,7 +1053,7 @@ extern "C" int pfx_batch_run(pfx_batch* b, double beta, int32_t use_graph, void*
         BCK(cudaStreamWaitEvent(b->cap, b->fork_ev, 0));
         BCK(cudaStreamBeginCapture(b->cap, cudaStreamCaptureModeRelaxed));
         const int64_t k0 = pfx_kernel_launches();
-        const int st = batch_enqueue(b, beta, b->cap, false);
+        const int st = batch_enqueue(b, b->cap, false);
         // recorded launches run at each replay: count them there, not here
         b->graph_kernels = pfx_kernel_launches() - k0;
         count_launches(-(int)b->graph_kernels);
@@ -1128,6 +1169,24 @@ extern "C" int pfx_batch_check_paths(pfx_batch* b, int32_t margin, uint8_t* near
     return PFX_OK;
 }
 
+// Device staging for `total` path points, and room for every pair's offset
+// and length.
+static int ensure_prow(pfx_batch* b, int64_t total, cudaStream_t s, int64_t** off, int64_t** len) {
+    const size_t need = (size_t)2 * total + 2 * (size_t)b->n;
+    if (need > b->prow_cap) {
+        BCK(cudaStreamSynchronize(s));
+        if (b->prow) cudaFree(b->prow);
+        b->prow = nullptr;
+        b->prow_cap = 0;
+        const size_t cap2 = need + need / 4 + 1024;
+        BCK(cudaMalloc(&b->prow, cap2 * sizeof(int64_t)));
+        b->prow_cap = cap2;
+    }
+    *off = b->prow + b->prow_cap - 2 * (size_t)b->n;
+    *len = *off + b->n;
+    return PFX_OK;
+}
+
 extern "C" int pfx_batch_copy_paths_rows(pfx_batch* b, void* stream, int64_t* host,
                                          const int64_t* offsets, const int64_t* lens,
                                          int64_t cap) {
@@ -1142,18 +1201,8 @@ extern "C" int pfx_batch_copy_paths_rows(pfx_batch* b, void* stream, int64_t* ho
     }
     int st = ensure_pref(b);
     if (st) return st;
-    const size_t need = (size_t)2 * total + 2 * (size_t)b->n;
-    if (need > b->prow_cap) {
-        BCK(cudaStreamSynchronize(s));
-        if (b->prow) cudaFree(b->prow);
-        b->prow = nullptr;
-        b->prow_cap = 0;
-        const size_t cap2 = need + need / 4 + 1024;
-        BCK(cudaMalloc(&b->prow, cap2 * sizeof(int64_t)));
-        b->prow_cap = cap2;
-    }
-    int64_t* d_off = b->prow + b->prow_cap - 2 * (size_t)b->n;
-    int64_t* d_len = d_off + b->n;
+    int64_t *d_off = nullptr, *d_len = nullptr;
+    if ((st = ensure_prow(b, total, s, &d_off, &d_len))) return st;
     std::vector<int64_t> ol((size_t)2 * b->n);
     std::copy(offsets, offsets + b->n, ol.begin());
     std::copy(lens, lens + b->n, ol.begin() + b->n);
@@ -1171,17 +1220,43 @@ extern "C" int pfx_batch_copy_paths(pfx_batch* b, void* stream, int64_t* wp_host
                                     const int64_t* offsets, int64_t cap) {
     if (!b || !wp_host || !offsets) return errf(PFX_ERR_ARG, "null argument");
     cudaStream_t s = (cudaStream_t)stream;
-    std::vector<int64_t> lens(b->n);
-    for (int i = 0; i < b->n; ++i)
-        BCK(cudaMemcpyAsync(&lens[i], b->plans[i].s2.wp_len, 8, cudaMemcpyDeviceToHost, s));
+    const int n = b->n;
+    // every pair's length in one copy, then, where the paths follow one another
+    // in the host array, every path in one copy
+    k_gather_results<<<(n + 127) / 128, 128, 0, s>>>(b->pout, n, b->res);
+    count_launches(1);
+    BCK(cudaGetLastError());
+    std::vector<int64_t> h((size_t)n * 9), ol((size_t)2 * n);
+    BCK(cudaMemcpyAsync(h.data(), b->res, h.size() * 8, cudaMemcpyDeviceToHost, s));
     BCK(cudaStreamSynchronize(s));
-    for (int i = 0; i < b->n; ++i) {
-        if (offsets[i] < 0 || offsets[i] + lens[i] > cap)
+    int64_t total = 0;
+    bool dense = true;
+    for (int i = 0; i < n; ++i) {
+        const int64_t len = h[(size_t)i * 9 + 8];
+        if (offsets[i] < 0 || offsets[i] + len > cap)
             return errf(PFX_ERR_ARG, "pair %d: path of %lld points at offset %lld exceeds %lld", i,
-                        (long long)lens[i], (long long)offsets[i], (long long)cap);
-        if (lens[i] > 0)
-            BCK(cudaMemcpyAsync(wp_host + 2 * offsets[i], b->plans[i].s2.wp, (size_t)lens[i] * 16,
-                                cudaMemcpyDeviceToHost, s));
+                        (long long)len, (long long)offsets[i], (long long)cap);
+        dense = dense && offsets[i] - offsets[0] == total;
+        ol[i] = total;
+        ol[n + i] = len;
+        total += len;
+    }
+    if (!dense) {
+        for (int i = 0; i < n; ++i)
+            if (ol[n + i] > 0)
+                BCK(cudaMemcpyAsync(wp_host + 2 * offsets[i], b->plans[i].s2.wp,
+                                    (size_t)ol[n + i] * 16, cudaMemcpyDeviceToHost, s));
+    } else if (total > 0) {
+        int st = ensure_pref(b);
+        if (st) return st;
+        int64_t *d_off = nullptr, *d_len = nullptr;
+        if ((st = ensure_prow(b, total, s, &d_off, &d_len))) return st;
+        BCK(cudaMemcpyAsync(d_off, ol.data(), ol.size() * 8, cudaMemcpyHostToDevice, s));
+        k_path_pack<<<dim3(16, n), 256, 0, s>>>(b->pref, d_off, d_len, b->prow);
+        count_launches(1);
+        BCK(cudaGetLastError());
+        BCK(cudaMemcpyAsync(wp_host + 2 * offsets[0], b->prow, (size_t)total * 16,
+                            cudaMemcpyDeviceToHost, s));
     }
     BCK(cudaStreamSynchronize(s));
     return PFX_OK;

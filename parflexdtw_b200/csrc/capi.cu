@@ -147,6 +147,8 @@ extern "C" void pfx_plan_destroy(pfx_plan* p) {
     cudaGetDevice(&cur);
     cudaSetDevice(p->device);
     for (int i = 0; i < p->nblocks; ++i) cudaFree(p->blocks[i]);
+    if (p->res_host) cudaFreeHost(p->res_host);
+    if (p->path_host) cudaFreeHost(p->path_host);
     if (p->aux) cudaStreamDestroy(p->aux);
     if (p->ev_fork) cudaEventDestroy(p->ev_fork);
     if (p->ev_join) cudaEventDestroy(p->ev_join);
@@ -202,15 +204,19 @@ int pfx::plan_init(pfx_plan* p, int64_t N, int64_t M, int32_t L, const int64_t* 
     PA(&p->s2.right_L, N);
     PA(&p->s2.seg_norm, 2 * ms);
     PA(&p->s2.seg_meta, 12 * ms);
-    PA(&p->s2.best, 1);
-    PA(&p->s2.best_end, 7);
+    // the result in one block: best cost, end (7), path length, status
+    PA(&p->res, 10);
+    p->s2.best = reinterpret_cast<double*>(p->res);
+    p->s2.best_end = p->res + 1;
+    p->s2.wp_len = p->res + 8;
+    p->s1.status = reinterpret_cast<int32_t*>(p->res + 9);
+    PA(&p->s2.diag_list, p->n4);
+    PA(&p->s2.diag_count, g.n1 + g.n2);
     PA(&p->s2.chain, 101 * 12);
     PA(&p->s2.chain_len, 1);
     PA(&p->s2.seg_pts, 101 * p->s2.seg_cap * 2);
     PA(&p->s2.seg_len, 101);
     PA(&p->s2.wp, 101 * p->s2.seg_cap * 2);
-    PA(&p->s2.wp_len, 1);
-    PA(&p->s1.status, 1);
     PA(&p->descs, nt);
     PA(&p->head, 1);
     PA(&p->head2, 1);
@@ -221,10 +227,9 @@ int pfx::plan_init(pfx_plan* p, int64_t N, int64_t M, int32_t L, const int64_t* 
     PA(&p->nsub, 1);
 #undef PA
     if (p->arena_mode) return PFX_OK;  // arenas are zeroed by their owner
-    CK(cudaMemset(p->s2.best_end, 0, 7 * sizeof(int64_t)));
+    CK(cudaMemset(p->res, 0, 10 * sizeof(int64_t)));
     CK(cudaMemset(p->s2.chain_len, 0, sizeof(int32_t)));
-    CK(cudaMemset(p->s2.wp_len, 0, sizeof(int64_t)));
-    CK(cudaMemset(p->s1.status, 0, sizeof(int32_t)));
+    CK(cudaMemset(p->s2.diag_count, 0, sizeof(int32_t) * (g.n1 + g.n2)));
     // backpointer words stage 1 never writes (past a tile's rows or steps)
     // read as 0, so that two plans' arrays compare equal
     CK(cudaMemset(p->s1.Bw, 0, (size_t)nt * g.b_words * sizeof(uint32_t)));
@@ -598,7 +603,7 @@ extern "C" int pfx_stage2_edges(pfx_plan* p, const double* C, int64_t ldc, void*
 
 extern "C" int pfx_stage2_prop(pfx_plan* p, void* stream) {
     if (!p) return fail(PFX_ERR_ARG, "null plan");
-    CK(launch_stage2_prop(p->g, p->s2, (cudaStream_t)stream));
+    CK(launch_stage2_prop(S2Pair{p->g, p->s2, 0}, nullptr, 1, (cudaStream_t)stream));
     return PFX_OK;
 }
 
@@ -616,7 +621,7 @@ extern "C" int pfx_snapshot_prop(pfx_plan* p, void* stream) {
     return PFX_OK;
 }
 
-static int64_t buffer_global(int64_t N, int64_t M, double beta) {
+int64_t pfx::buffer_global(int64_t N, int64_t M, double beta) {
     // Parflex.py:1520, evaluated in the same order
     const double mn = (double)(N < M ? N : M), mx = (double)(N < M ? M : N);
     const double bg = mn * (1 - (1 - beta) * mn / mx);
@@ -625,14 +630,16 @@ static int64_t buffer_global(int64_t N, int64_t M, double beta) {
 
 extern "C" int pfx_stage2_scan(pfx_plan* p, double beta, void* stream) {
     if (!p) return fail(PFX_ERR_ARG, "null plan");
-    CK(launch_sync_scan(p->g, p->s2, buffer_global(p->g.N, p->g.M, beta), (cudaStream_t)stream));
+    CK(launch_sync_scan(S2Pair{p->g, p->s2, buffer_global(p->g.N, p->g.M, beta)}, nullptr, 1,
+                        (cudaStream_t)stream));
     return PFX_OK;
 }
 
 extern "C" int pfx_stage2_stitch(pfx_plan* p, int from_best, int64_t i, int64_t j, int64_t edge,
                                  int64_t idx, void* stream) {
     if (!p) return fail(PFX_ERR_ARG, "null plan");
-    CK(launch_stitch(p->g, p->s2, (cudaStream_t)stream, from_best, i, j, edge, idx));
+    CK(launch_stitch(S2Pair{p->g, p->s2, 0}, nullptr, 1, (cudaStream_t)stream, from_best, i, j,
+                     edge, idx));
     return PFX_OK;
 }
 
@@ -674,22 +681,26 @@ extern "C" int pfx_result(pfx_plan* p, void* stream, double* best_cost, int64_t*
                           int64_t* wp_len) {
     if (!p) return fail(PFX_ERR_ARG, "null plan");
     cudaStream_t s = (cudaStream_t)stream;
-    double b = 0;
-    int64_t e[7];
-    int64_t n = 0;
-    int32_t kst = 0;
-    CK(cudaMemcpyAsync(&kst, p->s1.status, 4, cudaMemcpyDeviceToHost, s));
-    CK(cudaMemcpyAsync(&b, p->s2.best, 8, cudaMemcpyDeviceToHost, s));
-    CK(cudaMemcpyAsync(e, p->s2.best_end, 56, cudaMemcpyDeviceToHost, s));
-    CK(cudaMemcpyAsync(&n, p->s2.wp_len, 8, cudaMemcpyDeviceToHost, s));
+    if (!p->res_host) CK(cudaMallocHost(&p->res_host, 11 * sizeof(int64_t)));
+    int64_t* h = p->res_host;
+    CK(cudaMemcpyAsync(h, p->res, 10 * sizeof(int64_t), cudaMemcpyDeviceToHost, s));
+    // (a batch's plans share the batch's status word)
+    if (p->s1.status != reinterpret_cast<int32_t*>(p->res + 9))
+        CK(cudaMemcpyAsync(h + 9, p->s1.status, 4, cudaMemcpyDeviceToHost, s));
     CK(cudaStreamSynchronize(s));
+    int32_t kst;
+    memcpy(&kst, h + 9, 4);
     if (kst) {
         cudaMemsetAsync(p->s1.status, 0, 4, s);
         return fail(PFX_ERR_CUDA, "a bounded device wait ran out (status %d: 1 stage-1 wavefront, 2 cost GEMM); results invalid",
                     kst);
     }
+    double b;
+    memcpy(&b, h, 8);
+    const int64_t* e = h + 1;
+    const int64_t n = p->last_len = h[8];
     if (best_cost) *best_cost = b;
-    if (best_end7) memcpy(best_end7, e, sizeof(e));
+    if (best_end7) memcpy(best_end7, e, 7 * sizeof(int64_t));
     if (wp_len) *wp_len = n;
     if (!e[6]) return fail(PFX_ERR_NO_ENDPOINT, "%s", kStatus[PFX_ERR_NO_ENDPOINT]);
     return PFX_OK;
@@ -698,12 +709,32 @@ extern "C" int pfx_result(pfx_plan* p, void* stream, double* best_cost, int64_t*
 extern "C" int pfx_copy_path(pfx_plan* p, void* stream, int64_t* wp_host, int64_t cap) {
     if (!p || !wp_host) return fail(PFX_ERR_ARG, "null argument");
     cudaStream_t s = (cudaStream_t)stream;
-    int64_t n = 0;
-    CK(cudaMemcpyAsync(&n, p->s2.wp_len, 8, cudaMemcpyDeviceToHost, s));
-    CK(cudaStreamSynchronize(s));
-    if (n > cap) return fail(PFX_ERR_ARG, "path has %lld points, buffer holds %lld", (long long)n, (long long)cap);
-    if (n > 0) CK(cudaMemcpyAsync(wp_host, p->s2.wp, (size_t)n * 16, cudaMemcpyDeviceToHost, s));
-    CK(cudaStreamSynchronize(s));
+    if (!p->res_host) CK(cudaMallocHost(&p->res_host, 11 * sizeof(int64_t)));
+    int64_t* hn = p->res_host + 10;
+    // The length pfx_result last saw, and that many points, in one go; again
+    // with the right length in the rare case of another stitch since then.
+    // Through page-locked memory: a copy to pageable memory takes longer than
+    // both copies.
+    int64_t n = p->last_len <= cap ? p->last_len : 0;
+    for (;;) {
+        if (n > p->path_cap) {
+            cudaFreeHost(p->path_host);
+            p->path_host = nullptr;
+            p->path_cap = 0;
+            CK(cudaMallocHost(&p->path_host, (size_t)(n + n / 4 + 64) * 16));
+            p->path_cap = n + n / 4 + 64;
+        }
+        CK(cudaMemcpyAsync(hn, p->s2.wp_len, 8, cudaMemcpyDeviceToHost, s));
+        if (n > 0)
+            CK(cudaMemcpyAsync(p->path_host, p->s2.wp, (size_t)n * 16, cudaMemcpyDeviceToHost, s));
+        CK(cudaStreamSynchronize(s));
+        if (*hn > cap)
+            return fail(PFX_ERR_ARG, "path has %lld points, buffer holds %lld", (long long)*hn,
+                        (long long)cap);
+        if (*hn <= n) break;
+        n = *hn;
+    }
+    memcpy(wp_host, p->path_host, (size_t)*hn * 16);
     return PFX_OK;
 }
 

@@ -196,6 +196,8 @@ struct S2Buf {
     int64_t seg_cap;
     int64_t* wp;         // [K][2] final path, start first
     int64_t* wp_len;     // [1]
+    int2* diag_list;     // dependent slots by tile anti-diagonal (k_valid_lists)
+    int32_t* diag_count; // [n1 + n2 - 1], zero between launches
     const int32_t* tile_slot;  // [n1*n2] cost slab of each tile, -1 where stage 1
                                // skipped the tile (null: slab = tile index)
 };
@@ -310,10 +312,8 @@ cudaError_t launch_stage1(const double* C, const Geo& g, const S1Out& o, int til
 size_t stage1_smem_bytes_host(int32_t L, int nw);
 int stage1_pick_warps(const Geo& g, int num_sms);
 cudaError_t launch_fill(double* p, int64_t n, double v, cudaStream_t st);
-cudaError_t launch_stage2(const double* C, const void* Csk, int64_t skew_stride, bool f32,
-                          const Geo& g, const S2Buf& b, cudaStream_t st);
-// launch_stage2 in two parts: the edge tensors (the only part that reads the
-// cost slabs) and the cross-tile propagation.
+// Stage 2, first part: the edge tensors and valid marks (the only part that
+// reads the cost slabs).
 // With An (normalised features, [d][N] and [d][M]) the overlap costs are
 // computed from the features in the cost kernels' order, not read from C or
 // the slabs (a batch whose stage 1 built its cost itself keeps no slabs).
@@ -321,10 +321,20 @@ cudaError_t launch_stage2_edges(const double* C, const void* Csk, int64_t skew_s
                                 const Geo& g, const S2Buf& b, cudaStream_t st,
                                 const double* An = nullptr, const double* Bn = nullptr,
                                 int d = 0);
-cudaError_t launch_stage2_prop(const Geo& g, const S2Buf& b, cudaStream_t st);
-cudaError_t launch_sync_scan(const Geo& g, const S2Buf& b, int64_t buf, cudaStream_t st);
-cudaError_t launch_stitch(const Geo& g, const S2Buf& b, cudaStream_t st, int from_best,
-                          int64_t si, int64_t sj, int64_t se, int64_t sx);
+// One alignment of a stage-2 launch (buf: the scan's global buffer).
+struct S2Pair {
+    Geo g;
+    S2Buf b;
+    int64_t buf;
+};
+// The rest of stage 2, of one alignment (tab null) or of the npairs in the
+// device table tab; `one` then holds the largest n1, n2, L, N and M of the
+// table, which size the launches.  Propagation; overlap sync and edge scan;
+// stitched backtrace.
+cudaError_t launch_stage2_prop(const S2Pair& one, const S2Pair* tab, int npairs, cudaStream_t st);
+cudaError_t launch_sync_scan(const S2Pair& one, const S2Pair* tab, int npairs, cudaStream_t st);
+cudaError_t launch_stitch(const S2Pair& one, const S2Pair* tab, int npairs, cudaStream_t st,
+                          int from_best, int64_t si, int64_t sj, int64_t se, int64_t sx);
 // The tile chain of the stitched backtrace alone (b.chain, b.chain_len): it
 // reads only the start encodings on the tile edges, never the backpointers.
 cudaError_t launch_stitch_chain(const Geo& g, const S2Buf& b, cudaStream_t st, int from_best,

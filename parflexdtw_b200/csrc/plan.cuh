@@ -14,6 +14,11 @@ struct pfx_plan {
     size_t bytes;
     pfx::S1Out s1;
     pfx::S2Buf s2;
+    int64_t* res;        // device result block: best, end (7), path length, status
+    int64_t* res_host;   // page-locked copy, and the path length of pfx_copy_path
+    int64_t last_len;    // path length pfx_result last returned
+    void* path_host;     // page-locked staging of pfx_copy_path (path_cap points)
+    int64_t path_cap;
     double* D_prop;
     double* L_prop;
     int64_t n4;  // n1*n2*2*L
@@ -71,4 +76,6 @@ inline int64_t plan_slab_bytes(const pfx_plan* p) {
     return slabs * p->skew_stride * (p->fp32 ? 4 : 8);
 }
 int num_sms_cur();
+// The scan's global buffer (Parflex.py:1520).
+int64_t buffer_global(int64_t N, int64_t M, double beta);
 }  // namespace pfx
