@@ -3,6 +3,7 @@
 #include <stdio.h>
 
 #include <algorithm>
+#include <mutex>
 #include <atomic>
 #include <stdlib.h>
 #include <string.h>
@@ -358,6 +359,31 @@ extern "C" int pfx_plan_buffer(pfx_plan* p, int which, void** ptr, int64_t* nbyt
         default: return fail(PFX_ERR_ARG, "unknown buffer id %d", which);
     }
     return PFX_OK;
+}
+
+cudaError_t pfx::scratch_alloc(void** p, size_t bytes, cudaStream_t st) {
+    static std::mutex mu;
+    static cudaMemPool_t pools[64] = {};
+    int dev = 0;
+    cudaError_t e = cudaGetDevice(&dev);
+    if (e != cudaSuccess) return e;
+    if (dev < 0 || dev >= 64) return cudaMallocAsync(p, bytes, st);
+    cudaMemPool_t pool;
+    {
+        std::lock_guard<std::mutex> lock(mu);
+        if (!pools[dev]) {
+            cudaMemPoolProps props = {};
+            props.allocType = cudaMemAllocationTypePinned;
+            props.location.type = cudaMemLocationTypeDevice;
+            props.location.id = dev;
+            uint64_t keep = 256ull << 20;
+            if ((e = cudaMemPoolCreate(&pool, &props)) != cudaSuccess) return e;
+            cudaMemPoolSetAttribute(pool, cudaMemPoolAttrReleaseThreshold, &keep);
+            pools[dev] = pool;
+        }
+        pool = pools[dev];
+    }
+    return cudaMallocFromPoolAsync(p, bytes, pool, st);
 }
 
 static int check_ldc(const pfx_plan* p, const double* C, int64_t ldc) {

@@ -522,86 +522,202 @@ __device__ __forceinline__ float dz_at(const float* dy, const float* y, int relu
     return relu ? (y[i] > 0.f ? dy[i] : 0.f) : dy[i];
 }
 
-// Backward, data: dx[ci][iy][ix] = sum_{co, tap} w[co][ci][tap] dz[co][oy][ox]
-// over the outputs whose window covers (iy, ix).  One thread per input pixel.
-template <int S>
-__global__ void k_conv3x3_bwd_data(const float* __restrict__ w, int Cin, int H, int W, int Cout,
-                                   int Ho, int Wo, const float* __restrict__ y,
-                                   const float* __restrict__ dy, int relu, float* __restrict__ dx) {
+// The backward pass of a convolution works on the output pixels at which some
+// channel's dz is not 0.  In training they are few: a tile's score is one
+// logit, so dz of the last layer has one pixel per tile, the layer before it 9
+// per tile, and so on.  k_dz_pixels lists them (in no order) and marks them in
+// a map; dw and dx then skip everything else, and cost no more than a dense
+// pass where every pixel is listed.  (A listed pixel is one whose dz is not
+// equal to 0: NaN counts.)
+__global__ void __launch_bounds__(256) k_dz_pixels(const float* __restrict__ y,
+                                                   const float* __restrict__ dy, int relu,
+                                                   int Cout, int64_t npix,
+                                                   uint8_t* __restrict__ map,
+                                                   int32_t* __restrict__ list,
+                                                   int32_t* __restrict__ count) {
     const int64_t q = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-    if (q >= (int64_t)Cin * H * W) return;
-    const int ix = (int)(q % W), iy = (int)((q / W) % H), ci = (int)(q / ((int64_t)W * H));
-    float acc = 0.f;
-    for (int ky = 0; ky < 3; ++ky) {
-        const int ty = iy + 1 - ky;  // = oy * S
-        if (ty < 0 || ty % S) continue;
-        const int oy = ty / S;
-        if (oy >= Ho) continue;
-        for (int kx = 0; kx < 3; ++kx) {
-            const int tx = ix + 1 - kx;
-            if (tx < 0 || tx % S) continue;
-            const int ox = tx / S;
-            if (ox >= Wo) continue;
+    bool on = false;
+    if (q < npix) {
+#pragma unroll 16
+        for (int co = 0; co < Cout; ++co) on |= !(dz_at(dy, y, relu, co * npix + q) == 0.f);
+        map[q] = on;
+    }
+    const unsigned m = __ballot_sync(0xffffffffu, on);
+    const int lane = threadIdx.x & 31;
+    int at = 0;
+    if (lane == 0 && m) at = atomicAdd(count, __popc(m));
+    at = __shfl_sync(0xffffffffu, at, 0) + __popc(m & ((1u << lane) - 1u));
+    if (on) list[at] = (int32_t)q;
+}
+
+// Backward, data: dx[ci][iy][ix] = sum_{co, tap} w[co][ci][tap] dz[co][oy][ox]
+// over the outputs whose window covers (iy, ix).  One thread per input pixel
+// and 32 input channels, the weights in shared memory as [tap][co][ci]; a CTA
+// none of whose pixels is covered by a listed output stores zeros.  Bound by
+// the store of dx.  Layer 2 of the proposer (32 -> 32, stride 2, 313 x 360):
+// one thread per dx value, every output read, took 443 us.
+constexpr int kBdCi = 32;
+
+template <int S>
+__global__ void __launch_bounds__(256)
+    k_conv3x3_bwd_data(const float* __restrict__ w, int Cin, int H, int W, int Cout, int Ho,
+                       int Wo, const float* __restrict__ y, const float* __restrict__ dy,
+                       int relu, const uint8_t* __restrict__ map, float* __restrict__ dx) {
+    extern __shared__ __align__(16) float ws[];  // [9][Cout][32]
+    const int64_t npix = (int64_t)H * W;
+    const int64_t q = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+    const int ci0 = blockIdx.y * kBdCi, nci = min(kBdCi, Cin - ci0);
+    const int ix = (int)(q % W), iy = (int)(q / W);
+    // the outputs (oy, ox) = ((iy + 1 - ky) / S, ...) of each tap, where listed
+    unsigned taps = 0;
+    if (q < npix) {
+#pragma unroll
+        for (int tap = 0; tap < 9; ++tap) {
+            const int ty = iy + 1 - tap / 3, tx = ix + 1 - tap % 3;
+            if (ty < 0 || tx < 0 || ty % S || tx % S || ty / S >= Ho || tx / S >= Wo) continue;
+            if (map[(int64_t)(ty / S) * Wo + tx / S]) taps |= 1u << tap;
+        }
+    }
+    float acc[kBdCi];
+#pragma unroll
+    for (int c = 0; c < kBdCi; ++c) acc[c] = 0.f;
+    if (__syncthreads_or(taps != 0)) {
+        for (int i = threadIdx.x; i < 9 * Cout * kBdCi; i += blockDim.x) {
+            const int c = i % kBdCi, co = i / kBdCi % Cout, tap = i / kBdCi / Cout;
+            ws[i] = c < nci ? w[((int64_t)co * Cin + ci0 + c) * 9 + tap] : 0.f;
+        }
+        __syncthreads();
+        for (int tap = 0; tap < 9; ++tap) {
+            if (!(taps >> tap & 1u)) continue;
+            const int oy = (iy + 1 - tap / 3) / S, ox = (ix + 1 - tap % 3) / S;
+            // (several outputs' dz at once in flight)
+#pragma unroll 8
             for (int co = 0; co < Cout; ++co) {
-                const int64_t oi = ((int64_t)co * Ho + oy) * Wo + ox;
-                acc = fmaf(w[((int64_t)co * Cin + ci) * 9 + ky * 3 + kx], dz_at(dy, y, relu, oi),
-                           acc);
+                const float dz = dz_at(dy, y, relu, ((int64_t)co * Ho + oy) * Wo + ox);
+                const float4* w4 = reinterpret_cast<const float4*>(ws + (tap * Cout + co) * kBdCi);
+#pragma unroll
+                for (int c4 = 0; c4 < kBdCi / 4; ++c4) {
+                    const float4 v = w4[c4];
+                    acc[4 * c4 + 0] = fmaf(v.x, dz, acc[4 * c4 + 0]);
+                    acc[4 * c4 + 1] = fmaf(v.y, dz, acc[4 * c4 + 1]);
+                    acc[4 * c4 + 2] = fmaf(v.z, dz, acc[4 * c4 + 2]);
+                    acc[4 * c4 + 3] = fmaf(v.w, dz, acc[4 * c4 + 3]);
+                }
             }
         }
     }
-    dx[q] = acc;
+    if (q >= npix) return;
+#pragma unroll
+    for (int c = 0; c < kBdCi; ++c)
+        if (c < nci) dx[(int64_t)(ci0 + c) * npix + q] = acc[c];
 }
 
 // Backward, weights and bias: dw[co][ci][tap] += sum_pixels dz * x, db[co] +=
-// sum dz.  A CTA takes a 16 x 16 output tile and a chunk of 8 input
-// channels; per-CTA partial sums go to global memory with atomics.
-constexpr int kWgCi = 8;
+// sum dz over the listed pixels: the product of dz^T (32 x pixels) and the
+// input patches (pixels x 9 * 32).  A CTA takes up to 32 output and 32 input
+// channels and every gridDim.x-th batch of pixels, staged in shared memory; a
+// thread keeps 4 output channels x 9 taps of an input channel; with fewer
+// input channels the threads' slices of the batch are added up at the end.
+// Few CTAs, because each ends with an atomic per weight.  The proposer's
+// layers 2 and 1 (a CTA per 16 x 16 outputs and 8 input channels, every pixel):
+// 338 and 104 us.
+constexpr int kWgPix = 16;   // pixels per batch
+constexpr int kWgCtas = 64;
 
 template <int S>
 __global__ void __launch_bounds__(256)
     k_conv3x3_bwd_weight(const float* __restrict__ x, int Cin, int H, int W, int Cout, int Ho,
                          int Wo, const float* __restrict__ y, const float* __restrict__ dy,
-                         int relu, float* __restrict__ dw, float* __restrict__ db) {
-    constexpr int PT = (kCvT - 1) * S + 3;
-    extern __shared__ float sm[];
-    float* dz = sm;                          // [Cout][256]
-    float* patch = sm + Cout * kCvT * kCvT;  // [kWgCi][PT*PT]
-    const int ox0 = blockIdx.x * kCvT, oy0 = blockIdx.y * kCvT, ci0 = blockIdx.z * kWgCi;
-    const int nci = min(kWgCi, Cin - ci0);
-    for (int q = threadIdx.x; q < Cout * kCvT * kCvT; q += 256) {
-        const int co = q / (kCvT * kCvT), p = q % (kCvT * kCvT);
-        const int ox = ox0 + p % kCvT, oy = oy0 + p / kCvT;
-        dz[q] = (ox < Wo && oy < Ho) ? dz_at(dy, y, relu, ((int64_t)co * Ho + oy) * Wo + ox) : 0.f;
+                         int relu, const int32_t* __restrict__ list,
+                         const int32_t* __restrict__ count, float* __restrict__ dw,
+                         float* __restrict__ db) {
+    __shared__ float xs[kWgPix * 32 * 9];          // [pixel][ci][tap]
+    __shared__ __align__(16) float dzs[kWgPix][32];  // [pixel][co]
+    __shared__ int2 at[kWgPix];                      // input row, column of tap 0
+    const int n = *count;
+    const int ci0 = blockIdx.y * 32, co0 = blockIdx.z * 32;
+    const int nci = min(32, Cin - ci0), nco = min(32, Cout - co0);
+    const int per = 8 * nci, slices = 256 / per;
+    const int slice = threadIdx.x / per, cg = threadIdx.x % per / nci, ci = threadIdx.x % nci;
+    const bool act = slice < slices;
+    float acc[4][9], accb[4];
+#pragma unroll
+    for (int c = 0; c < 4; ++c) {
+        accb[c] = 0.f;
+#pragma unroll
+        for (int t = 0; t < 9; ++t) acc[c][t] = 0.f;
     }
-    const int ix0 = ox0 * S - 1, iy0 = oy0 * S - 1;
-    for (int q = threadIdx.x; q < nci * PT * PT; q += 256) {
-        const int c = q / (PT * PT), r = q % (PT * PT);
-        const int iy = iy0 + r / PT, ix = ix0 + r % PT;
-        patch[q] = (iy >= 0 && iy < H && ix >= 0 && ix < W)
-                       ? x[((int64_t)(ci0 + c) * H + iy) * W + ix]
-                       : 0.f;
+    for (int p0 = blockIdx.x * kWgPix; p0 < n; p0 += gridDim.x * kWgPix) {
+        const int np = min(kWgPix, n - p0);
+        __syncthreads();  // the previous batch is consumed
+        if (threadIdx.x < np) {
+            const int pix = list[p0 + threadIdx.x];
+            at[threadIdx.x] = make_int2(pix / Wo * S - 1, pix % Wo * S - 1);
+        }
+        __syncthreads();
+        for (int q = threadIdx.x; q < nci * 9; q += 256) {
+            const int c = q / 9, ky = q % 9 / 3, kx = q % 3;
+            const float* xc = x + (int64_t)(ci0 + c) * H * W;
+#pragma unroll 8
+            for (int p = 0; p < np; ++p) {
+                const int iy = at[p].x + ky, ix = at[p].y + kx;
+                xs[p * nci * 9 + q] = (iy >= 0 && iy < H && ix >= 0 && ix < W)
+                                          ? xc[(int64_t)iy * W + ix]
+                                          : 0.f;
+            }
+        }
+        for (int q = threadIdx.x; q < np * 32; q += 256) {
+            const int p = q >> 5, c = q & 31;
+            dzs[p][c] = c < nco ? dz_at(dy, y, relu,
+                                        (int64_t)(co0 + c) * Ho * Wo + list[p0 + p])
+                                : 0.f;
+        }
+        __syncthreads();
+        if (!act) continue;
+        for (int p = slice; p < np; p += slices) {
+            const float4 d4 = *reinterpret_cast<const float4*>(&dzs[p][4 * cg]);
+            const float d[4] = {d4.x, d4.y, d4.z, d4.w};
+            const float* xp = xs + (p * nci + ci) * 9;
+#pragma unroll
+            for (int t = 0; t < 9; ++t) {
+                const float xv = xp[t];
+#pragma unroll
+                for (int c = 0; c < 4; ++c) acc[c][t] = fmaf(d[c], xv, acc[c][t]);
+            }
+#pragma unroll
+            for (int c = 0; c < 4; ++c) accb[c] += d[c];
+        }
     }
+    if (blockIdx.x * kWgPix >= n) return;
+    // the slices' sums, in shared memory where there are several
     __syncthreads();
-    const int ncomb = Cout * nci * 9;
-    for (int cmb = threadIdx.x; cmb < ncomb; cmb += 256) {
-        const int tap = cmb % 9, c = (cmb / 9) % nci, co = cmb / (9 * nci);
-        const int ky = tap / 3, kx = tap % 3;
-        const float* dzc = dz + co * kCvT * kCvT;
-        const float* pc = patch + c * PT * PT;
-        float acc = 0.f;
-        for (int p = 0; p < kCvT * kCvT; ++p) {
-            const int py = p / kCvT, px = p % kCvT;
-            acc = fmaf(dzc[p], pc[(py * S + ky) * PT + px * S + kx], acc);
-        }
-        atomicAdd(dw + ((int64_t)co * Cin + ci0 + c) * 9 + tap, acc);
+    if (slices > 1) {
+        for (int q = threadIdx.x; q < 32 * nci * 9; q += 256) xs[q] = 0.f;
+        for (int q = threadIdx.x; q < 32; q += 256) dzs[0][q] = 0.f;
+        __syncthreads();
     }
-    if (blockIdx.z == 0) {
-        for (int co = threadIdx.x; co < Cout; co += 256) {
-            float acc = 0.f;
-            for (int p = 0; p < kCvT * kCvT; ++p) acc += dz[co * kCvT * kCvT + p];
-            atomicAdd(db + co, acc);
+    if (act) {
+#pragma unroll
+        for (int c = 0; c < 4; ++c) {
+            const int co = 4 * cg + c;
+            if (co >= nco) continue;
+            if (slices > 1) {
+#pragma unroll
+                for (int t = 0; t < 9; ++t) atomicAdd(&xs[(co * nci + ci) * 9 + t], acc[c][t]);
+                if (ci == 0) atomicAdd(&dzs[0][co], accb[c]);
+            } else {
+#pragma unroll
+                for (int t = 0; t < 9; ++t)
+                    atomicAdd(dw + ((int64_t)(co0 + co) * Cin + ci0 + ci) * 9 + t, acc[c][t]);
+                if (ci == 0 && ci0 == 0) atomicAdd(db + co0 + co, accb[c]);
+            }
         }
     }
+    if (slices <= 1) return;
+    __syncthreads();
+    for (int q = threadIdx.x; q < nco * nci * 9; q += 256)
+        atomicAdd(dw + ((int64_t)(co0 + q / (nci * 9)) * Cin + ci0) * 9 + q % (nci * 9), xs[q]);
+    for (int q = threadIdx.x; q < nco && ci0 == 0; q += 256) atomicAdd(db + co0 + q, dzs[0][q]);
 }
 
 // Tile scores: the max logit over each tile's region of the logit map
@@ -934,22 +1050,38 @@ static cudaError_t conv_bwd_t(const float* x, int Cin, int H, int W, const float
                               const float* y, int relu, const float* dy, float* dx, float* dw,
                               float* db, cudaStream_t st) {
     const int Ho = (H - 1) / S + 1, Wo = (W - 1) / S + 1;
-    if (dx) {
-        const int64_t n = (int64_t)Cin * H * W;
-        k_conv3x3_bwd_data<S><<<blocks_for(n, 256), 256, 0, st>>>(w, Cin, H, W, Cout, Ho, Wo, y,
-                                                                 dy, relu, dx);
-        count_launches(1);
-    }
-    const dim3 grid(blocks_for(Wo, kCvT), blocks_for(Ho, kCvT), blocks_for(Cin, kWgCi));
-    constexpr int PT = (kCvT - 1) * S + 3;
-    const size_t smem = ((size_t)Cout * kCvT * kCvT + (size_t)kWgCi * PT * PT) * sizeof(float);
-    cudaError_t e = cudaFuncSetAttribute(k_conv3x3_bwd_weight<S>,
-                                         cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    const int64_t npix = (int64_t)Ho * Wo;
+    // the listed pixels: count, list, map
+    char* tmp = nullptr;
+    cudaError_t e = scratch_alloc((void**)&tmp, 16 + (size_t)npix * 5, st);
     if (e != cudaSuccess) return e;
-    k_conv3x3_bwd_weight<S><<<grid, 256, smem, st>>>(x, Cin, H, W, Cout, Ho, Wo, y, dy, relu, dw,
-                                                     db);
-    count_launches(1);
-    return cudaGetLastError();
+    int32_t* count = reinterpret_cast<int32_t*>(tmp);
+    int32_t* list = reinterpret_cast<int32_t*>(tmp + 16);
+    uint8_t* map = reinterpret_cast<uint8_t*>(list + npix);
+    e = cudaMemsetAsync(count, 0, 4, st);
+    if (e == cudaSuccess) {
+        k_dz_pixels<<<blocks_for(npix, 256), 256, 0, st>>>(y, dy, relu, Cout, npix, map, list,
+                                                           count);
+        const dim3 gw(kWgCtas, blocks_for(Cin, 32), blocks_for(Cout, 32));
+        k_conv3x3_bwd_weight<S><<<gw, 256, 0, st>>>(x, Cin, H, W, Cout, Ho, Wo, y, dy, relu, list,
+                                                    count, dw, db);
+        count_launches(2);
+        e = cudaGetLastError();
+    }
+    if (e == cudaSuccess && dx) {
+        const size_t sm = sizeof(float) * 9 * Cout * kBdCi;
+        e = cudaFuncSetAttribute(k_conv3x3_bwd_data<S>,
+                                 cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
+        if (e == cudaSuccess) {
+            const dim3 gd(blocks_for((int64_t)H * W, 256), blocks_for(Cin, kBdCi));
+            k_conv3x3_bwd_data<S><<<gd, 256, sm, st>>>(w, Cin, H, W, Cout, Ho, Wo, y, dy, relu,
+                                                       map, dx);
+            count_launches(1);
+            e = cudaGetLastError();
+        }
+    }
+    const cudaError_t ef = cudaFreeAsync(tmp, st);
+    return e != cudaSuccess ? e : ef;
 }
 
 cudaError_t cnn_conv_backward(const float* x, int Cin, int H, int W, const float* w, int Cout,
