@@ -239,6 +239,11 @@ cudaError_t launch_compact_descs(const TileDesc* in, int n, const uint8_t* mask,
 // warps each, claimed through *head; for alignments with few tiles.
 cudaError_t launch_stage1_cluster(int cn, int cw, const TileDesc* descs, int ntiles, int* head,
                                   const Geo& g, int32_t* status, bool fp32, cudaStream_t st);
+// FlexDTW of one R x W tile (g.N x g.M, g.L >= both) of a row-major cost with
+// all of D, P and B as outputs, on a cluster; *done false where it takes the
+// other way (launch_stage1): no scratch memory, or rings that do not fit.
+cudaError_t launch_tile_full(const double* C, const Geo& g, double* D, int32_t* P, int8_t* B,
+                             cudaStream_t st, bool* done);
 // Clusters of that kernel that can run at once on this device (0: none).
 int stage1_cluster_max(int cn, int cw, const Geo& g, bool fp32);
 // Whether the queue kernel's rings fit at tile length L with nw warps per

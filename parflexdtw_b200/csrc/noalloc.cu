@@ -7,8 +7,9 @@
 // device-wide synchronisation that cudaMalloc / cudaFree can cause, once per
 // block; a host application or plugin framework that reserves all device
 // memory up front may forbid the library from allocating at all.
-// pfx_flexdtw_tile allocates the kernel's scratch (tile edge rows and packed
-// backpointers) with cudaMallocAsync on every call; this variant keeps that
+// pfx_flexdtw_tile allocates its scratch (for a small or narrow tile the edge
+// rows and packed backpointers, else skewed copies of the tile too) with
+// cudaMallocAsync on every call; this variant runs the one-CTA kernel with its
 // scratch in one file-scope device array instead.
 //
 // Limits and sharing:

@@ -19,6 +19,8 @@
 // bounded and a warp that gives up goes on to the tile's end barrier.
 #include <cooperative_groups.h>
 
+#include <string.h>
+
 #include <algorithm>
 #include <utility>
 #include <vector>
@@ -47,10 +49,13 @@ __device__ __forceinline__ bool wait_progress_cl(const int* p, int target,
     return false;
 }
 
-template <int CW, bool STD, typename T, int QD>
+// FULL: every cell's D takes its cost's place in the slab and its internal start
+// encoding (Wave) goes to Psk in the same layout (the single-tile call).
+template <int CW, bool STD, typename T, int QD, bool FULL>
 __global__ void __launch_bounds__(CW * 32, 1)
     k_stage1_cl(const TileDesc* __restrict__ descs, const int ntiles, int* __restrict__ head,
-                const Geo g, int32_t* __restrict__ status, const int RB, const int queue_at) {
+                const Geo g, int32_t* __restrict__ status, const int RB, const int queue_at,
+                int2* __restrict__ Psk) {
     using V2 = typename Vec2<T>::type;
     namespace cg = cooperative_groups;
     cg::cluster_group cl = cg::this_cluster();
@@ -163,7 +168,12 @@ __global__ void __launch_bounds__(CW * 32, 1)
                 if (lane == 0 && b.tau0 + 2 * kBlk <= sc.span)
                     prefetch_next_block(Ct + (int64_t)k * sc.span * 32, b.tau0 + kBlk);
                 if (b.tau0 == 0) queue_start<QD, T>(st.q, b.Cs);
-                run_block<STD, true, T, QD>(g, st, b, td, sc.nS, &bw);
+                if (FULL) {
+                    const int64_t at = ((int64_t)k * sc.span + b.tau0) * 32 + lane;
+                    b.oD = const_cast<V2*>(Ct) + at;
+                    b.oP = Psk + at;
+                }
+                run_block<STD, true, FULL, T, QD>(g, st, b, td, sc.nS, &bw);
             }
             rs = ring_next(rs, RB);
             ws = ring_next(ws, RB);
@@ -196,9 +206,9 @@ struct ClConfig {
     S1Mem mem;
 };
 
-template <int CW, bool STD, typename T, int QD>
+template <int CW, bool STD, typename T, int QD, bool FULL>
 static cudaError_t cl_config(const S1Mem& m, int cn, int nclusters, ClConfig* c) {
-    auto kern = k_stage1_cl<CW, STD, T, QD>;
+    auto kern = k_stage1_cl<CW, STD, T, QD, FULL>;
     const cudaError_t e = cudaFuncSetAttribute(
         kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)m.bytes);
     if (e != cudaSuccess) return e;
@@ -217,12 +227,13 @@ static cudaError_t cl_config(const S1Mem& m, int cn, int nclusters, ClConfig* c)
 }
 
 // max != null: only the number of clusters that can run at once.
-template <int CW, bool STD, typename T, int QD>
+template <int CW, bool STD, typename T, int QD, bool FULL>
 static cudaError_t cl_launch(const S1Mem& m, int cn, const TileDesc* descs, int ntiles, int* head,
-                             const Geo& g, int32_t* status, cudaStream_t st, int* max) {
-    auto kern = k_stage1_cl<CW, STD, T, QD>;
+                             const Geo& g, int32_t* status, cudaStream_t st, int* max,
+                             int2* Psk = nullptr) {
+    auto kern = k_stage1_cl<CW, STD, T, QD, FULL>;
     ClConfig c;
-    cudaError_t e = cl_config<CW, STD, T, QD>(m, cn, 1, &c);
+    cudaError_t e = cl_config<CW, STD, T, QD, FULL>(m, cn, 1, &c);
     if (e != cudaSuccess) return e;
     int fit = 0;
     e = cudaOccupancyMaxActiveClusters(&fit, kern, &c.cfg);
@@ -236,7 +247,7 @@ static cudaError_t cl_launch(const S1Mem& m, int cn, const TileDesc* descs, int 
     if (n <= 0) return cudaSuccess;
     c.cfg.gridDim = dim3((unsigned)(cn * n));
     c.cfg.stream = st;
-    e = cudaLaunchKernelEx(&c.cfg, kern, descs, ntiles, head, g, status, m.rb, m.queue_at);
+    e = cudaLaunchKernelEx(&c.cfg, kern, descs, ntiles, head, g, status, m.rb, m.queue_at, Psk);
     count_launches(1);
     return e;
 }
@@ -250,8 +261,10 @@ static cudaError_t cl_dispatch(int cn, int cw, const TileDesc* descs, int ntiles
     if (m.rb == 0) return cudaErrorInvalidValue;
 #define PFX_CL(CW, QD)                                                                        \
     return std_steps                                                                          \
-               ? cl_launch<CW, true, T, QD>(m, cn, descs, ntiles, head, g, status, st, max)   \
-               : cl_launch<CW, false, T, QD>(m, cn, descs, ntiles, head, g, status, st, max)
+               ? cl_launch<CW, true, T, QD, false>(m, cn, descs, ntiles, head, g, status, st, \
+                                                  max)                                      \
+               : cl_launch<CW, false, T, QD, false>(m, cn, descs, ntiles, head, g, status,    \
+                                                   st, max)
     if (cw == 16) PFX_CL(16, 0);
     if (m.qd == 0) return cudaErrorInvalidValue;
     if (cw == 12) PFX_CL(12, 4);
@@ -265,6 +278,111 @@ cudaError_t launch_stage1_cluster(int cn, int cw, const TileDesc* descs, int nti
                                   const Geo& g, int32_t* status, bool fp32, cudaStream_t st) {
     return fp32 ? cl_dispatch<float>(cn, cw, descs, ntiles, head, g, status, st, nullptr)
                 : cl_dispatch<double>(cn, cw, descs, ntiles, head, g, status, st, nullptr);
+}
+
+// The tile's full outputs from the skewed ones: 32 rows x 64 columns per CTA
+// through shared memory (D and P in the cost's layout, codes from the packed
+// backpointers); P = 0 on row 0 and column 0, code 3 is -1. Where the DP's
+// waits ran out D is NaN, not a number that could pass for a result.
+__global__ void __launch_bounds__(256)
+    k_unskew(const double* __restrict__ Dsk, const int* __restrict__ Psk,
+             const uint32_t* __restrict__ Bw, const int32_t* __restrict__ status, int R, int W,
+             double* __restrict__ D, int32_t* __restrict__ P, int8_t* __restrict__ B) {
+    __shared__ double sd[32][65];
+    __shared__ int sp[32][65];
+    const bool failed = *status != 0;
+    const int span = ceil_div32(W + kStripRows - 1, kBlk) * kBlk;
+    const int k = blockIdx.y >> 1, h = (blockIdx.y & 1) * 32, c0 = blockIdx.x * 64;
+    for (int q = threadIdx.x; q < 95 * 32; q += 256) {
+        const int rho = q & 31, tau = c0 + h + (q >> 5), c = tau - h - rho - c0;
+        if (c < 0 || c >= 64 || tau >= span) continue;
+        const int64_t at = ((int64_t)k * span + tau) * 64 + h + rho;
+        sd[rho][c] = Dsk[at];
+        sp[rho][c] = Psk[at];
+    }
+    __syncthreads();
+    for (int q = threadIdx.x; q < 32 * 64; q += 256) {
+        const int x = q & 63, rho = h + (q >> 6), r = 64 * k + rho, c = c0 + x;
+        if (r >= R || c >= W) continue;
+        const int tau = c + rho;
+        const uint32_t word = __ldg(Bw + bp_word_index2(W, r, tau));
+        const int code = (int)((word >> ((tau & 15) * 2)) & 3u);
+        const int64_t at = (int64_t)r * W + c;
+        D[at] = failed ? __longlong_as_double(0x7ff8000000000000ll) : sd[rho - h][x];
+        P[at] = r == 0 || c == 0 ? 0 : sp[rho - h][x];
+        B[at] = (int8_t)(code == 3 ? -1 : code);
+    }
+}
+
+// A queue of one tile.
+__global__ void k_one_tile(const TileDesc d, TileDesc* __restrict__ out, int* __restrict__ head) {
+    *out = d;
+    head[0] = 0;
+    head[1] = 0;  // status
+}
+
+// One tile with all of D, P and B as row-major outputs: cost into the skewed
+// layout, the DP on one cluster with D written over the cost, and back.
+// Bound by the DP's chain of steps. Against one CTA that writes each cell's
+// values itself (stage1_f64.cu), 1500 x 1801: 9.4 ms of kernels -> 1.32 (DP
+// 1.26, the passes before and after it 0.06); its caller has the sizes.
+cudaError_t launch_tile_full(const double* C, const Geo& g, double* D, int32_t* P, int8_t* B,
+                             cudaStream_t st, bool* done) {
+    *done = false;
+    const int R = (int)g.N, W = (int)g.M;
+    const int nS = ceil_div32(R, kStripRows);
+    // as many warps as strips, four per SM up to 8 SMs, then eight
+    const int cw = nS > 48 ? 8 : 4;
+    int cn = 1;
+    while (cn < 8 && cn * cw < nS) cn *= 2;
+    Geo gt = g;
+    const Sched2 s = make_sched2(g.L, g.L, cn * cw);
+    const S1Mem m = stage1_mem(s.lag, cw, cta_budget(16), 8, 4);
+    if (m.rb == 0 || m.qd == 0) return cudaSuccess;
+    // scratch: slab, P, backpointers, edges, descriptor, queue head and status
+    auto up = [](size_t b) { return (b + 255) & ~(size_t)255; };
+    const size_t slab = up((size_t)nS * ceil_div32(W + kStripRows - 1, kBlk) * kBlk * 64 * 8);
+    const size_t bw = up((size_t)tile_b_words2(g.L) * 4), ed = up((size_t)2 * g.L * 12);
+    char* tmp = nullptr;
+    if (cudaMallocAsync((void**)&tmp, slab + slab / 2 + bw + ed + 512, st) != cudaSuccess) {
+        cudaGetLastError();  // no room: the caller's other way needs less
+        return cudaSuccess;
+    }
+    double* Dsk = reinterpret_cast<double*>(tmp);
+    int2* Psk = reinterpret_cast<int2*>(tmp + slab);
+    TileDesc d;
+    memset(&d, 0, sizeof(d));
+    d.Csk = Dsk;
+    d.Bw = reinterpret_cast<uint32_t*>(tmp + slab + slab / 2);
+    d.eD = reinterpret_cast<double*>(tmp + slab + slab / 2 + bw);
+    d.eP = reinterpret_cast<int32_t*>(d.eD + 2 * g.L);
+    d.R = R;
+    d.W = W;
+    d.L = g.L;
+    char* misc = tmp + slab + slab / 2 + bw + ed;
+    TileDesc* dd = reinterpret_cast<TileDesc*>(misc + 256);
+    int* head = reinterpret_cast<int*>(misc);
+    k_one_tile<<<1, 1, 0, st>>>(d, dd, head);
+    count_launches(1);
+    cudaError_t e = cudaGetLastError();
+    if (e == cudaSuccess) e = launch_relayout_skew(C, g.ldc, gt, Dsk, 0, st);
+    const bool std_steps = g.S == 3 && g.kind[0] == 0 && g.kind[1] == 1 && g.kind[2] == 2;
+#define PFX_FULL(CW)                                                                           \
+    (std_steps ? cl_launch<CW, true, double, 4, true>(m, cn, dd, 1, head, g, head + 1, st,     \
+                                                      nullptr, Psk)                            \
+               : cl_launch<CW, false, double, 4, true>(m, cn, dd, 1, head, g, head + 1, st,    \
+                                                       nullptr, Psk))
+    if (e == cudaSuccess) e = cw == 8 ? PFX_FULL(8) : PFX_FULL(4);
+#undef PFX_FULL
+    if (e == cudaSuccess) {
+        k_unskew<<<dim3((unsigned)ceil_div32(W, 64), (unsigned)(2 * nS)), 256, 0, st>>>(
+            Dsk, reinterpret_cast<const int*>(Psk), d.Bw, head + 1, R, W, D, P, B);
+        count_launches(1);
+        e = cudaGetLastError();
+    }
+    const cudaError_t ef = cudaFreeAsync(tmp, st);
+    *done = true;
+    return e != cudaSuccess ? e : ef;
 }
 
 int stage1_cluster_max(int cn, int cw, const Geo& g, bool fp32) {

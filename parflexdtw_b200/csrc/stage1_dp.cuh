@@ -336,6 +336,8 @@ struct Block {
     uint32_t kd;                       // D address is that times 2 (FP32 form: 1), + kd)
     typename Vec2<T>::type* pD;        // PUSH: the ring slot in a cluster peer's
     int2* pP;                          // shared memory, or null
+    typename Vec2<T>::type* oD;        // FULL: D and P of every cell at step tau0, this
+    int2* oP;                          // lane, in the cost's layout (oD may be the cost)
     uint32_t incW, incR;               // and their moves per two steps (ring lanes)
     int span, tau0, k, R, W, lane, nP;
 };
@@ -384,7 +386,7 @@ enum StripKind { kInner, kTop, kBottom };
 // step's parity.  kTop: strip 0 of several (row 0 is the cost itself, rows 1
 // and 2 have predecessors on it); kBottom: the last strip of several, whose
 // lanes past the last row count for nothing and whose last row is stored.
-template <StripKind KIND, bool PUSH, typename T, int QD>
+template <StripKind KIND, bool PUSH, bool FULL, typename T, int QD>
 __device__ __forceinline__ bool fast_step(Wave<T, QD>& st, const Block<T>& b, const int u, int t,
                                           T rc, T w0, T w1, T w2, double* eD, int32_t* eP,
                                           uint32_t& bitsA, uint32_t& bitsB) {
@@ -435,6 +437,10 @@ __device__ __forceinline__ bool fast_step(Wave<T, QD>& st, const Block<T>& b, co
             eP[c] = isA ? oAP : oBP;
         }
     }
+    if (FULL) {
+        b.oD[t * 32] = make_v2<T>(oAD, oBD);
+        b.oP[t * 32] = make_int2(oAP, oBP);
+    }
     bitsA = bitsA * 4 + codeA;  // the first step ends up highest
     bitsB = bitsB * 4 + codeB;
     st.m1A = addr(m0A, (T)1);
@@ -445,7 +451,7 @@ __device__ __forceinline__ bool fast_step(Wave<T, QD>& st, const Block<T>& b, co
 
 // The fast loop: steps 0 .. 15 of a block, or up to the first that needs the
 // exact routine.  Returns the steps done.
-template <StripKind KIND, bool PUSH, typename T, int QD>
+template <StripKind KIND, bool PUSH, bool FULL, typename T, int QD>
 __device__ __forceinline__ int fast_steps(Wave<T, QD>& st, Block<T>& b, const TileDesc& td, T& rc,
                                           T w0, T w1, T w2,
                                           const typename Vec2<T>::type*& cp, uint32_t& bitsA,
@@ -455,11 +461,13 @@ __device__ __forceinline__ int fast_steps(Wave<T, QD>& st, Block<T>& b, const Ti
     int t = 0;
 #pragma unroll 1
     for (; t < kBlk; t += 2) {
-        if (!fast_step<KIND, PUSH, T, QD>(st, b, 0, t, rc, w0, w1, w2, eD, eP, bitsA, bitsB))
+        if (!fast_step<KIND, PUSH, FULL, T, QD>(st, b, 0, t, rc, w0, w1, w2, eD, eP, bitsA,
+                                                bitsB))
             return t;
         queue_next<QD, T>(st.q, 0, t, cp, true);
         rc = addr(rc, (T)1);
-        if (!fast_step<KIND, PUSH, T, QD>(st, b, 1, t + 1, rc, w0, w1, w2, eD, eP, bitsA, bitsB))
+        if (!fast_step<KIND, PUSH, FULL, T, QD>(st, b, 1, t + 1, rc, w0, w1, w2, eD, eP, bitsA,
+                                                bitsB))
             return t + 1;
         queue_next<QD, T>(st.q, 1, t + 1, cp + 32, true);
         rc = addr(rc, (T)1);
@@ -478,7 +486,7 @@ __device__ __forceinline__ int fast_steps(Wave<T, QD>& st, Block<T>& b, const Ti
 // 0 or next to them may occur; mask: cells past the last row / column or on
 // it.  Outputs of cells outside the tile are arbitrary (nothing inside reads
 // them) but for their code, 0.
-template <bool STD, bool PUSH, typename T, int QD>
+template <bool STD, bool PUSH, bool FULL, typename T, int QD>
 __device__ __forceinline__ void careful_step(const Geo& g, Wave<T, QD>& st, const Block<T>& b,
                                              const TileDesc& td, const int u, int t,
                                              const bool rim, const bool mask, T rc,
@@ -540,6 +548,10 @@ __device__ __forceinline__ void careful_step(const Geo& g, Wave<T, QD>& st, cons
         if (actA) store_edges(td, rA, cA, b.R, b.W, oAD, oAP);
         if (actB) store_edges(td, rB, cB, b.R, b.W, oBD, oBP);
     }
+    if (FULL) {
+        b.oD[t * 32] = make_v2<T>(oAD, oBD);
+        b.oP[t * 32] = make_int2(oAP, oBP);
+    }
     bitsA = bitsA * 4 + (actA ? codeA : 0);
     bitsB = bitsB * 4 + (actB ? codeB : 0);
     st.m1A = addr(m0A, (T)1);
@@ -548,7 +560,7 @@ __device__ __forceinline__ void careful_step(const Geo& g, Wave<T, QD>& st, cons
 }
 
 // The careful loop: steps t .. 15 of a block.
-template <bool STD, bool PUSH, typename T, int QD>
+template <bool STD, bool PUSH, bool FULL, typename T, int QD>
 __device__ __forceinline__ void careful_steps(const Geo& g, Wave<T, QD>& st, Block<T>& b,
                                               const TileDesc& td, int t, const bool rim,
                                               const bool mask, T rc,
@@ -569,7 +581,8 @@ __device__ __forceinline__ void careful_steps(const Geo& g, Wave<T, QD>& st, Blo
         if constexpr (QD == 0) st.q.q[0] = st.q.q[1];
         // (the register queue's load goes before the step, which is long)
         if constexpr (QD == 0) queue_next<QD, T>(st.q, 1, t, cp, t < ahead);
-        careful_step<STD, PUSH, T, QD>(g, st, b, td, t & 1, t, rim, mask, rc, cc, bitsA, bitsB);
+        careful_step<STD, PUSH, FULL, T, QD>(g, st, b, td, t & 1, t, rim, mask, rc, cc, bitsA,
+                                             bitsB);
         if constexpr (QD > 0) queue_next<QD, T>(st.q, 1, t, cp, t < ahead);
         cp += 32;
         rc = addr(rc, (T)1);
@@ -606,7 +619,7 @@ __device__ __forceinline__ void careful_steps(const Geo& g, Wave<T, QD>& st, Blo
 // start encodings; lanes exchange their rows through shared memory (see
 // Rings).  The fast loop is unrolled two steps deep only and holds no rare
 // code: its size decides how well it is fetched.
-template <bool STD, bool PUSH, typename T, int QD>
+template <bool STD, bool PUSH, bool FULL, typename T, int QD>
 __device__ __forceinline__ void run_block(const Geo& g, Wave<T, QD>& st, Block<T>& b,
                                           const TileDesc& td, const int nS, uint2* bw) {
     using V2 = typename Vec2<T>::type;
@@ -621,15 +634,17 @@ __device__ __forceinline__ void run_block(const Geo& g, Wave<T, QD>& st, Block<T
     int t = 0;
     if (STD && !left && !right && !(top && bottom)) {
         if (top)
-            t = fast_steps<kTop, PUSH, T, QD>(st, b, td, rc, w0, w1, w2, cp, bitsA, bitsB);
+            t = fast_steps<kTop, PUSH, FULL, T, QD>(st, b, td, rc, w0, w1, w2, cp, bitsA, bitsB);
         else if (bottom)
-            t = fast_steps<kBottom, PUSH, T, QD>(st, b, td, rc, w0, w1, w2, cp, bitsA, bitsB);
+            t = fast_steps<kBottom, PUSH, FULL, T, QD>(st, b, td, rc, w0, w1, w2, cp, bitsA,
+                                                       bitsB);
         else
-            t = fast_steps<kInner, PUSH, T, QD>(st, b, td, rc, w0, w1, w2, cp, bitsA, bitsB);
+            t = fast_steps<kInner, PUSH, FULL, T, QD>(st, b, td, rc, w0, w1, w2, cp, bitsA,
+                                                      bitsB);
     }
     if (t < kBlk)
-        careful_steps<STD, PUSH, T, QD>(g, st, b, td, t, top || left, bottom || right, rc, cp,
-                                        ahead, bitsA, bitsB);
+        careful_steps<STD, PUSH, FULL, T, QD>(g, st, b, td, t, top || left, bottom || right, rc,
+                                              cp, ahead, bitsA, bitsB);
     // step t's code belongs in bits 2t, 2t+1: reverse the sixteen pairs
     bitsA = __brev(bitsA);
     bitsB = __brev(bitsB);

@@ -262,7 +262,7 @@ __global__ void __launch_bounds__(NW * 32, 16 / NW)
                 if (lane == 0 && b.tau0 + 2 * kBlk <= sc.span)
                     prefetch_next_block(Ct + (int64_t)k * sc.span * 32, b.tau0 + kBlk);
                 if (b.tau0 == 0) queue_start<QD, T>(st.q, b.Cs);
-                run_block<STD, false, T, QD>(g, st, b, td, sc.nS, nullptr);
+                run_block<STD, false, false, T, QD>(g, st, b, td, sc.nS, nullptr);
             }
             rs = ring_next(rs, RB);
             ws = ring_next(ws, RB);
