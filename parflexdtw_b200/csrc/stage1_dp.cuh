@@ -53,14 +53,16 @@ __device__ __forceinline__ bool qless_exact(double b, double nd, double a, doubl
 // FP32 form: RN32(b/nd) < RN32(a/md).  The cross products of two FP32 values
 // and two integers below 2^24 are exact in FP64, so their difference has the
 // sign of the exact comparison: <= 0 decides "not less"; a relative margin of
-// 2^-21 (two FP32 roundings are at most 2^-24 each) decides "less"; in
-// between the two IEEE divisions decide.
+// 2^-21 (two FP32 roundings are at most 2^-24 each) decides "less" where no
+// quotient can be subnormal (the mdists' product is below 2^35); in between
+// the two IEEE divisions decide.
 __device__ __forceinline__ bool qless_exact(float b, float nd, float a, float md) {
     const double U = __dmul_rn((double)b, (double)md);
     const double V = __dmul_rn((double)a, (double)nd);
     const double diff = __dadd_rn(V, -U);
     if (diff <= 0.0) return false;
-    if (diff > __dmul_rn(__dadd_rn(fabs(U), fabs(V)), 0x1p-21)) return true;
+    const double mag = __dadd_rn(fabs(U), fabs(V));
+    if (diff > __dmul_rn(mag, 0x1p-21) && mag >= 0x1p-60) return true;
     return __fdiv_rn(b, nd) < __fdiv_rn(a, md);
 }
 
@@ -129,45 +131,85 @@ __device__ __forceinline__ bool decide_quot(double a_new, double m_new, double a
     win = d > 0.0;
     return fabs(d) > t;
 }
-// FP32 form: the cross products of FP32 values and integers below 2^24 are
-// exact in FP64 (see the FP32 qless_exact): d <= 0 decides "not below", a
-// relative margin of 2^-21 decides "below".  Infinite values never decide.
-__device__ __forceinline__ bool decide_quot(float a_new, float m_new, float a_inc, float m_inc,
-                                            bool& win) {
-    const double U = __dmul_rn((double)a_new, (double)m_inc);
-    const double V = __dmul_rn((double)a_inc, (double)m_new);
-    const double d = __dadd_rn(V, -U);
-    win = d > __dmul_rn(__dadd_rn(fabs(U), fabs(V)), 0x1p-21);
-    return (win || d <= 0.0) && fabs(d) < CUDART_INF;
+// FP32 form: RN(a / m) itself, for 0 or 2^-80 <= |a| < 2^120 and an integer 1 <= m <
+// 2^17 (twice the tile length at most, which shared memory keeps far below).
+// One step of Markstein's division (IBM J. Res. Dev. 34, 1990) from the
+// approximate reciprocal y, whose relative error is below 2^-22: q is within
+// 5.3 ulps of a / m, so a - q m has at most 22 bits and the first FMA forms it
+// exactly; the second one rounds a value within 2^-19 ulp of a / m. The
+// quotient a / m is at least ulp / 2m >= 2^-18 ulp off every midpoint between two
+// FP32 values (it is no midpoint itself: those times m have 25 bits or more), so
+// both round alike.
+__device__ __forceinline__ float quot(float a, float m) {
+    float y;
+    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(m));
+    const float q = __fmul_rn(a, y);
+    return __fmaf_rn(__fmaf_rn(-m, q, a), y, q);
 }
 
 // Steps (1,1), (1,2), (2,1) at one cell, mdists given: branch-free selection.
 // Returns false when a comparison is too close to call or a value is not
 // finite; the caller then recomputes the cell with select_exact.  RIM: in1 /
 // in2 say whether the (1,2) / (2,1) predecessor exists (else all do).
-template <bool RIM, typename T>
-__device__ __forceinline__ bool select_std(T cval, T w0, T w1, T w2, T x1D, int x1P, T m0, T x2D,
-                                           int x2P, T m1, bool in1, T x3D, int x3P, T m2, bool in2,
-                                           T& oD, int& oP, int& code) {
-    const T a0 = addr(x1D, mulr(cval, w0));
-    const T a1 = addr(x2D, mulr(cval, w1));
-    const T a2 = addr(x3D, mulr(cval, w2));
+template <bool RIM>
+__device__ __forceinline__ bool select_std(double cval, double w0, double w1, double w2,
+                                           double x1D, int x1P, double m0, double x2D, int x2P,
+                                           double m1, bool in1, double x3D, int x3P, double m2,
+                                           bool in2, double& oD, int& oP, int& code) {
+    const double a0 = addr(x1D, mulr(cval, w0));
+    const double a1 = addr(x2D, mulr(cval, w1));
+    const double a2 = addr(x3D, mulr(cval, w2));
     bool win1, win2;
     bool ok1 = decide_quot(a1, m1, a0, m0, win1);
     if (RIM) {
         win1 = win1 && in1;
-        ok1 = in1 ? ok1 : a0 < (T)CUDART_INF;
+        ok1 = in1 ? ok1 : a0 < CUDART_INF;
     }
-    const T bA = win1 ? a1 : a0, bM = win1 ? m1 : m0;
+    const double bA = win1 ? a1 : a0, bM = win1 ? m1 : m0;
     bool ok2 = decide_quot(a2, m2, bA, bM, win2);
     if (RIM) {
         win2 = win2 && in2;
-        ok2 = in2 ? ok2 : bA < (T)CUDART_INF;
+        ok2 = in2 ? ok2 : bA < CUDART_INF;
     }
     oD = win2 ? a2 : bA;
     oP = win2 ? x3P : (win1 ? x2P : x1P);
     code = win2 ? 2 : (win1 ? 1 : 0);
     return ok1 && ok2;
+}
+
+// FP32 form: the three quotients, correctly rounded, compared as the reference
+// compares them: near ties, which a few in a hundred warp steps hold at FP32's
+// precision, need no second look. Values outside quot's range go to
+// select_exact (RIM: but for 0; in the fast loop that test would cost every
+// cell three instructions). Against FP64 cross products, which took eight
+// conversions per cell and left those near ties undecided: stage 1 of 64 pairs
+// of 1000 to 8000 frames in tiles of 1000, 7.1 -> 5.3 ms.
+template <bool RIM>
+__device__ __forceinline__ bool select_std(float cval, float w0, float w1, float w2, float x1D,
+                                           int x1P, float m0, float x2D, int x2P, float m1,
+                                           bool in1, float x3D, int x3P, float m2, bool in2,
+                                           float& oD, int& oP, int& code) {
+    const float a0 = addr(x1D, mulr(cval, w0));
+    float a1 = addr(x2D, mulr(cval, w1));
+    float a2 = addr(x3D, mulr(cval, w2));
+    if (RIM) {  // a missing predecessor: the incumbent again, never strictly below it
+        a1 = in1 ? a1 : a0;
+        m1 = in1 ? m1 : m0;
+        a2 = in2 ? a2 : a0;
+        m2 = in2 ? m2 : m0;
+    }
+    const float q0 = quot(a0, m0), q1 = quot(a1, m1), q2 = quot(a2, m2);
+    const bool win1 = q1 < q0;
+    const bool win2 = q2 < (win1 ? q1 : q0);
+    oD = win2 ? a2 : (win1 ? a1 : a0);
+    oP = win2 ? x3P : (win1 ? x2P : x1P);
+    code = win2 ? 2 : (win1 ? 1 : 0);
+    const bool below = fabsf(a0) + fabsf(a1) + fabsf(a2) < 0x1p120f;  // false for NaN
+    if (RIM) {
+        const auto fits = [](float a) { return a == 0.0f || fabsf(a) >= 0x1p-80f; };
+        return below && fits(a0) && fits(a1) && fits(a2);
+    }
+    return below && fminf(fminf(fabsf(a0), fabsf(a1)), fabsf(a2)) >= 0x1p-80f;
 }
 
 // The cost of the coming steps.  QD = 0: two steps ahead in registers.  QD > 0:
@@ -411,9 +453,9 @@ __device__ __forceinline__ bool fast_step(Wave<T, QD>& st, const Block<T>& b, co
     }
     T oAD, oBD;
     int oAP, oBP, codeA, codeB;
-    bool okA = select_std<false, T>(cc.x, w0, w1, w2, st.x1D, st.x1P, m0A, st.x2D, st.x2P, st.m1A,
+    bool okA = select_std<false>(cc.x, w0, w1, w2, st.x1D, st.x1P, m0A, st.x2D, st.x2P, st.m1A,
                                     true, st.x3D, st.x3P, m2A, true, oAD, oAP, codeA);
-    bool okB = select_std<KIND == kTop, T>(cc.y, w0, w1, w2, st.aD2, st.aP2, m0B, st.aD3, st.aP3,
+    bool okB = select_std<KIND == kTop>(cc.y, w0, w1, w2, st.aD2, st.aP2, m0B, st.aD3, st.aP3,
                                            st.m1B, true, st.x2D, st.x2P, st.m1A, lane != 0, oBD,
                                            oBP, codeB);
     if (KIND == kTop && lane == 0) {
@@ -521,9 +563,9 @@ __device__ __forceinline__ void careful_step(const Geo& g, Wave<T, QD>& st, cons
     int oAP, oBP, codeA, codeB;
     bool okA = false, okB = false;
     if (STD) {
-        okA = select_std<true, T>(cc.x, w0, w1, w2, st.x1D, st.x1P, m0A, st.x2D, st.x2P, st.m1A,
+        okA = select_std<true>(cc.x, w0, w1, w2, st.x1D, st.x1P, m0A, st.x2D, st.x2P, st.m1A,
                                   cA >= 2, st.x3D, st.x3P, m2A, true, oAD, oAP, codeA);
-        okB = select_std<true, T>(cc.y, w0, w1, w2, st.aD2, st.aP2, m0B, st.aD3, st.aP3, st.m1B,
+        okB = select_std<true>(cc.y, w0, w1, w2, st.aD2, st.aP2, m0B, st.aD3, st.aP3, st.m1B,
                                   cB >= 2, st.x2D, st.x2P, st.m1A, rB >= 2, oBD, oBP, codeB);
     }
     const bool actA = rA < b.R && cA >= 0 && cA < b.W;
