@@ -808,8 +808,7 @@ extern "C" int pfx_batch_complete(pfx_batch* b, int32_t i, double beta, const ui
     } else {
         double* An = p.feat;
         double* Bn = p.feat + (int64_t)b->d * p.g.N;
-        BCK(launch_l2norm(F1, b->d, p.g.N, An, s));
-        BCK(launch_l2norm(F2, b->d, p.g.M, Bn, s));
+        BCK(launch_l2norm(F1, F2, b->d, p.g.N, p.g.M, An, Bn, s));
         BCK(launch_cost_skew(An, Bn, b->d, p.g, b->slabs, p.skew_stride, s, p.tile_slot,
                              p.tile_list, (int)list.size(), b->cost_fma != 0));
     }
@@ -957,8 +956,7 @@ static int batch_enqueue(pfx_batch* b, cudaStream_t s, bool timed) {
             } else {
                 double* An = p.feat;
                 double* Bn = p.feat + (int64_t)b->d * p.g.N;
-                BCK(launch_l2norm(F1, b->d, p.g.N, An, cs));
-                BCK(launch_l2norm(F2, b->d, p.g.M, Bn, cs));
+                BCK(launch_l2norm(F1, F2, b->d, p.g.N, p.g.M, An, Bn, cs));
                 if (!b->gen_cost)  // (else stage 1 builds each tile's cost)
                     BCK(launch_cost_skew(An, Bn, b->d, p.g, static_cast<double*>(p.Csk),
                                          p.skew_stride, cs, slot, list, p.n_kept,

@@ -511,8 +511,7 @@ extern "C" int pfx_plan_load_features(pfx_plan* p, const double* F1, const doubl
     cudaStream_t s = (cudaStream_t)stream;
     double* An = p->feat;
     double* Bn = p->feat + (int64_t)d * p->g.N;
-    CK(launch_l2norm(F1, d, p->g.N, An, s));
-    CK(launch_l2norm(F2, d, p->g.M, Bn, s));
+    CK(launch_l2norm(F1, F2, d, p->g.N, p->g.M, An, Bn, s));
     CK(launch_cost_skew(An, Bn, d, p->g, static_cast<double*>(p->Csk), p->skew_stride, s,
                         active_mask(p)));
     p->cost_loaded = 1;

@@ -317,7 +317,8 @@ cudaError_t launch_relayout_skew_f32(const double* C64, const float* C32, int64_
 cudaError_t launch_cost_skew(const double* An, const double* Bn, int d, const Geo& g, double* Csk,
                              int64_t skew_stride, cudaStream_t st, const int32_t* slot = nullptr,
                              const int32_t* list = nullptr, int nlist = 0, bool fma = false);
-cudaError_t launch_l2norm(const double* F, int d, int64_t n, double* out, cudaStream_t st);
+cudaError_t launch_l2norm(const double* F1, const double* F2, int d, int64_t N, int64_t M,
+                          double* An, double* Bn, cudaStream_t st);
 cudaError_t launch_stage1(const double* C, const Geo& g, const S1Out& o, int tile0, int ntiles,
                           int nw, bool full, cudaStream_t st);
 size_t stage1_smem_bytes_host(int32_t L, int nw);
