@@ -339,27 +339,31 @@ cudaError_t launch_tile_full(const double* C, const Geo& g, double* D, int32_t* 
     const Sched2 s = make_sched2(g.L, g.L, cn * cw);
     const S1Mem m = stage1_mem(s.lag, cw, cta_budget(16), 8, 4);
     if (m.rb == 0 || m.qd == 0) return cudaSuccess;
-    // scratch: slab, P, backpointers, edges, descriptor, queue head and status
+    // scratch: slab and P (large: from the library's own pool, taking 60 MB from
+    // the default one costs about 1.5 ms), and backpointers, edges, descriptor,
+    // queue head and status
     auto up = [](size_t b) { return (b + 255) & ~(size_t)255; };
     const size_t slab = up((size_t)nS * ceil_div32(W + kStripRows - 1, kBlk) * kBlk * 64 * 8);
     const size_t bw = up((size_t)tile_b_words2(g.L) * 4), ed = up((size_t)2 * g.L * 12);
-    char* tmp = nullptr;
-    if (cudaMallocAsync((void**)&tmp, slab + slab / 2 + bw + ed + 512, st) != cudaSuccess) {
+    char *big = nullptr, *tmp = nullptr;
+    if (scratch_alloc((void**)&big, slab + slab / 2, st) != cudaSuccess ||
+        cudaMallocAsync((void**)&tmp, bw + ed + 512, st) != cudaSuccess) {
         cudaGetLastError();  // no room: the caller's other way needs less
+        if (big) cudaFreeAsync(big, st);
         return cudaSuccess;
     }
-    double* Dsk = reinterpret_cast<double*>(tmp);
-    int2* Psk = reinterpret_cast<int2*>(tmp + slab);
+    double* Dsk = reinterpret_cast<double*>(big);
+    int2* Psk = reinterpret_cast<int2*>(big + slab);
     TileDesc d;
     memset(&d, 0, sizeof(d));
     d.Csk = Dsk;
-    d.Bw = reinterpret_cast<uint32_t*>(tmp + slab + slab / 2);
-    d.eD = reinterpret_cast<double*>(tmp + slab + slab / 2 + bw);
+    d.Bw = reinterpret_cast<uint32_t*>(tmp);
+    d.eD = reinterpret_cast<double*>(tmp + bw);
     d.eP = reinterpret_cast<int32_t*>(d.eD + 2 * g.L);
     d.R = R;
     d.W = W;
     d.L = g.L;
-    char* misc = tmp + slab + slab / 2 + bw + ed;
+    char* misc = tmp + bw + ed;
     TileDesc* dd = reinterpret_cast<TileDesc*>(misc + 256);
     int* head = reinterpret_cast<int*>(misc);
     k_one_tile<<<1, 1, 0, st>>>(d, dd, head);
@@ -380,9 +384,9 @@ cudaError_t launch_tile_full(const double* C, const Geo& g, double* D, int32_t* 
         count_launches(1);
         e = cudaGetLastError();
     }
-    const cudaError_t ef = cudaFreeAsync(tmp, st);
+    const cudaError_t eb = cudaFreeAsync(big, st), ef = cudaFreeAsync(tmp, st);
     *done = true;
-    return e != cudaSuccess ? e : ef;
+    return e != cudaSuccess ? e : (eb != cudaSuccess ? eb : ef);
 }
 
 int stage1_cluster_max(int cn, int cw, const Geo& g, bool fp32) {
