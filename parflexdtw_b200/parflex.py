@@ -107,10 +107,58 @@ def _upload_staged(arr: np.ndarray) -> torch.Tensor:
     return out
 
 
+# Bytes of a piece of a host copy: pieces are copied between pageable and
+# page-locked memory (by all host threads) while the previous one is on the bus.
+# 64 MB up: 2.1 -> 1.5 ms against one page-locked copy and then one transfer.
+_PIECE_BYTES = 8 << 20
+
+
+def _upload(arr: np.ndarray) -> torch.Tensor:
+    """A C-contiguous host array to the device, piece by piece through
+    page-locked memory of its size (torch keeps it for later calls)."""
+    src = torch.from_numpy(arr).view(-1)
+    n, piece = src.numel(), _PIECE_BYTES // arr.itemsize
+    pinned = torch.empty(n, dtype=src.dtype, pin_memory=True)
+    out = torch.empty(n, dtype=src.dtype, device="cuda")
+    for a in range(0, n, piece):
+        pinned[a:a + piece].copy_(src[a:a + piece])
+        out[a:a + piece].copy_(pinned[a:a + piece], non_blocking=True)
+    return out.view(arr.shape)
+
+
+def _download(*tensors) -> list:
+    """Contiguous device tensors as NumPy arrays of the caller's own, through
+    two page-locked pieces: while one is filled from the device, host threads
+    copy the other out (and touch the new arrays' pages, which is what takes
+    a plain copy of fresh memory its time)."""
+    outs = [torch.empty(t.shape, dtype=t.dtype) for t in tensors]
+    stage = torch.empty((2, _PIECE_BYTES), dtype=torch.uint8, pin_memory=True)
+    pending = None  # (event, staged bytes, where they go)
+    k = 0
+    for t, o in zip(tensors, outs):
+        src, dst = t.view(-1).view(torch.uint8), o.view(-1).view(torch.uint8)
+        for a in range(0, src.numel(), _PIECE_BYTES):
+            part = src[a:a + _PIECE_BYTES]
+            buf = stage[k, :part.numel()]
+            buf.copy_(part, non_blocking=True)
+            ev = torch.cuda.Event()
+            ev.record(torch.cuda.current_stream(t.device))
+            if pending is not None:
+                pending[0].synchronize()
+                pending[2].copy_(pending[1])
+            pending = (ev, buf, dst[a:a + _PIECE_BYTES])
+            k ^= 1
+    if pending is not None:
+        pending[0].synchronize()
+        pending[2].copy_(pending[1])
+    return [o.numpy() for o in outs]
+
+
 def cost_matrix_to_gpu(C) -> torch.Tensor:
     """Host (or device) cost matrix as a contiguous FP64 CUDA tensor.  Host
     arrays above one staging chunk go through the double-buffered staged
-    upload; smaller ones through one page-locked copy."""
+    upload; smaller ones piece by piece through page-locked memory of their
+    size."""
     if isinstance(C, torch.Tensor):
         t = C if C.is_cuda else C.cuda()
         return t.to(torch.float64).contiguous()
@@ -118,7 +166,7 @@ def cost_matrix_to_gpu(C) -> torch.Tensor:
     if arr.size > _STAGE_ELEMS and arr.ndim == 2:
         with _stage_lock:
             return _upload_staged(arr)
-    return torch.from_numpy(arr).pin_memory().cuda(non_blocking=True)
+    return _upload(arr)
 
 
 # the reference's name for the same upload (gpu_flexdtw.py:112-116); FP64 here
@@ -191,24 +239,23 @@ def _find_best_endpoint(D, P, buffer):
     cstart = np.where(p >= 0, p, 0)
     with np.errstate(divide="ignore", invalid="ignore"):
         avg = D[rows, cols] / ((rows - rstart) + (cols - cstart))
-    best, br, bc = np.inf, -1, -1
-    debug = []
-    for k in range(rows.shape[0]):
-        r, c, a = int(rows[k]), int(cols[k]), float(avg[k])
-        if a < best:
-            best, br, bc = a, r, c
-        debug.append((c - W + 1, a, r, c) if r == R - 1 else (R - 1 - r, a, r, c))
-    return best, br, bc, debug
+    off = np.where(rows == R - 1, cols - W + 1, R - 1 - rows)
+    debug = list(zip(off.tolist(), avg.tolist(), rows.tolist(), cols.tolist()))
+    # the first of the smallest below infinity (no NaN is)
+    below = np.where(avg < np.inf, avg, np.inf)
+    k = int(np.argmin(below)) if below.size else -1
+    if k < 0 or below[k] == np.inf:
+        return np.inf, -1, -1, debug
+    return float(avg[k]), int(rows[k]), int(cols[k]), debug
 
 
 def _backtrace_tile(B, steps, r, c):
     """backtrace_flexdtw (FlexDTW.py:161-186), start-first (2, K)."""
     path = [(r, c)]
-    S = steps.shape[0]
+    moves, code = [(int(a), int(b)) for a, b in steps], B.item
     while r != 0 and c != 0:
-        s = int(B[r, c])
-        s = s + S if s < 0 else s
-        r, c = r - int(steps[s, 0]), c - int(steps[s, 1])
+        dr, dc = moves[code(r, c)]  # (a negative code counts from the end)
+        r, c = r - dr, c - dc
         path.append((r, c))
     path.reverse()
     return np.array(path, dtype=np.int64).T
@@ -227,7 +274,7 @@ def _tile_full(C_dev: torch.Tensor, r0, r1, c0, c1, steps, weights):
     L.check(L.load().pfx_flexdtw_tile(
         base, C_dev.stride(0), R, W, L.i64_array(st.reshape(-1)), L.f64_array(w),
         st.shape[0], D.data_ptr(), P.data_ptr(), B.data_ptr(), current_stream_ptr()))
-    return D.cpu().numpy(), P.cpu().numpy(), B.cpu().numpy()
+    return tuple(_download(D, P, B))
 
 
 def flexdtw_chunk_from_global_C(C_dev, L2_global, r0, r1, c0, c1, steps, weights,

@@ -54,3 +54,15 @@ def test_values(kind, steps, weights, oracle_mod):
         _, _, Do, Po, Bo = oracle_mod.flexdtw(C, steps, weights)
     assert np.array_equal(D, Do, equal_nan=True)
     assert np.array_equal(P, Po) and np.array_equal(B, Bo)
+
+
+@pytest.mark.parametrize("n", [1, 1023, (1 << 20) - 1, 1 << 20, (1 << 20) + 1, 3 * (1 << 20) + 17])
+def test_host_copies(n):
+    """Uploads and downloads in pieces of 8 MB return what went in."""
+    from parflexdtw_b200.parflex import _download, cost_matrix_to_gpu
+    C = np.random.default_rng(n).random((1, n))
+    up = cost_matrix_to_gpu(C)
+    codes = torch.arange(n, device="cuda").to(torch.int8)
+    D, B = _download(up, codes)
+    assert up.shape == C.shape and np.array_equal(D, C)
+    assert B.dtype == np.int8 and np.array_equal(B, codes.cpu().numpy())
