@@ -83,28 +83,41 @@ __global__ void __launch_bounds__(kRegionThreads) k_region_skew(const Tin* __res
 // strip (k_cost_skew takes two strips at once: 32 cells).  Column features of the CTA's window are
 // staged in shared memory split by column parity; at one instruction every
 // lane reads the same parity at consecutive half-indices (conflict-free).
-constexpr int kCT = 256;                // steps per CTA
+constexpr int kCT = 576;                // steps per CTA at most
 constexpr int kCV = 8;                  // steps per register pass
-constexpr int kCostThreads = 256;       // 8 warps x 32 steps
+constexpr int kCostThreads = 256;       // 8 warps, one pass after the other each
 constexpr int kCX = kCT + 66;           // window columns (x = c - ts + 64), even
 constexpr int kCH = kCX / 2;            // per parity
+
+// A tile's steps are cut into chunks of at most ct (a multiple of 64) steps,
+// alike but for the last and a multiple of 64, one pass per warp, each.
+__host__ __device__ inline int cost_chunks(int span, int ct) { return ceil_div32(span, ct); }
+__host__ __device__ inline int cost_chunk_len(int span, int ct) {
+    return (ceil_div32(span, cost_chunks(span, ct)) + 63) / 64 * 64;
+}
 
 // Two strips per CTA (blockIdx.y = strip pair): rows 64k + rho of strips 2kk
 // and 2kk + 1 sit at the same column for a given step, so each column vector
 // read from shared memory serves four cells of a lane.  The rows' features
 // are staged in shared memory too ([f][strip][64 rows], one 16-byte (A, B)
 // pair per lane: conflict-free), which keeps the registers to 32 sums.
+//
+// Bound by the FP64 pipe (24 operations per cell with 12 features: 79 % busy,
+// and shared memory three quarters as long), so the rest is kept out of the
+// passes: cells inside the tile are stored without tests, and a CTA takes up
+// to 576 steps for its 66 extra columns. 36000 x 36000 in tiles of 2000: 2.81 ->
+// 2.27 ms (570 Gcells/s) against 256 steps, a division per staged element and
+// tests on every store, which made half of the instructions.
 template <int DMAX, bool FMA>
 __global__ void __launch_bounds__(kCostThreads, 2)
     k_cost_skew(const double* __restrict__ An, const double* __restrict__ Bn, const int d,
                 const Geo g, double* __restrict__ Csk, const int64_t stride,
-                const int32_t* __restrict__ slot, const int32_t* __restrict__ list) {
+                const int32_t* __restrict__ slot, const int32_t* __restrict__ list, const int ct) {
     extern __shared__ __align__(16) double sB[];  // [d][2][kCH], then sA [d][2][64]
     double* sA = sB + d * kCX;
-    const int nchunk = ceil_div32(make_sched2(g.L, g.L, 1).span, kCT);
+    const int nchunk = cost_chunks(make_sched2(g.L, g.L, 1).span, ct);
     const int tile = list ? list[blockIdx.x / nchunk] : (int)(blockIdx.x / nchunk);
     const int kk = blockIdx.y;
-    const int ts = (int)(blockIdx.x % nchunk) * kCT;
     const int slab = slot ? slot[tile] : tile;  // slab index; < 0: tile skipped
     if (slab < 0) return;
     int64_t r0, c0;
@@ -112,20 +125,27 @@ __global__ void __launch_bounds__(kCostThreads, 2)
     tile_rect(g, tile / g.n2, tile % g.n2, &r0, &c0, &R, &W);
     const int span = ceil_div32(W + kStripRows - 1, kBlk) * kBlk;
     const int nS = ceil_div32(R, kStripRows);
+    const int len = cost_chunk_len(span, ct);
+    const int ts = (int)(blockIdx.x % nchunk) * len;
     if (2 * kk >= nS || ts >= span) return;
+    const int te = ts + len < span ? ts + len : span;  // the CTA's steps: [ts, te)
     const bool two = 2 * kk + 1 < nS;
     // the features, as asynchronous copies all in flight at once (one
     // memory latency per CTA, not one per element of a thread)
-    for (int q = threadIdx.x; q < d * kCX; q += kCostThreads) {
-        const int f = q / kCX, x = q - f * kCX;
+    for (int x = threadIdx.x; x < te - ts + 66; x += kCostThreads) {
         const int c = ts - 64 + x;
         const bool in = c >= 0 && c < W;
-        cp_async8(sB + (f * 2 + (x & 1)) * kCH + (x >> 1), in ? Bn + (int64_t)f * g.M + c0 + c : Bn,
-                  in);
+        const double* src = Bn + (in ? c0 + c : 0);
+        double* dst = sB + (x & 1) * kCH + (x >> 1);
+#pragma unroll 4
+        for (int f = 0; f < d; ++f, src += g.M, dst += 2 * kCH) cp_async8(dst, src, in);
     }
-    for (int q = threadIdx.x; q < d * 128; q += kCostThreads) {
-        const int f = q >> 7, r = 128 * kk + (q & 127);
-        cp_async8(sA + q, r < R ? An + (int64_t)f * g.N + r0 + r : An, r < R);
+    {
+        const int r = 128 * kk + (threadIdx.x & 127), f0 = threadIdx.x >> 7;
+        const double* src = An + (r < R ? r0 + r : 0) + f0 * g.N;
+        double* dst = sA + (threadIdx.x & 127) + f0 * 128;
+#pragma unroll 2
+        for (int f = f0; f < d; f += 2, src += 2 * g.N, dst += 256) cp_async8(dst, src, r < R);
     }
     cp_async_wait_all();
     __syncthreads();
@@ -134,18 +154,16 @@ __global__ void __launch_bounds__(kCostThreads, 2)
     const double2* sA2 = reinterpret_cast<const double2*>(sA);  // [f][strip][32 lanes]
     double2* out0 = reinterpret_cast<double2*>(Csk + (int64_t)slab * stride) +
                     (int64_t)(2 * kk) * span * 32 + lane;
-    double2* out1 = out0 + (int64_t)span * 32;
 #pragma unroll 1
-    for (int blk = 0; blk < 32 / kCV; ++blk) {
-        const int t0 = ts + 32 * warp + kCV * blk;  // warp-uniform
-        if (t0 >= span) break;
+    for (int t0 = ts + kCV * warp; t0 < te; t0 += kCV * kCostThreads / 32) {
+        // (te - ts is a multiple of 16, as spans are: every pass is whole)
         // A's column at t0 + v is window x = t0 - ts + 64 - 2*lane + v (even at v = 0);
         // b[j] holds x = xA0 - 1 + j, j = 0..8 (B at v uses b[v], A uses b[v + 1])
         const int h0 = ((t0 - ts + 64) >> 1) - lane;  // half-index of xA0
         double accA0[kCV], accB0[kCV], accA1[kCV], accB1[kCV];
 #pragma unroll
         for (int f = 0; f < DMAX; ++f) {
-            if (f >= d) break;
+            if (DMAX == kMaxFeat && f >= d) break;
             const double* se = sB + (f * 2) * kCH;  // even x
             const double* so = se + kCH;             // odd x
             double b[kCV + 1];
@@ -174,17 +192,26 @@ __global__ void __launch_bounds__(kCostThreads, 2)
                 }
             }
         }
+        double2* o0 = out0 + (int64_t)t0 * 32;
+        double2* o1 = o0 + (int64_t)span * 32;
+        if (128 * kk + 127 < R && t0 >= 63 && t0 + kCV <= W) {  // every cell inside the tile
 #pragma unroll
-        for (int v = 0; v < kCV; ++v) {
-            const int tau = t0 + v;
-            if (tau < span) {
-                const int cA = tau - 2 * lane, cB = cA - 1;
+            for (int v = 0; v < kCV; ++v) {
+                __stcs(o0 + v * 32,
+                       make_double2(__dsub_rn(1.0, accA0[v]), __dsub_rn(1.0, accB0[v])));
+                __stcs(o1 + v * 32,
+                       make_double2(__dsub_rn(1.0, accA1[v]), __dsub_rn(1.0, accB1[v])));
+            }
+        } else {
+#pragma unroll
+            for (int v = 0; v < kCV; ++v) {
+                const int cA = t0 + v - 2 * lane, cB = cA - 1;
                 const bool inA = cA >= 0 && cA < W, inB = cB >= 0 && cB < W;
-                __stcs(out0 + (int64_t)tau * 32,
+                __stcs(o0 + v * 32,
                        make_double2((rA0 < R && inA) ? __dsub_rn(1.0, accA0[v]) : 0.0,
                                     (rB0 < R && inB) ? __dsub_rn(1.0, accB0[v]) : 0.0));
                 if (two)
-                    __stcs(out1 + (int64_t)tau * 32,
+                    __stcs(o1 + v * 32,
                            make_double2((rA1 < R && inA) ? __dsub_rn(1.0, accA1[v]) : 0.0,
                                         (rB1 < R && inB) ? __dsub_rn(1.0, accB1[v]) : 0.0));
             }
@@ -319,22 +346,22 @@ static cudaError_t cost_skew_t(const double* An, const double* Bn, int d, const 
         return cudaGetLastError();
     }
     const size_t smem = (size_t)d * (kCX + 128) * sizeof(double);
-    dim3 grid = region_grid(g, kCT, nt);
-    grid.y = (grid.y + 1) / 2;  // strip pairs
-    cudaError_t e;
-    if (d == 12) {
-        e = cudaFuncSetAttribute(k_cost_skew<12, FMA>,
-                                 cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-        if (e != cudaSuccess) return e;
-        k_cost_skew<12, FMA><<<grid, kCostThreads, smem, st>>>(An, Bn, d, g, Csk, stride, slot,
-                                                               list);
-    } else {
-        e = cudaFuncSetAttribute(k_cost_skew<kMaxFeat, FMA>,
-                                 cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-        if (e != cudaSuccess) return e;
-        k_cost_skew<kMaxFeat, FMA><<<grid, kCostThreads, smem, st>>>(An, Bn, d, g, Csk, stride,
-                                                                     slot, list);
-    }
+    // long chunks where the grid has four waves (two CTAs per SM) of them
+    // (12000 x 12000 in tiles of 2000: 0.29 ms, with chunks of 128 steps 0.32; 2200 x
+    // 2200 in tiles of 500: 0.038 ms, with one chunk per strip 0.044)
+    int dev = 0, sms = 0, ct = kCT;
+    cudaGetDevice(&dev);
+    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    const Sched2 sL = make_sched2(g.L, g.L, 1);
+    const int64_t rows = (nt < 0 ? (int64_t)g.n1 * g.n2 : nt) * ((sL.nS + 1) / 2);
+    while (ct > 128 && rows * cost_chunks(sL.span, ct) < 8 * sms) ct = (ct / 2 + 63) / 64 * 64;
+    const dim3 grid((unsigned)((nt < 0 ? (int64_t)g.n1 * g.n2 : nt) * cost_chunks(sL.span, ct)),
+                    (unsigned)((sL.nS + 1) / 2));
+    auto kern = d == 12 ? k_cost_skew<12, FMA> : k_cost_skew<kMaxFeat, FMA>;
+    const cudaError_t e =
+        cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (e != cudaSuccess) return e;
+    kern<<<grid, kCostThreads, smem, st>>>(An, Bn, d, g, Csk, stride, slot, list, ct);
     count_launches(1);
     return cudaGetLastError();
 }
