@@ -233,13 +233,12 @@ struct pfx_batch {
     std::vector<std::vector<uint8_t>> mask_host, done;
     bool ran = false;  // a run since pfx_batch_set_masks
     // path checks and row-layout copies (allocated on first use)
-    PathRef* pref = nullptr;
+    PathRef* pref = nullptr;  // filled on first use
+    bool pref_ready = false;
     S2Pair* s2tab = nullptr;  // every pair's stage 2, in wave order (NaN beta: stale)
     double s2tab_beta = 0.0;
     int32_t* rows = nullptr;  // lo | hi block-row scratch
     size_t rows_cap = 0;
-    int64_t* prow = nullptr;  // device staging of row-layout paths, + offsets and lengths
-    size_t prow_cap = 0;
 };
 
 static void batch_free(pfx_batch* b) {
@@ -273,7 +272,6 @@ static void batch_free(pfx_batch* b) {
     if (b->pref) cudaFree(b->pref);
     if (b->s2tab) cudaFree(b->s2tab);
     if (b->rows) cudaFree(b->rows);
-    if (b->prow) cudaFree(b->prow);
     cudaSetDevice(cur);
     delete b;
 }
@@ -560,6 +558,10 @@ extern "C" int pfx_batch_create(int32_t n, const int64_t* N, const int64_t* M, c
             e = cudaMemcpy(b->gpairs, gp.data(), gp.size() * sizeof(GPair),
                            cudaMemcpyHostToDevice);
     }
+    // (here, not in the first run: a cudaMalloc can take milliseconds)
+    if (e == cudaSuccess) e = cudaMalloc(&b->s2tab, (size_t)n * sizeof(S2Pair));
+    b->s2tab_beta = NAN;
+    if (e == cudaSuccess) e = cudaMalloc(&b->pref, (size_t)n * sizeof(PathRef));
     if (e == cudaSuccess) e = cudaMemset(b->status, 0, 4);
     if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&b->cap, cudaStreamNonBlocking);
     for (int k = 0; k < kSide && e == cudaSuccess; ++k) {
@@ -1026,11 +1028,10 @@ extern "C" int pfx_batch_run(pfx_batch* b, double beta, int32_t use_graph, void*
         b->done = b->mask_host;
         b->ran = true;
     }
-    if (!b->s2tab || b->s2tab_beta != beta) {
+    if (b->s2tab_beta != beta) {
         // every pair's stage 2 in wave order (waves and beta are fixed until
         // the next pfx_batch_set_masks or another beta)
         BCK(cudaStreamSynchronize(s));  // an earlier run may still read the table
-        if (!b->s2tab) BCK(cudaMalloc(&b->s2tab, (size_t)b->n * sizeof(S2Pair)));
         std::vector<S2Pair> tab((size_t)b->n);
         for (int q = 0; q < b->n; ++q) {
             const pfx_plan& p = b->plans[b->wave_pairs[q]];
@@ -1123,7 +1124,7 @@ extern "C" int pfx_batch_results(pfx_batch* b, void* stream, double* best_cost, 
 }
 
 static int ensure_pref(pfx_batch* b) {
-    if (b->pref) return PFX_OK;
+    if (b->pref_ready) return PFX_OK;
     std::vector<PathRef> h((size_t)b->n);
     int64_t to = 0, ro = 0;
     for (int i = 0; i < b->n; ++i) {
@@ -1133,8 +1134,8 @@ static int ensure_pref(pfx_batch* b) {
         to += (int64_t)p.g.n1 * p.g.n2;
         ro += p.g.N + 2;  // block rows for any block size >= 1
     }
-    BCK(cudaMalloc(&b->pref, h.size() * sizeof(PathRef)));
     BCK(cudaMemcpy(b->pref, h.data(), h.size() * sizeof(PathRef), cudaMemcpyHostToDevice));
+    b->pref_ready = true;
     return PFX_OK;
 }
 
@@ -1167,23 +1168,31 @@ extern "C" int pfx_batch_check_paths(pfx_batch* b, int32_t margin, uint8_t* near
     return PFX_OK;
 }
 
-// Device staging for `total` path points, and room for every pair's offset
-// and length.
-static int ensure_prow(pfx_batch* b, int64_t total, cudaStream_t s, int64_t** off, int64_t** len) {
-    const size_t need = (size_t)2 * total + 2 * (size_t)b->n;
-    if (need > b->prow_cap) {
-        BCK(cudaStreamSynchronize(s));
-        if (b->prow) cudaFree(b->prow);
-        b->prow = nullptr;
-        b->prow_cap = 0;
-        const size_t cap2 = need + need / 4 + 1024;
-        BCK(cudaMalloc(&b->prow, cap2 * sizeof(int64_t)));
-        b->prow_cap = cap2;
+// Device staging of a call, in stream order: `total` path points, then every
+// pair's offset and length.
+struct PathStage {
+    int64_t* rows = nullptr;
+    int64_t* off = nullptr;
+    int64_t* len = nullptr;
+    cudaStream_t st;
+    explicit PathStage(cudaStream_t s) : st(s) {}
+    PathStage(const PathStage&) = delete;
+    PathStage& operator=(const PathStage&) = delete;
+    ~PathStage() {
+        if (rows) cudaFreeAsync(rows, st);
     }
-    *off = b->prow + b->prow_cap - 2 * (size_t)b->n;
-    *len = *off + b->n;
-    return PFX_OK;
-}
+    cudaError_t alloc(int64_t total, int n) {
+        const cudaError_t e =
+            scratch_alloc((void**)&rows, ((size_t)2 * total + 2 * (size_t)n) * 8, st);
+        if (e != cudaSuccess) {
+            rows = nullptr;
+            return e;
+        }
+        off = rows + 2 * total;
+        len = off + n;
+        return cudaSuccess;
+    }
+};
 
 extern "C" int pfx_batch_copy_paths_rows(pfx_batch* b, void* stream, int64_t* host,
                                          const int64_t* offsets, const int64_t* lens,
@@ -1199,17 +1208,17 @@ extern "C" int pfx_batch_copy_paths_rows(pfx_batch* b, void* stream, int64_t* ho
     }
     int st = ensure_pref(b);
     if (st) return st;
-    int64_t *d_off = nullptr, *d_len = nullptr;
-    if ((st = ensure_prow(b, total, s, &d_off, &d_len))) return st;
+    PathStage ps(s);
+    BCK(ps.alloc(total, b->n));
     std::vector<int64_t> ol((size_t)2 * b->n);
     std::copy(offsets, offsets + b->n, ol.begin());
     std::copy(lens, lens + b->n, ol.begin() + b->n);
-    BCK(cudaMemcpyAsync(d_off, ol.data(), ol.size() * 8, cudaMemcpyHostToDevice, s));
-    k_path_to_rows<<<dim3(16, b->n), 256, 0, s>>>(b->pref, d_off, d_len, b->prow);
+    BCK(cudaMemcpyAsync(ps.off, ol.data(), ol.size() * 8, cudaMemcpyHostToDevice, s));
+    k_path_to_rows<<<dim3(16, b->n), 256, 0, s>>>(b->pref, ps.off, ps.len, ps.rows);
     count_launches(1);
     BCK(cudaGetLastError());
     if (total > 0)
-        BCK(cudaMemcpyAsync(host, b->prow, (size_t)2 * total * 8, cudaMemcpyDeviceToHost, s));
+        BCK(cudaMemcpyAsync(host, ps.rows, (size_t)2 * total * 8, cudaMemcpyDeviceToHost, s));
     BCK(cudaStreamSynchronize(s));
     return PFX_OK;
 }
@@ -1247,13 +1256,13 @@ extern "C" int pfx_batch_copy_paths(pfx_batch* b, void* stream, int64_t* wp_host
     } else if (total > 0) {
         int st = ensure_pref(b);
         if (st) return st;
-        int64_t *d_off = nullptr, *d_len = nullptr;
-        if ((st = ensure_prow(b, total, s, &d_off, &d_len))) return st;
-        BCK(cudaMemcpyAsync(d_off, ol.data(), ol.size() * 8, cudaMemcpyHostToDevice, s));
-        k_path_pack<<<dim3(16, n), 256, 0, s>>>(b->pref, d_off, d_len, b->prow);
+        PathStage ps(s);
+        BCK(ps.alloc(total, n));
+        BCK(cudaMemcpyAsync(ps.off, ol.data(), ol.size() * 8, cudaMemcpyHostToDevice, s));
+        k_path_pack<<<dim3(16, n), 256, 0, s>>>(b->pref, ps.off, ps.len, ps.rows);
         count_launches(1);
         BCK(cudaGetLastError());
-        BCK(cudaMemcpyAsync(wp_host + 2 * offsets[0], b->prow, (size_t)total * 16,
+        BCK(cudaMemcpyAsync(wp_host + 2 * offsets[0], ps.rows, (size_t)total * 16,
                             cudaMemcpyDeviceToHost, s));
     }
     BCK(cudaStreamSynchronize(s));
