@@ -343,6 +343,10 @@ int pfx_batch_features(pfx_batch *batch, int32_t i, double **F1, double **F2);
  * pair's upload overlaps the work on other pairs). */
 int pfx_batch_load_async(pfx_batch *batch, int32_t i, const double *F1, const double *F2,
                          void *stream);
+/* Copies every pair's features from device memory on the batch's device into
+ * its input buffers, on `stream`: F[2 i] is pair i's F1 (d x N[i], row-major by
+ * feature), F[2 i + 1] its F2; a null entry is left as it is. */
+int pfx_batch_load_device(pfx_batch *batch, const double *const *F, void *stream);
 /* The plan of pair i (owned by the batch: do not destroy; do not load a
  * cost into it).  pfx_result / pfx_copy_path / pfx_plan_buffer read pair
  * i's results after pfx_batch_run. */

@@ -112,15 +112,29 @@ class Batch:
         into the batch's device buffers on the current stream."""
         if len(pairs) != self.n:
             raise ValueError(f"{len(pairs)} pairs for a batch of {self.n}")
-        for i, (F1, F2) in enumerate(pairs):
-            a, b = self.feature_views(i)
-            for dst, src in ((a, F1), (b, F2)):
+        here = torch.cuda.current_device() == self.device
+        ptrs = (ct.c_void_p * (2 * self.n))()
+        keep, rest = [], []  # keep: alive until the copies are submitted
+        for i, pair in enumerate(pairs):
+            F1, F2 = pair
+            for k, src in ((0, F1), (1, F2)):
                 t = src if isinstance(src, torch.Tensor) else torch.from_numpy(
                     np.ascontiguousarray(src, dtype=np.float64))
-                if tuple(t.shape) != tuple(dst.shape):
-                    raise ValueError(f"pair {i}: features {tuple(t.shape)} for a buffer "
-                                     f"{tuple(dst.shape)}")
-                dst.copy_(t, non_blocking=non_blocking)
+                want = (self.d, self.shapes[i][k])
+                if tuple(t.shape) != want:
+                    raise ValueError(f"pair {i}: features {tuple(t.shape)} for a buffer {want}")
+                if (here and type(t) is torch.Tensor and t.is_cuda
+                        and t.get_device() == self.device and t.dtype == torch.float64
+                        and t.layout == torch.strided and t.is_contiguous()
+                        and not t.requires_grad and not t.is_neg()):
+                    ptrs[2 * i + k] = t.data_ptr()
+                    keep.append(t)
+                else:
+                    rest.append((i, k, t))
+        if keep:  # device arrays as they are: one launch for up to 128 of them
+            _lib.check(_lib.load().pfx_batch_load_device(self._h, ptrs, current_stream_ptr()))
+        for i, k, t in rest:
+            self.feature_views(i)[k].copy_(t, non_blocking=non_blocking)
 
     def set_masks(self, masks, stream=None):
         """Restrict each pair to its tile mask (a CUDA uint8 tensor holding

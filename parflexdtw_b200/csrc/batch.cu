@@ -58,6 +58,40 @@ __global__ void __launch_bounds__(256) k_scatter_segments(const char* __restrict
     for (int64_t i = done + threadIdx.x; i < g.bytes; i += blockDim.x) dst[i] = src[i];
 }
 
+// Up to kCopyMany device-to-device copies of 8-byte words in one launch: blockIdx.y
+// is the copy, blockIdx.x a chunk of it (16-byte words where both ends are
+// aligned). Replaces a copy per sequence: 128 of 1000 to 8000 frames x 128
+// features 0.78 -> 0.20 ms on the device, and 1.2 ms of their submission.
+constexpr int kCopyMany = 128;
+constexpr int kCopyWords = 256 * 16;  // per chunk
+struct CopyMany {
+    const double* src[kCopyMany];
+    double* dst[kCopyMany];
+    int64_t n[kCopyMany];
+};
+__global__ void __launch_bounds__(256) k_copy_many(const __grid_constant__ CopyMany c) {
+    const int64_t i0 = (int64_t)blockIdx.x * kCopyWords, n = c.n[blockIdx.y] - i0;
+    if (n <= 0) return;
+    const double* src = c.src[blockIdx.y] + i0;
+    double* dst = c.dst[blockIdx.y] + i0;
+    const bool wide = ((reinterpret_cast<uintptr_t>(src) | reinterpret_cast<uintptr_t>(dst)) & 15) == 0;
+    if (wide && n >= kCopyWords) {
+        const double2* s2 = reinterpret_cast<const double2*>(src) + threadIdx.x;
+        double2* d2 = reinterpret_cast<double2*>(dst) + threadIdx.x;
+        double2 v[8];
+#pragma unroll
+        for (int k = 0; k < 8; ++k) v[k] = __ldcs(s2 + 256 * k);
+#pragma unroll
+        for (int k = 0; k < 8; ++k) d2[256 * k] = v[k];
+        return;
+    }
+#pragma unroll 8
+    for (int k = 0; k < kCopyWords / 256; ++k) {
+        const int i = threadIdx.x + 256 * k;
+        if (i < n) dst[i] = src[i];
+    }
+}
+
 __global__ void k_gather_results(const PairOut* __restrict__ po, int n, int64_t* __restrict__ out) {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
@@ -885,6 +919,45 @@ extern "C" int pfx_batch_load_async(pfx_batch* b, int32_t i, const double* F1,
                         cudaMemcpyHostToDevice, s));
     BCK(cudaMemcpyAsync(d2, F2, sizeof(double) * (size_t)b->d * b->plans[i].g.M,
                         cudaMemcpyHostToDevice, s));
+    return PFX_OK;
+}
+
+extern "C" int pfx_batch_load_device(pfx_batch* b, const double* const* F, void* stream) {
+    if (!b || !F) return errf(PFX_ERR_ARG, "null argument");
+    cudaStream_t s = (cudaStream_t)stream;
+    CopyMany c;
+    int m = 0;
+    int64_t longest = 0;
+    auto flush = [&]() -> cudaError_t {
+        if (m == 0) return cudaSuccess;
+        k_copy_many<<<dim3((unsigned)((longest + kCopyWords - 1) / kCopyWords), (unsigned)m), 256,
+                      0, s>>>(c);
+        count_launches(1);
+        m = 0;
+        longest = 0;
+        return cudaGetLastError();
+    };
+    const char* lo = reinterpret_cast<const char*>(b->arena);
+    for (int i = 0; i < 2 * b->n; ++i) {
+        if (!F[i]) continue;
+        const Geo& g = b->plans[i / 2].g;
+        double* dst = b->fin + b->fin_off[i / 2] + (i & 1 ? (int64_t)b->d * g.N : 0);
+        const int64_t n = (int64_t)b->d * (i & 1 ? g.M : g.N);
+        const char* src = reinterpret_cast<const char*>(F[i]);
+        if (src >= lo && src < lo + b->arena_bytes) {
+            // from the batch's own buffers: in order, after the copies before it
+            BCK(flush());
+            if (F[i] != dst)
+                BCK(cudaMemcpyAsync(dst, F[i], (size_t)n * 8, cudaMemcpyDeviceToDevice, s));
+            continue;
+        }
+        c.src[m] = F[i];
+        c.dst[m] = dst;
+        c.n[m] = n;
+        longest = std::max(longest, n);
+        if (++m == kCopyMany) BCK(flush());
+    }
+    BCK(flush());
     return PFX_OK;
 }
 
