@@ -436,19 +436,21 @@ extern "C" int pfx_batch_create(int32_t n, const int64_t* N, const int64_t* M, c
     }
     b->wave_first.push_back(n);
     const int waves = (int)b->wave_first.size() - 1;
-    // stage-1 warps per tile: from the largest wave's tile count
+    // stage-1 warps per tile: from the tiles of the wave with most of them
+    int64_t whole = 0;
     for (int w = 0; w < waves; ++w) {
-        int64_t t = 0;
+        int64_t t = 0, tw = 0;
         for (int q = b->wave_first[w]; q < b->wave_first[w + 1]; ++q) {
             const Geo& g = b->plans[b->wave_pairs[q]].g;
             t += (int64_t)g.n1 * g.n2;
+            tw += whole_tiles(g, maxL);
         }
+        whole = std::max(whole, tw);
         b->wave_tiles.push_back(t);
         b->max_wave_tiles = std::max(b->max_wave_tiles, t);
     }
     b->nw = nw ? nw
-               : stage1_queue_warps(b->max_wave_tiles, maxL,
-                                    num_sms_cur());
+               : stage1_queue_warps(whole, maxL, num_sms_cur());
     if (b->nw == 0 || !stage1_queue_fits(maxL, 16)) {
         batch_free(b);
         return errf(PFX_ERR_TOO_LARGE, "L=%d: the stage-1 rings do not fit in shared memory", maxL);

@@ -168,7 +168,7 @@ int pfx::plan_init(pfx_plan* p, int64_t N, int64_t M, int32_t L, const int64_t* 
     cudaGetDevice(&p->device);
     const Geo& g = p->g;
     const int64_t nt = (int64_t)g.n1 * g.n2;
-    p->nw = nw ? nw : stage1_queue_warps(nt, L, num_sms_cur());
+    p->nw = nw ? nw : stage1_queue_warps(whole_tiles(p->g, L), L, num_sms_cur());
     p->nw_default = p->nw;
     if (p->nw == 0 || !stage1_queue_fits(L, 16))
         return fail(PFX_ERR_TOO_LARGE, "L=%d: the stage-1 rings do not fit in shared memory", L);

@@ -249,6 +249,18 @@ int stage1_cluster_max(int cn, int cw, const Geo& g, bool fp32);
 // Whether the queue kernel's rings fit at tile length L with nw warps per
 // tile; its modelled time for ntiles tiles; the nw of the least (0: none fits).
 bool stage1_queue_fits(int32_t L, int nw);
+// How many L x L tiles have the area of all tiles of g, rounded up (L: g.L or
+// a batch's largest).
+inline int64_t whole_tiles(const Geo& g, int32_t L) {
+    int64_t cells = 0;
+    for (int t = 0; t < g.n1 * g.n2; ++t) {
+        int64_t r0, c0;
+        int32_t R, W;
+        tile_rect(g, t / g.n2, t % g.n2, &r0, &c0, &R, &W);
+        cells += (int64_t)R * W;
+    }
+    return (cells + (int64_t)L * L - 1) / ((int64_t)L * L);
+}
 double stage1_queue_ns(int64_t ntiles, int32_t L, int nw, int num_sms);
 int stage1_queue_warps(int64_t ntiles, int32_t L, int num_sms);
 // Modelled pipeline steps of an R x W tile on nw warps, and the time of a

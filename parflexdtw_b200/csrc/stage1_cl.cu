@@ -403,19 +403,21 @@ int stage1_cluster_max(int cn, int cw, const Geo& g, bool fp32) {
 
 // The cluster kernel's time per step with `warps` warps on an SM (tiles of 4000
 // x 4000 on 2, 4 and 8 CTAs of 4 warps: 217, 217 and 215 ns; 2 and 4 of 8: 260
-// and 248; 2 of 12: 304; 2 of 16: 363).
+// and 248; 80 of them on 2 of 12: 294; on 2 of 16: 409).
 static double cluster_step_ns(int warps) {
-    return warps <= 4 ? 217.0 : warps <= 8 ? 255.0 : warps <= 12 ? 304.0 : 363.0;
+    return warps <= 4 ? 217.0 : warps <= 8 ? 255.0 : warps <= 12 ? 300.0 : 405.0;
 }
 
 // Modelled as in stage1_queue_ns.  Measured, stage 1: 16 tiles of 4000 x 4000
-// 3.06 ms on 8 CTAs of 4 warps each (6.33 on one CTA of 16, 5.17 on two), 80
-// tiles (17 of them smaller) 4.62 ms with 2 CTAs of 12 warps each (6.41; 5.28 on
-// two of 16), 9 tiles of 1999 x 1999 1.55 ms on 4 CTAs of 4 (2.01).
+// 2.71 ms on 8 CTAs (6.33 on one CTA of 16 warps, 5.17 on two), 80 tiles (17
+// of them smaller) 4.29 ms with 2 CTAs of 12 warps each (6.41 on one of 16; 4.88
+// on two of 16), 9 tiles of 1999 x 1999 1.14 ms on 8 CTAs (1.48 on 4 of 4 warps,
+// 2.01 on one of 16), 12 tiles of 1000 x 1000 0.60 ms (0.68 on one of 8).
 S1Plan stage1_plan(const Geo& g, int ntiles, bool fp32, int num_sms) {
-    S1Plan best{0, stage1_queue_warps(ntiles, g.L, num_sms), 0};
+    const int64_t whole = whole_tiles(g, g.L);
+    S1Plan best{0, stage1_queue_warps(whole, g.L, num_sms), 0};
     if (ntiles > num_sms) return best;
-    double t = stage1_queue_ns(ntiles, g.L, best.cw, num_sms);
+    double t = stage1_queue_ns(whole, g.L, best.cw, num_sms);
     // the tiles' steps on one CTA of 16 warps, in queue order (largest first)
     std::vector<std::pair<int64_t, double>> alone;
     for (int i = 0; i < ntiles; ++i) {

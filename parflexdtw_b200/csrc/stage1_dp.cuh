@@ -419,18 +419,23 @@ __device__ __forceinline__ uint32_t d_address(uint32_t p, uint32_t kd) {
     return p * (2 * (uint32_t)sizeof(T) / (uint32_t)sizeof(int2)) + kd;
 }
 
-// What a strip is to its tile: rows 0 and 1 or the last row change a step.
-enum StripKind { kInner, kTop, kBottom };
+// What a strip is to its tile: rows 0 and 1 or the last row change a step; kRim:
+// an inner strip's blocks that reach columns 0 and 1, the last one, or past it;
+// kCorner: such blocks of strip 0 and the last strip, and all of a lone strip.
+enum StripKind { kInner, kTop, kBottom, kRim, kCorner };
 
 // One step of the fast loop: standard steps, every cell of the strip's rows
 // inside the tile has c >= 18 and is off the last column.  Returns false, with
 // the wave unchanged, when some lane's cell needs the exact routine.  u: the
 // step's parity.  kTop: strip 0 of several (row 0 is the cost itself, rows 1
 // and 2 have predecessors on it); kBottom: the last strip of several, whose
-// lanes past the last row count for nothing and whose last row is stored.
+// lanes past the last row count for nothing and whose last row is stored; kRim:
+// cells outside the columns count for nothing, column 0 is the cost itself,
+// column 1 has predecessors on it and the last column is stored; kCorner: all
+// of these.
 template <StripKind KIND, bool PUSH, bool FULL, typename T, int QD>
-__device__ __forceinline__ bool fast_step(Wave<T, QD>& st, const Block<T>& b, const int u, int t,
-                                          T rc, T w0, T w1, T w2, double* eD, int32_t* eP,
+__device__ __forceinline__ bool fast_step(Wave<T, QD>& st, const Block<T>& b,
+                                          const TileDesc& td, const int u, int t, T rc, T w0, T w1, T w2, double* eD, int32_t* eP,
                                           uint32_t& bitsA, uint32_t& bitsB) {
     constexpr int SD = 2 * (int)sizeof(T), SP = (int)sizeof(int2);
     const int lane = b.lane;
@@ -444,27 +449,72 @@ __device__ __forceinline__ bool fast_step(Wave<T, QD>& st, const Block<T>& b, co
     }
     __syncwarp();
     ld_pair(d_address<T>(b.r, b.kd) + u * SD, b.r + u * SP, x1n, x3n, p1n, p3n);
-    const T m0A = addr(rc, -fabs((T)st.x1P));
+    T m0A = addr(rc, -fabs((T)st.x1P));
     T m2A = addr(rc, -fabs((T)st.x3P));
     T m0B = addr(rc, -fabs((T)st.aP2));
     if (KIND == kTop) {
         if (lane == 1) m2A = rc;
         if (lane == 0) m0B = rc;
     }
+    const int rA = 64 * b.k + 2 * lane;
+    constexpr bool kRimmed = KIND == kRim || KIND == kCorner;
+    const int cA = b.tau0 + t - 2 * lane, cB = cA - 1;  // (kRimmed)
+    if (kRimmed) {
+        if (cA == 1) m0A = m2A = rc;
+        if (cB == 1) m0B = rc;
+    }
+    if (KIND == kCorner) {
+        if (rA == 2) m2A = rc;
+        if (rA == 0) m0B = rc;
+    }
     T oAD, oBD;
     int oAP, oBP, codeA, codeB;
-    bool okA = select_std<false>(cc.x, w0, w1, w2, st.x1D, st.x1P, m0A, st.x2D, st.x2P, st.m1A,
-                                    true, st.x3D, st.x3P, m2A, true, oAD, oAP, codeA);
-    bool okB = select_std<KIND == kTop>(cc.y, w0, w1, w2, st.aD2, st.aP2, m0B, st.aD3, st.aP3,
-                                           st.m1B, true, st.x2D, st.x2P, st.m1A, lane != 0, oBD,
-                                           oBP, codeB);
+    bool okA = select_std<kRimmed>(cc.x, w0, w1, w2, st.x1D, st.x1P, m0A, st.x2D, st.x2P, st.m1A,
+                                   !kRimmed || cA != 1, st.x3D, st.x3P, m2A, true, oAD, oAP,
+                                   codeA);
+    bool okB = select_std<KIND == kTop || kRimmed>(
+        cc.y, w0, w1, w2, st.aD2, st.aP2, m0B, st.aD3, st.aP3, st.m1B, !kRimmed || cB != 1,
+        st.x2D, st.x2P, st.m1A, KIND == kTop ? lane != 0 : KIND != kCorner || rA != 0, oBD, oBP,
+        codeB);
+    if (KIND == kRim) {
+        if (cA == 0) {
+            oAD = cc.x;
+            oAP = -rA;
+        }
+        if (cB == 0) {
+            oBD = cc.y;
+            oBP = -rA - 1;
+        }
+        // columns 1 .. W - 1 are the ones with a selection
+        const bool selA = (unsigned)(cA - 1) < (unsigned)(b.W - 1);
+        const bool selB = (unsigned)(cB - 1) < (unsigned)(b.W - 1);
+        okA = okA || !selA;
+        okB = okB || !selB;
+        codeA = selA ? codeA : 0;
+        codeB = selB ? codeB : 0;
+    }
+    if (KIND == kCorner) {
+        if (rA == 0 || cA == 0) {
+            oAD = cc.x;
+            oAP = rA == 0 ? cA : -rA;
+        }
+        if (cB == 0) {
+            oBD = cc.y;
+            oBP = -rA - 1;
+        }
+        const bool selA = (unsigned)(cA - 1) < (unsigned)(b.W - 1) && rA != 0 && rA < b.R;
+        const bool selB = (unsigned)(cB - 1) < (unsigned)(b.W - 1) && rA + 1 < b.R;
+        okA = okA || !selA;
+        okB = okB || !selB;
+        codeA = selA ? codeA : 0;
+        codeB = selB ? codeB : 0;
+    }
     if (KIND == kTop && lane == 0) {
         oAD = cc.x;
         oAP = b.tau0 + t;
         codeA = 0;
         okA = true;
     }
-    const int rA = 64 * b.k + 2 * lane;
     if (KIND == kBottom) {
         okA = okA || rA >= b.R;
         okB = okB || rA + 1 >= b.R;
@@ -478,6 +528,18 @@ __device__ __forceinline__ bool fast_step(Wave<T, QD>& st, const Block<T>& b, co
             eD[c] = (double)(isA ? oAD : oBD);
             eP[c] = isA ? oAP : oBP;
         }
+    }
+    if (KIND == kRim && (cA == b.W - 1 || cB == b.W - 1)) {
+        const bool isA = cA == b.W - 1;
+        const int r = rA + (isA ? 0 : 1);
+        eD[r] = (double)(isA ? oAD : oBD);
+        eP[r] = b.W == 1 ? 0 : (isA ? oAP : oBP);
+    }
+    if (KIND == kCorner) {
+        if (rA < b.R && (unsigned)cA < (unsigned)b.W)
+            store_edges(td, rA, cA, b.R, b.W, oAD, oAP);
+        if (rA + 1 < b.R && (unsigned)cB < (unsigned)b.W)
+            store_edges(td, rA + 1, cB, b.R, b.W, oBD, oBP);
     }
     if (FULL) {
         b.oD[t * 32] = make_v2<T>(oAD, oBD);
@@ -496,22 +558,23 @@ __device__ __forceinline__ bool fast_step(Wave<T, QD>& st, const Block<T>& b, co
 template <StripKind KIND, bool PUSH, bool FULL, typename T, int QD>
 __device__ __forceinline__ int fast_steps(Wave<T, QD>& st, Block<T>& b, const TileDesc& td, T& rc,
                                           T w0, T w1, T w2,
-                                          const typename Vec2<T>::type*& cp, uint32_t& bitsA,
-                                          uint32_t& bitsB) {
-    double* eD = KIND == kBottom ? td.eD : nullptr;
-    int32_t* eP = KIND == kBottom ? td.eP : nullptr;
+                                          const typename Vec2<T>::type*& cp, const int ahead,
+                                          uint32_t& bitsA, uint32_t& bitsB) {
+    double* eD = KIND == kBottom ? td.eD : KIND == kRim ? td.eD + td.L : nullptr;
+    int32_t* eP = KIND == kBottom ? td.eP : KIND == kRim ? td.eP + td.L : nullptr;
+    constexpr bool rimmed = KIND == kRim || KIND == kCorner;
     int t = 0;
 #pragma unroll 1
     for (; t < kBlk; t += 2) {
-        if (!fast_step<KIND, PUSH, FULL, T, QD>(st, b, 0, t, rc, w0, w1, w2, eD, eP, bitsA,
+        if (!fast_step<KIND, PUSH, FULL, T, QD>(st, b, td, 0, t, rc, w0, w1, w2, eD, eP, bitsA,
                                                 bitsB))
             return t;
-        queue_next<QD, T>(st.q, 0, t, cp, true);
+        queue_next<QD, T>(st.q, 0, t, cp, !rimmed || t < ahead);
         rc = addr(rc, (T)1);
-        if (!fast_step<KIND, PUSH, FULL, T, QD>(st, b, 1, t + 1, rc, w0, w1, w2, eD, eP, bitsA,
+        if (!fast_step<KIND, PUSH, FULL, T, QD>(st, b, td, 1, t + 1, rc, w0, w1, w2, eD, eP, bitsA,
                                                 bitsB))
             return t + 1;
-        queue_next<QD, T>(st.q, 1, t + 1, cp + 32, true);
+        queue_next<QD, T>(st.q, 1, t + 1, cp + 32, !rimmed || t + 1 < ahead);
         rc = addr(rc, (T)1);
         cp += 64;
         b.w += b.incW;
@@ -639,20 +702,26 @@ __device__ __forceinline__ void careful_steps(const Geo& g, Wave<T, QD>& st, Blo
     }
 }
 
+constexpr int kCornerWidth = 800;  // see run_block
+
 // One block of 16 steps of a strip, in two loops.
 //
-// The fast loop (standard steps, every cell of the block in a column from 18
-// to the last but one, strips of a tile of several) has no bounds tests, no
-// divisions and one branch per step, out of the loop when some cell is too
-// close to call; strip 0 and the last strip have a copy of their own each,
-// because the strips after strip 0 follow at its pace and a tile ends with its
-// last strip.  The careful loop does the rest: the remaining steps of such a
-// block, and the first five blocks of a strip and those that reach the tile's
-// last column or past it.  There (`rim`) cells on row 0 / column 0 and
-// predecessors on them (mdist r + c) or missing are handled by selects around
-// the same selection, and (`mask`) cells past the last row or column; undecided
-// cells -- with other step sets than the standard one, all cells -- take the
-// exact routine.
+// The fast loop (standard steps) has no divisions and one branch per step, out
+// of the loop when some cell is too close to call. It has a copy for each kind
+// of block: inner ones, every cell of which has all its predecessors in the
+// tile and off its rim (columns from 18 to the last but one), need no tests at
+// all; strip 0 and the last strip a few, because the strips after strip 0
+// follow at its pace and a tile ends with its last strip; blocks at the tile's
+// first and last columns selects around the selection, because a strip starts
+// when the one above has done its first six blocks. With the careful loop for
+// those, 12 tiles of 1000 x 1000 take 0.68 ms (0.60), 504 of them 1.85 (1.77).
+// The corners' copy, for which every warp of a tile would wait to be fetched,
+// is used from kCornerWidth columns on (504 tiles of 1000 x 1000 1.77 -> 1.74
+// ms, 399 of 2000 x 2000 4.97 -> 4.87, 80 of 4000 x 4000 4.28 -> 4.15; but 28 of
+// 100 x 100 88 -> 93 us and 25 of 500 x 500 0.295 -> 0.298 ms).
+// The careful loop does the rest: the remaining steps of a block, cells too
+// close to call taking the exact routine, and other step sets, with which all
+// cells take it.
 //
 // What bounds it: warp instructions issued, then the FP64 pipe (half rate), so
 // the step is written for few of both.  mdist of a predecessor that the
@@ -674,15 +743,24 @@ __device__ __forceinline__ void run_block(const Geo& g, Wave<T, QD>& st, Block<T
     const bool left = b.tau0 < 80, right = b.tau0 + 17 > b.W;
     const bool top = b.k == 0, bottom = b.k == nS - 1;
     int t = 0;
-    if (STD && !left && !right && !(top && bottom)) {
-        if (top)
-            t = fast_steps<kTop, PUSH, FULL, T, QD>(st, b, td, rc, w0, w1, w2, cp, bitsA, bitsB);
-        else if (bottom)
-            t = fast_steps<kBottom, PUSH, FULL, T, QD>(st, b, td, rc, w0, w1, w2, cp, bitsA,
-                                                       bitsB);
-        else
-            t = fast_steps<kInner, PUSH, FULL, T, QD>(st, b, td, rc, w0, w1, w2, cp, bitsA,
+    if (STD) {
+        if ((top || bottom) && (left || right || top == bottom)) {
+            if (b.W >= kCornerWidth)
+                t = fast_steps<kCorner, PUSH, FULL, T, QD>(st, b, td, rc, w0, w1, w2, cp, ahead,
+                                                           bitsA, bitsB);
+        } else if (left || right) {
+            t = fast_steps<kRim, PUSH, FULL, T, QD>(st, b, td, rc, w0, w1, w2, cp, ahead, bitsA,
+                                                    bitsB);
+        } else if (top) {
+            t = fast_steps<kTop, PUSH, FULL, T, QD>(st, b, td, rc, w0, w1, w2, cp, ahead, bitsA,
+                                                    bitsB);
+        } else if (bottom) {
+            t = fast_steps<kBottom, PUSH, FULL, T, QD>(st, b, td, rc, w0, w1, w2, cp, ahead,
+                                                       bitsA, bitsB);
+        } else {
+            t = fast_steps<kInner, PUSH, FULL, T, QD>(st, b, td, rc, w0, w1, w2, cp, ahead, bitsA,
                                                       bitsB);
+        }
     }
     if (t < kBlk)
         careful_steps<STD, PUSH, FULL, T, QD>(g, st, b, td, t, top || left, bottom || right, rc,

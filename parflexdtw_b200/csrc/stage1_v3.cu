@@ -291,11 +291,11 @@ static int queue_qd(int nw, bool std_steps, bool gen) { return std_steps && !gen
 
 // Modelled time of a tile: pipeline steps times the time of a step.  A strip
 // needs the one above it 80 steps ahead, published in blocks of 16; measured,
-// lags below 164 steps cost as much as 164 (each block then waits for its
-// producer).
+// lags below 120 steps cost as much as 120 (each block then waits for its
+// producer; 164 before the strips' first blocks had a fast loop).
 double stage1_model_steps(int32_t R, int32_t W, int nw) {
     const Sched2 s = make_sched2(R, W, nw);
-    return (s.nS - 1) * std::max(s.lag, 164) + s.span;
+    return (s.nS - 1) * std::max(s.lag, 120) + s.span;
 }
 
 // Time of a step (ns) with `ctas` CTAs of nw warps on an SM (tiles of 1000 x
@@ -320,10 +320,12 @@ double stage1_queue_ns(int64_t ntiles, int32_t L, int nw, int num_sms) {
 // Warps per tile: the choice of the least modelled time (stage1_queue_ns;
 // the FP64 rings are the larger, so they decide what fits).  Fewer warps per
 // tile fill the strip pipeline better but take longer per tile, which decides
-// where the last wave of tiles leaves SMs idle.  Measured with 4 / 8 / 16
-// warps: 399 tiles of 2000 x 2000 5.76 / 5.10 / 7.26 ms, 143 of them 4.74 /
-// 2.17 / 2.06 ms; 504 tiles of 1000 x 1000 1.85 / 2.14 / 3.81 ms, 323 of 500
-// x 500 0.52 / 0.69 / 1.13 ms.
+// where the last wave of tiles leaves SMs idle (ntiles: by their area, as the
+// small tiles at a matrix's edges fill in at the end: 576 whole and 24 small
+// tiles of 1000 x 1000 1.81 / 2.17 ms with 4 / 8 warps, by their number 8).
+// Measured with 4 / 8 / 16 warps: 399 tiles of 2000 x 2000 5.66 / 4.97 / 7.26 ms,
+// 143 of them 4.66 / 2.12 / 2.00 ms; 504 tiles of 1000 x 1000 1.77 / 1.94 / 3.8
+// ms, 323 of 500 x 500 0.47 / 0.61 / 1.1 ms, 25 of 500 x 500 0.33 / 0.30 ms.
 int stage1_queue_warps(int64_t ntiles, int32_t L, int num_sms) {
     int best = 0;
     double t = 0.0;
