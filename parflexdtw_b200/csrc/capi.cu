@@ -861,7 +861,7 @@ extern "C" int pfx_flexdtw_tile(const double* C, int64_t ldc, int32_t R, int32_t
         if (e == cudaSuccess) e = cudaMemsetAsync(P, 0, (size_t)R * W * 4, s);
         if (e == cudaSuccess) e = cudaMemsetAsync(B, 0, (size_t)R * W, s);
     } else {
-        e = launch_stage1(C, g, o, 0, 1, 8, true, s);
+        e = launch_stage1(C, g, o, s);
     }
     cudaFreeAsync(o.edge_D, s);
     cudaFreeAsync(o.edge_P, s);

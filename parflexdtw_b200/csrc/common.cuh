@@ -331,10 +331,8 @@ cudaError_t launch_cost_skew(const double* An, const double* Bn, int d, const Ge
                              const int32_t* list = nullptr, int nlist = 0, bool fma = false);
 cudaError_t launch_l2norm(const double* F1, const double* F2, int d, int64_t N, int64_t M,
                           double* An, double* Bn, cudaStream_t st);
-cudaError_t launch_stage1(const double* C, const Geo& g, const S1Out& o, int tile0, int ntiles,
-                          int nw, bool full, cudaStream_t st);
+cudaError_t launch_stage1(const double* C, const Geo& g, const S1Out& o, cudaStream_t st);
 size_t stage1_smem_bytes_host(int32_t L, int nw);
-int stage1_pick_warps(const Geo& g, int num_sms);
 cudaError_t launch_fill(double* p, int64_t n, double v, cudaStream_t st);
 // Stage 2, first part: the edge tensors and valid marks (the only part that
 // reads the cost slabs).

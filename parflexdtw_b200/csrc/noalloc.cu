@@ -154,6 +154,6 @@ extern "C" int pfx_flexdtw_tile_noalloc(const double* C, int64_t ldc, int32_t R,
     o.full_D = D;
     o.full_P = P;
     o.full_B = B;
-    const cudaError_t e = launch_stage1(C, g, o, 0, 1, 8, true, s);
+    const cudaError_t e = launch_stage1(C, g, o, s);
     return e == cudaSuccess ? PFX_OK : report_status(PFX_ERR_CUDA, cudaGetErrorString(e));
 }

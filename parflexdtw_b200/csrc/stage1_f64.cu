@@ -1,4 +1,6 @@
-// Stage 1: FlexDTW on every L x L tile, FP64, one CTA per tile.
+// FlexDTW of one tile with all of D, P and B as outputs, FP64, on one CTA: the
+// small and narrow tiles of pfx_flexdtw_tile (the others take the cluster
+// kernel of stage1_cl.cu) and pfx_flexdtw_tile_noalloc.
 //
 // Recurrence (FlexDTW.py:326-370): D[0,:] = C[0,:], D[:,0] = C[:,0], P = 0 and
 // B = 0 on those boundary cells.  For r, c >= 1 and each step s in the
@@ -36,11 +38,14 @@
 
 namespace pfx {
 
-template <int NW, bool FULL, bool STD>
-__global__ void __launch_bounds__(NW * 32, 1)
-    k_stage1_f64(const double* __restrict__ C, const Geo g, const S1Out out, const int tile0) {
+constexpr int kStage1Warps = 8;
+
+template <bool STD>
+__global__ void __launch_bounds__(kStage1Warps * 32, 1)
+    k_stage1_f64(const double* __restrict__ C, const Geo g, const S1Out out) {
+    constexpr int NW = kStage1Warps;
     extern __shared__ __align__(16) unsigned char smem_raw[];
-    const int tile = tile0 + (int)blockIdx.x;
+    const int tile = (int)blockIdx.x;
     const int ti = tile / g.n2, tj = tile % g.n2;
     int64_t r0, c0;
     int32_t R, W;
@@ -143,12 +148,10 @@ __global__ void __launch_bounds__(NW * 32, 1)
                         eD[g.L + r] = oD;
                         eP[g.L + r] = oP;
                     }
-                    if (FULL) {
-                        const int64_t f = (int64_t)r * W + c;
-                        out.full_D[f] = oD;
-                        out.full_P[f] = oP;
-                        out.full_B[f] = (int8_t)(code == 3 ? -1 : code);
-                    }
+                    const int64_t f = (int64_t)r * W + c;
+                    out.full_D[f] = oD;
+                    out.full_P[f] = oP;
+                    out.full_B[f] = (int8_t)(code == 3 ? -1 : code);
                 }
                 bits |= (uint32_t)code << (2 * t);
                 h2D = h1D;
@@ -173,42 +176,21 @@ inline size_t stage1_smem_bytes(int32_t L, int nw) {
 
 size_t stage1_smem_bytes_host(int32_t L, int nw) { return stage1_smem_bytes(L, nw); }
 
-template <int NW, bool FULL, bool STD>
-static cudaError_t launch_stage1_t(const double* C, const Geo& g, const S1Out& o, int tile0,
-                                   int ntiles, cudaStream_t st) {
-    const size_t smem = stage1_smem_bytes(g.L, NW);
-    cudaError_t e = cudaFuncSetAttribute(k_stage1_f64<NW, FULL, STD>,
-                                         cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+template <bool STD>
+static cudaError_t launch_stage1_t(const double* C, const Geo& g, const S1Out& o,
+                                   cudaStream_t st) {
+    const size_t smem = stage1_smem_bytes(g.L, kStage1Warps);
+    const cudaError_t e = cudaFuncSetAttribute(
+        k_stage1_f64<STD>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return e;
-    k_stage1_f64<NW, FULL, STD><<<ntiles, NW * 32, smem, st>>>(C, g, o, tile0);
+    k_stage1_f64<STD><<<1, kStage1Warps * 32, smem, st>>>(C, g, o);
     count_launches(1);
     return cudaGetLastError();
 }
 
-// Warps per CTA: 16 when the tile count leaves SMs free (one CTA per SM,
-// 16 strips in flight per tile), else 8 (more CTAs resident per SM).
-int stage1_pick_warps(const Geo& g, int num_sms) {
-    const int64_t tiles = (int64_t)g.n1 * g.n2;
-    if (g.L < 256) return 8;
-    return tiles <= (int64_t)num_sms ? 16 : 8;
-}
-
-cudaError_t launch_stage1(const double* C, const Geo& g, const S1Out& o, int tile0, int ntiles,
-                          int nw, bool full, cudaStream_t st) {
-    if (ntiles <= 0) return cudaSuccess;
+cudaError_t launch_stage1(const double* C, const Geo& g, const S1Out& o, cudaStream_t st) {
     const bool std_steps = g.S == 3 && g.kind[0] == 0 && g.kind[1] == 1 && g.kind[2] == 2;
-    if (full) {
-        if (std_steps)
-            return nw == 16 ? launch_stage1_t<16, true, true>(C, g, o, tile0, ntiles, st)
-                            : launch_stage1_t<8, true, true>(C, g, o, tile0, ntiles, st);
-        return nw == 16 ? launch_stage1_t<16, true, false>(C, g, o, tile0, ntiles, st)
-                        : launch_stage1_t<8, true, false>(C, g, o, tile0, ntiles, st);
-    }
-    if (std_steps)
-        return nw == 16 ? launch_stage1_t<16, false, true>(C, g, o, tile0, ntiles, st)
-                        : launch_stage1_t<8, false, true>(C, g, o, tile0, ntiles, st);
-    return nw == 16 ? launch_stage1_t<16, false, false>(C, g, o, tile0, ntiles, st)
-                    : launch_stage1_t<8, false, false>(C, g, o, tile0, ntiles, st);
+    return std_steps ? launch_stage1_t<true>(C, g, o, st) : launch_stage1_t<false>(C, g, o, st);
 }
 
 }  // namespace pfx
