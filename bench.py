@@ -297,7 +297,7 @@ def b200_arm(args, spec):
         if kv.get("workload") == spec.name:
             traffic = float(kv["bytes_per_launch"])
     roofline = {"bound": "hbm",
-                "kernel": "stage 1: k_stage1_cl (largest tiles, 2-CTA clusters) + k_stage1_v3 "
+                "kernel": "stage 1: k_stage1_cl (largest tiles, clusters of CTAs) + k_stage1_v3 "
                           "(other tiles, second stream), timed together",
                 "achieved": achieved,
                 "peak": peak, "unit": "GB/s", "frac": achieved / peak, "traffic": traffic,

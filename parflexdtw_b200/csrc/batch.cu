@@ -1054,24 +1054,6 @@ static int batch_enqueue(pfx_batch* b, cudaStream_t s, bool timed) {
         // stage 2 reads the cost slabs only in its edge gather: that part is
         // joined back into the main stream, so the next wave may overwrite the
         // pool while the rest of this wave's stage 2 runs on the side streams
-        BCK(cost_fork(q1 - q0, &nc));
-        for (int q = q0; q < q1; ++q) {
-            const cudaStream_t cs = cost_stream(q - q0, nc);
-            const pfx_plan& p = b->plans[b->wave_pairs[q]];
-            if (b->gen_cost)  // no slabs kept: overlap costs from the features
-                BCK(launch_stage2_edges(nullptr, nullptr, 0, false, p.g, p.s2, cs, p.feat,
-                                        p.feat + (int64_t)b->d * p.g.N, b->d));
-            else
-                BCK(launch_stage2_edges(nullptr, p.Csk, p.skew_stride, p.fp32 != 0, p.g, p.s2,
-                                        cs));
-        }
-        BCK(cost_join(nc));
-        BCK(mark(w, 3));
-        BCK(cudaEventRecord(b->fork_ev, s));
-        // the rest of the wave's stage 2: a launch per step for all its pairs
-        const cudaStream_t ss = b->side[w % kSide];
-        used_side = std::max(used_side, w % kSide + 1);
-        BCK(cudaStreamWaitEvent(ss, b->fork_ev, 0));
         S2Pair one;
         memset(&one, 0, sizeof(one));
         for (int q = q0; q < q1; ++q) {
@@ -1083,6 +1065,13 @@ static int batch_enqueue(pfx_batch* b, cudaStream_t s, bool timed) {
             one.g.M = std::max(one.g.M, g.M);
         }
         const S2Pair* tab = b->s2tab + q0;
+        BCK(launch_stage2_edges(one, tab, q1 - q0, s));
+        BCK(mark(w, 3));
+        BCK(cudaEventRecord(b->fork_ev, s));
+        // the rest of the wave's stage 2: a launch per step for all its pairs
+        const cudaStream_t ss = b->side[w % kSide];
+        used_side = std::max(used_side, w % kSide + 1);
+        BCK(cudaStreamWaitEvent(ss, b->fork_ev, 0));
         BCK(launch_stage2_prop(one, tab, q1 - q0, ss));
         BCK(launch_sync_scan(one, tab, q1 - q0, ss));
         BCK(launch_stitch(one, tab, q1 - q0, ss, 1, 0, 0, 0, 0));
@@ -1110,7 +1099,13 @@ extern "C" int pfx_batch_run(pfx_batch* b, double beta, int32_t use_graph, void*
         std::vector<S2Pair> tab((size_t)b->n);
         for (int q = 0; q < b->n; ++q) {
             const pfx_plan& p = b->plans[b->wave_pairs[q]];
-            tab[q] = S2Pair{p.g, p.s2, buffer_global(p.g.N, p.g.M, beta)};
+            // (with the in-kernel cost no slabs are kept: costs from the features)
+            const S2Src src = b->gen_cost
+                                  ? S2Src{nullptr, nullptr, 0, p.feat,
+                                          p.feat + (int64_t)b->d * p.g.N, b->d, 0}
+                                  : S2Src{nullptr, p.Csk, p.skew_stride, nullptr, nullptr, 0,
+                                          p.fp32 != 0};
+            tab[q] = S2Pair{p.g, p.s2, buffer_global(p.g.N, p.g.M, beta), src};
         }
         BCK(cudaMemcpy(b->s2tab, tab.data(), tab.size() * sizeof(S2Pair),
                        cudaMemcpyHostToDevice));

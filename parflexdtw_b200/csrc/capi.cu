@@ -615,14 +615,16 @@ extern "C" int pfx_stage2_edges(pfx_plan* p, const double* C, int64_t ldc, void*
     if (p->gen_cost) {
         // a batch whose stage 1 built each tile's cost itself keeps no slabs:
         // the overlap costs come from the normalised features
-        CK(launch_stage2_edges(nullptr, nullptr, 0, false, g, p->s2, (cudaStream_t)stream,
-                               p->feat, p->feat + (int64_t)p->feat_d * g.N, p->feat_d));
+        const S2Src src{nullptr, nullptr, 0, p->feat, p->feat + (int64_t)p->feat_d * g.N,
+                        p->feat_d, 0};
+        CK(launch_stage2_edges(S2Pair{g, p->s2, 0, src}, nullptr, 1, (cudaStream_t)stream));
         return PFX_OK;
     }
     // the FP32 form reads overlap costs from its own FP32 slabs (the values
     // its DP used), never from an FP64 C
-    CK(launch_stage2_edges(p->fp32 ? nullptr : C, p->Csk, p->skew_stride, p->fp32 != 0, g,
-                           p->s2, (cudaStream_t)stream));
+    const S2Src src{p->fp32 ? nullptr : C, p->Csk, p->skew_stride, nullptr, nullptr, 0,
+                    p->fp32 != 0};
+    CK(launch_stage2_edges(S2Pair{g, p->s2, 0, src}, nullptr, 1, (cudaStream_t)stream));
     return PFX_OK;
 }
 

@@ -334,25 +334,27 @@ cudaError_t launch_l2norm(const double* F1, const double* F2, int d, int64_t N, 
 cudaError_t launch_stage1(const double* C, const Geo& g, const S1Out& o, cudaStream_t st);
 size_t stage1_smem_bytes_host(int32_t L, int nw);
 cudaError_t launch_fill(double* p, int64_t n, double v, cudaStream_t st);
-// Stage 2, first part: the edge tensors and valid marks (the only part that
-// reads the cost slabs).
-// With An (normalised features, [d][N] and [d][M]) the overlap costs are
-// computed from the features in the cost kernels' order, not read from C or
-// the slabs (a batch whose stage 1 built its cost itself keeps no slabs).
-cudaError_t launch_stage2_edges(const double* C, const void* Csk, int64_t skew_stride, bool f32,
-                                const Geo& g, const S2Buf& b, cudaStream_t st,
-                                const double* An = nullptr, const double* Bn = nullptr,
-                                int d = 0);
+// Where k_edges takes overlap costs from: the normalised features (An, Bn, d),
+// else a row-major cost (C, the Geo's ldc), else the cost slabs.
+struct S2Src {
+    const double* C;
+    const void* Csk;
+    int64_t skew_stride;
+    const double *An, *Bn;
+    int32_t d, f32;
+};
 // One alignment of a stage-2 launch (buf: the scan's global buffer).
 struct S2Pair {
     Geo g;
     S2Buf b;
     int64_t buf;
+    S2Src src;
 };
-// The rest of stage 2, of one alignment (tab null) or of the npairs in the
-// device table tab; `one` then holds the largest n1, n2, L, N and M of the
-// table, which size the launches.  Propagation; overlap sync and edge scan;
-// stitched backtrace.
+// Stage 2 of one alignment (tab null) or of the npairs in the device table tab;
+// `one` then holds the largest n1, n2, L, N and M of the table, which size the
+// launches.  The edge tensors and valid marks (the only part that reads the cost
+// slabs); propagation; overlap sync and edge scan; stitched backtrace.
+cudaError_t launch_stage2_edges(const S2Pair& one, const S2Pair* tab, int npairs, cudaStream_t st);
 cudaError_t launch_stage2_prop(const S2Pair& one, const S2Pair* tab, int npairs, cudaStream_t st);
 cudaError_t launch_sync_scan(const S2Pair& one, const S2Pair* tab, int npairs, cudaStream_t st);
 cudaError_t launch_stitch(const S2Pair& one, const S2Pair* tab, int npairs, cudaStream_t st,

@@ -39,7 +39,7 @@ struct pfx_plan {
     // stage-1 tile queue of this plan (descriptors in queue order) and its head
     pfx::TileDesc* descs;
     int* head;
-    // stage 1 of few tiles: the largest on 2-CTA clusters, the rest on single
+    // stage 1 of few tiles: all or the largest on clusters, the rest on single
     // CTAs in a second stream (created on first use, plans outside a batch)
     int* head2;
     cudaStream_t aux;
