@@ -2,9 +2,8 @@
 // element (tile, strip k, step tau, lane, half) = C[r0 + 64k + 2*lane + half]
 // [c0 + tau - 2*lane - half], zero outside the tile.
 //
-// One CTA fills a 64-row x (TC + 63)-column window of C in shared memory --
-// copied from a row-major C, or computed from the normalised features -- and
-// writes the TC skewed steps it covers as contiguous 512-byte rows.
+// From a row-major C, one CTA fills a 64-row x (TC + 63)-column window in shared
+// memory and writes the TC skewed steps it covers as contiguous rows.
 //
 // From features the value is 1 - sum_f A[f][row] * B[f][col] with the sum
 // taken in the fixed order f = 0, 1, ..., d-1 and every product and sum
@@ -17,19 +16,26 @@
 
 namespace pfx {
 
-constexpr int kTC = 256;               // skewed steps per CTA
-constexpr int kWinStride = kTC + 64;   // window columns (TC + 63 used, 1 pad); the
-                                       // diagonal read stride 319 is odd: conflict-free
+// Skewed steps per CTA of the relayout, by the slab's type: with FP64 slabs 128
+// (two CTAs per SM, one reading while the other writes; 24000 x 24000: 1.96 ms
+// against 2.27 with 256 and 2.42 with 64, whose windows overlap by half), with
+// FP32 slabs 256 (12000 x 12000: 0.43 ms against 0.44 with 128).
+template <typename T>
+constexpr int kTC = sizeof(T) == 8 ? 128 : 256;
+// Window columns (kTC + 63 used, 1 pad); the diagonal read stride is odd:
+// conflict-free.
+template <typename T>
+constexpr int kWinStride = kTC<T> + 64;
 constexpr int kMaxFeat = 16;           // features staged in shared memory
 
 template <typename T>
 __device__ __forceinline__ void write_skewed(const T* __restrict__ S, T* __restrict__ Cs,
                                              int span, int k, int ts) {
-    const int nt = (span - ts) < kTC ? (span - ts) : kTC;
+    const int nt = (span - ts) < kTC<T> ? (span - ts) : kTC<T>;
     for (int q = threadIdx.x; q < nt * 64; q += blockDim.x) {
         const int tt = q >> 6, rho = q & 63;
         const int x = tt - rho + 63;  // window column of (rho, ts + tt - rho)
-        Cs[((int64_t)k * span + ts + tt) * 64 + rho] = S[rho * kWinStride + x];
+        Cs[((int64_t)k * span + ts + tt) * 64 + rho] = S[rho * kWinStride<T> + x];
     }
 }
 
@@ -43,11 +49,11 @@ __global__ void __launch_bounds__(kRegionThreads) k_region_skew(const Tin* __res
                                                                int64_t stride,
                                                                const int32_t* __restrict__ slot) {
     extern __shared__ __align__(16) unsigned char S_raw[];
-    Tout* S = reinterpret_cast<Tout*>(S_raw);  // [64][kWinStride]
+    Tout* S = reinterpret_cast<Tout*>(S_raw);  // [64][kWinStride<Tout>]
     // blockIdx.x enumerates (tile, step chunk) pairs, blockIdx.y the strip
-    const int nchunk = ceil_div32(make_sched2(g.L, g.L, 1).span, kTC);
+    const int nchunk = ceil_div32(make_sched2(g.L, g.L, 1).span, kTC<Tout>);
     const int tile = (int)(blockIdx.x / nchunk), k = blockIdx.y;
-    const int ts = (int)(blockIdx.x % nchunk) * kTC;
+    const int ts = (int)(blockIdx.x % nchunk) * kTC<Tout>;
     const int slab = slot ? slot[tile] : tile;  // slab index; < 0: tile skipped
     if (slab < 0) return;
     const int ti = tile / g.n2, tj = tile % g.n2;
@@ -57,13 +63,13 @@ __global__ void __launch_bounds__(kRegionThreads) k_region_skew(const Tin* __res
     const Sched2 sc = make_sched2(R, W, 1);
     if (k >= sc.nS || ts >= sc.span) return;
     const int col0 = ts - 63;  // tile-local column of window column 0
-    // 40 elements per thread, issued as independent loads before the stores
-    constexpr int kPer = 64 * kWinStride / kRegionThreads;
+    // 24 (40) elements per thread, issued as independent loads before the stores
+    constexpr int kPer = 64 * kWinStride<Tout> / kRegionThreads;
     Tout v[kPer];
 #pragma unroll
     for (int u = 0; u < kPer; ++u) {
         const int q = threadIdx.x + u * kRegionThreads;
-        const int rho = q / kWinStride, x = q % kWinStride;
+        const int rho = q / kWinStride<Tout>, x = q % kWinStride<Tout>;
         const int r = 64 * k + rho, c = col0 + x;
         v[u] = (r < R && c >= 0 && c < W) ? (Tout)__ldcs(C + (r0 + r) * ldc + c0 + c) : (Tout)0;
     }
@@ -313,12 +319,12 @@ static dim3 region_grid(const Geo& g, int per_cta, int64_t ntiles = -1) {
 template <typename Tin, typename Tout>
 static cudaError_t relayout_t(const Tin* C, int64_t ldc, const Geo& g, Tout* Csk, int64_t stride,
                               cudaStream_t st, const int32_t* slot) {
-    const size_t smem = (size_t)64 * kWinStride * sizeof(Tout);
+    const size_t smem = (size_t)64 * kWinStride<Tout> * sizeof(Tout);
     auto kern = k_region_skew<Tin, Tout>;
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                          (int)smem);
     if (e != cudaSuccess) return e;
-    kern<<<region_grid(g, kTC), kRegionThreads, smem, st>>>(C, ldc, g, Csk, stride, slot);
+    kern<<<region_grid(g, kTC<Tout>), kRegionThreads, smem, st>>>(C, ldc, g, Csk, stride, slot);
     count_launches(1);
     return cudaGetLastError();
 }
