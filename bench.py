@@ -310,9 +310,8 @@ def b200_arm(args, spec):
                                   "k_stage1_cl (8.50 B, profiles/k_stage1_cl_ncu_small.md), "
                                   "scaled by cells",
                 "limiter": "the strip pipeline, not HBM: each strip follows the one above "
-                           "it; about 226 warp instructions per 64-cell warp-step at 39 % "
-                           "issue, FP64 pipe 16 %, the pipeline fill and drain of 32 warps "
-                           "per tile the largest stall (profiles/k_stage1_cl_ncu_small.md)"}
+                           "it by 120 steps or more, and a step takes 215 ns (4 warps on an "
+                           "SM) to 300 ns (12 warps) of dependent instructions"}
 
     # --- row-major C input: the relayout into the tile-skewed layout --------
     C_dev = pf.cost_matrix_from_features_gpu(F1, F2)
