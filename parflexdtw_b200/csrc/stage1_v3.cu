@@ -37,8 +37,8 @@
 // loop that holds nothing else; see run_block.  The cost queue runs two steps
 // ahead.
 //
-// Measured (592 tiles of 2000 x 2000, B200): 6.57 ms with 8 warps per tile,
-// 6.65 ms with 4 (356 Gcells/s), against 9.47 ms (4 warps) with shuffles,
+// Measured (592 tiles of 2000 x 2000, B200): 6.28 ms with 8 warps per tile
+// (377 Gcells/s), 6.53 with 4, against 9.47 ms (4 warps) with shuffles,
 // per-lane ring selects, one loop for all blocks and the exact routine inside
 // it.  An inner fast step costs 52 thread instructions per cell (79 before), 19
 // of them on the half-rate FP64 pipe; a careful one 112.
