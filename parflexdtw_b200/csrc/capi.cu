@@ -12,6 +12,7 @@
 #include <vector>
 
 #include "plan.cuh"
+#include "prop_list.cuh"
 
 
 
@@ -168,6 +169,9 @@ int pfx::plan_init(pfx_plan* p, int64_t N, int64_t M, int32_t L, const int64_t* 
     cudaGetDevice(&p->device);
     const Geo& g = p->g;
     const int64_t nt = (int64_t)g.n1 * g.n2;
+    if (!prop_list_fits(g.n1, g.n2, L))
+        return fail(PFX_ERR_TOO_LARGE, "%d x %d tiles of length %d: more edge slots than the "
+                    "propagation's lists can number", g.n1, g.n2, L);
     p->nw = nw ? nw : stage1_queue_warps(whole_tiles(p->g, L), L, num_sms_cur());
     p->nw_default = p->nw;
     if (p->nw == 0 || !stage1_queue_fits(L, 16))

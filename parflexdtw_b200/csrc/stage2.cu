@@ -16,6 +16,7 @@
 #include <cmath>
 
 #include "common.cuh"
+#include "prop_list.cuh"
 
 namespace pfx {
 
@@ -226,10 +227,10 @@ __device__ __forceinline__ int64_t tiles_before(const Geo& g, int a) {
 
 // The valid slots that depend on another slot, gathered per tile
 // anti-diagonal (diagonal a's at diag_list[tiles_before(a) * 2 L ..),
-// diag_count[a] of them, in no order) with the slot each reads; those that do
-// not get their value here.  Few slots are valid, so the propagation reads 8
-// bytes per such slot instead of a byte per slot, and the only thing left to
-// wait for on a diagonal is the value of the slot before.
+// diag_count[a] of them, in no order) with the slot each reads (prop_list.cuh);
+// those that do not get their value here.  Few slots are valid, so the
+// propagation reads 8 bytes per such slot instead of a byte per slot, and the
+// only thing left to wait for on a diagonal is the value of the slot before.
 __global__ void __launch_bounds__(256) k_valid_lists(const S2Pair one,
                                                      const S2Pair* __restrict__ tab) {
     const S2Pair& p = tab ? tab[blockIdx.y] : one;
@@ -246,8 +247,8 @@ __global__ void __launch_bounds__(256) k_valid_lists(const S2Pair one,
             b.D_arr[k] = b.edge_D[k];
             b.L_arr[k] = (double)(dr + dc);
         } else if (how != kPropNone) {
-            const int t = (int)(k / (2 * g.L));
-            const int a = t / g.n2 + t % g.n2;
+            const int t = (int)(k / (2 * g.L)), i = t / g.n2;
+            const int a = i + t % g.n2;
             // one atomic for the warp's slots of a diagonal
             const unsigned same = __match_any_sync(__activemask(), a);
             const int lane = threadIdx.x & 31, lead = __ffs(same) - 1;
@@ -255,33 +256,37 @@ __global__ void __launch_bounds__(256) k_valid_lists(const S2Pair one,
             if (lane == lead) at = atomicAdd(b.diag_count + a, __popc(same));
             at = __shfl_sync(same, at, lead) + __popc(same & ((1u << lane) - 1u));
             b.diag_list[tiles_before(g, a) * 2 * g.L + at] =
-                make_int2((int32_t)k, how == kPropCopy ? ~(int32_t)src : (int32_t)src);
+                make_int2(prop_place(g.n2, 2 * g.L, a, i, k),
+                          prop_back(k, src, how == kPropCopy));
         }
     }
 }
 
 // What a dependent slot adds to the slot it reads (copy: nothing).
 struct PropItem {
-    int32_t k, src;  // k < 0: none
+    int64_t k, src;  // k < 0: none
     bool copy;
     double eD, eC, dr, dc;
 };
 
-__device__ __forceinline__ PropItem prop_item(const Geo& g, const S2Buf& b, int2 v) {
+// Entry v of anti-diagonal a.
+__device__ __forceinline__ PropItem prop_item(const Geo& g, const S2Buf& b, int a, int2 v) {
     PropItem it;
-    it.k = v.x;
+    int i;
+    it.k = prop_slot(g.n2, 2 * g.L, a, v.x, &i);
+    it.src = prop_src(it.k, v.y);
     it.copy = v.y < 0;
-    it.src = it.copy ? ~v.y : v.y;
-    it.eD = b.edge_D[v.x];
-    it.eC = b.edge_Cf[v.x];
-    const int pos = (int)(v.x % g.L);
-    const int64_t te = v.x / g.L;
+    it.eD = b.edge_D[it.k];
+    it.eC = b.edge_Cf[it.k];
+    const int q = v.x % (2 * g.L);
+    const bool top = q < g.L;
+    const int pos = top ? q : q - g.L;
     int64_t r0, c0;
     int32_t R, W, sr, sc;
-    tile_rect(g, (int)((te >> 1) / g.n2), (int)((te >> 1) % g.n2), &r0, &c0, &R, &W);
-    decode_start(b.edge_P[v.x], &sr, &sc);
-    it.dr = (double)abs(((te & 1) == 0 ? R - 1 : pos) - sr);
-    it.dc = (double)abs(((te & 1) == 0 ? pos : W - 1) - sc);
+    tile_rect(g, i, a - i, &r0, &c0, &R, &W);
+    decode_start(b.edge_P[it.k], &sr, &sc);
+    it.dr = (double)abs((top ? R - 1 : pos) - sr);
+    it.dc = (double)abs((top ? pos : W - 1) - sc);
     return it;
 }
 
@@ -314,7 +319,7 @@ __global__ void __launch_bounds__(kPropThreads) k_propagate(const S2Pair one,
     auto first = [&](int a, int n) {
         PropItem it;
         it.k = -1;
-        if (tid < n) it = prop_item(g, b, list_of(a)[tid]);
+        if (tid < n) it = prop_item(g, b, a, list_of(a)[tid]);
         return it;
     };
     int n = b.diag_count[0];
@@ -322,8 +327,8 @@ __global__ void __launch_bounds__(kPropThreads) k_propagate(const S2Pair one,
     PropItem it = first(0, n);
     for (int a = 0; a < nd; ++a) {
         if (it.k >= 0) prop_apply(b, it);
-        for (int x = tid + nthr; x < n; x += nthr) prop_apply(b, prop_item(g, b, list_of(a)[x]));
-        const int ilo = a - (g.n2 - 1) > 0 ? a - (g.n2 - 1) : 0;
+        for (int x = tid + nthr; x < n; x += nthr) prop_apply(b, prop_item(g, b, a, list_of(a)[x]));
+        const int ilo = diag_row0(g.n2, a);
         const int ihi = a < g.n1 - 1 ? a : g.n1 - 1;
         // the diagonal's tiles on the first tile row / column
         if (tid == nthr - 1 && ilo == 0) prop_inherit(g, b, 0, a);
