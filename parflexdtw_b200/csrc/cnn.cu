@@ -13,6 +13,8 @@
 // map costs one small (P1 x d) x (d x P2) product instead of the full C.
 #include <cuda_bf16.h>
 
+#include <algorithm>
+
 #include "common.cuh"
 
 namespace pfx {
@@ -528,16 +530,20 @@ __device__ __forceinline__ float dz_at(const float* dy, const float* y, int relu
 // per tile, and so on.  k_dz_pixels lists them (in no order) and marks them in
 // a map; dw and dx then skip everything else, and cost no more than a dense
 // pass where every pixel is listed.  (A listed pixel is one whose dz is not
-// equal to 0: NaN counts.)
+// equal to 0: NaN counts.)  The list is made and used in bands of up to kDzBand
+// pixels, as offsets from the band's first (q0), so that its entries have 32
+// bits and its memory is bounded whatever the map's size.
+constexpr int64_t kDzBand = (int64_t)1 << 28;
+
 __global__ void __launch_bounds__(256) k_dz_pixels(const float* __restrict__ y,
                                                    const float* __restrict__ dy, int relu,
-                                                   int Cout, int64_t npix,
+                                                   int Cout, int64_t npix, int64_t q0, int32_t nq,
                                                    uint8_t* __restrict__ map,
                                                    int32_t* __restrict__ list,
                                                    int32_t* __restrict__ count) {
-    const int64_t q = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+    const int64_t at0 = blockIdx.x * (int64_t)blockDim.x + threadIdx.x, q = q0 + at0;
     bool on = false;
-    if (q < npix) {
+    if (at0 < nq) {
 #pragma unroll 16
         for (int co = 0; co < Cout; ++co) on |= !(dz_at(dy, y, relu, co * npix + q) == 0.f);
         map[q] = on;
@@ -547,7 +553,7 @@ __global__ void __launch_bounds__(256) k_dz_pixels(const float* __restrict__ y,
     int at = 0;
     if (lane == 0 && m) at = atomicAdd(count, __popc(m));
     at = __shfl_sync(0xffffffffu, at, 0) + __popc(m & ((1u << lane) - 1u));
-    if (on) list[at] = (int32_t)q;
+    if (on) list[at] = (int32_t)at0;
 }
 
 // Backward, data: dx[ci][iy][ix] = sum_{co, tap} w[co][ci][tap] dz[co][oy][ox]
@@ -628,7 +634,7 @@ template <int S>
 __global__ void __launch_bounds__(256)
     k_conv3x3_bwd_weight(const float* __restrict__ x, int Cin, int H, int W, int Cout, int Ho,
                          int Wo, const float* __restrict__ y, const float* __restrict__ dy,
-                         int relu, const int32_t* __restrict__ list,
+                         int relu, int64_t q0, const int32_t* __restrict__ list,
                          const int32_t* __restrict__ count, float* __restrict__ dw,
                          float* __restrict__ db) {
     __shared__ float xs[kWgPix * 32 * 9];          // [pixel][ci][tap]
@@ -651,8 +657,8 @@ __global__ void __launch_bounds__(256)
         const int np = min(kWgPix, n - p0);
         __syncthreads();  // the previous batch is consumed
         if (threadIdx.x < np) {
-            const int pix = list[p0 + threadIdx.x];
-            at[threadIdx.x] = make_int2(pix / Wo * S - 1, pix % Wo * S - 1);
+            const int64_t pix = q0 + list[p0 + threadIdx.x];
+            at[threadIdx.x] = make_int2((int)(pix / Wo) * S - 1, (int)(pix % Wo) * S - 1);
         }
         __syncthreads();
         for (int q = threadIdx.x; q < nci * 9; q += 256) {
@@ -669,7 +675,7 @@ __global__ void __launch_bounds__(256)
         for (int q = threadIdx.x; q < np * 32; q += 256) {
             const int p = q >> 5, c = q & 31;
             dzs[p][c] = c < nco ? dz_at(dy, y, relu,
-                                        (int64_t)(co0 + c) * Ho * Wo + list[p0 + p])
+                                        (int64_t)(co0 + c) * Ho * Wo + q0 + list[p0 + p])
                                 : 0.f;
         }
         __syncthreads();
@@ -1051,20 +1057,23 @@ static cudaError_t conv_bwd_t(const float* x, int Cin, int H, int W, const float
                               float* db, cudaStream_t st) {
     const int Ho = (H - 1) / S + 1, Wo = (W - 1) / S + 1;
     const int64_t npix = (int64_t)Ho * Wo;
-    // the listed pixels: count, list, map
+    // the listed pixels: count, list of a band, map
+    const int64_t band = std::min(npix, kDzBand);
     char* tmp = nullptr;
-    cudaError_t e = scratch_alloc((void**)&tmp, 16 + (size_t)npix * 5, st);
+    cudaError_t e = scratch_alloc((void**)&tmp, 16 + (size_t)band * 4 + (size_t)npix, st);
     if (e != cudaSuccess) return e;
     int32_t* count = reinterpret_cast<int32_t*>(tmp);
     int32_t* list = reinterpret_cast<int32_t*>(tmp + 16);
-    uint8_t* map = reinterpret_cast<uint8_t*>(list + npix);
-    e = cudaMemsetAsync(count, 0, 4, st);
-    if (e == cudaSuccess) {
-        k_dz_pixels<<<blocks_for(npix, 256), 256, 0, st>>>(y, dy, relu, Cout, npix, map, list,
-                                                           count);
-        const dim3 gw(kWgCtas, blocks_for(Cin, 32), blocks_for(Cout, 32));
-        k_conv3x3_bwd_weight<S><<<gw, 256, 0, st>>>(x, Cin, H, W, Cout, Ho, Wo, y, dy, relu, list,
-                                                    count, dw, db);
+    uint8_t* map = reinterpret_cast<uint8_t*>(list + band);
+    const dim3 gw(kWgCtas, blocks_for(Cin, 32), blocks_for(Cout, 32));
+    for (int64_t q0 = 0; q0 < npix && e == cudaSuccess; q0 += band) {
+        const int32_t nq = (int32_t)std::min(band, npix - q0);
+        e = cudaMemsetAsync(count, 0, 4, st);
+        if (e != cudaSuccess) break;
+        k_dz_pixels<<<blocks_for(nq, 256), 256, 0, st>>>(y, dy, relu, Cout, npix, q0, nq, map,
+                                                         list, count);
+        k_conv3x3_bwd_weight<S><<<gw, 256, 0, st>>>(x, Cin, H, W, Cout, Ho, Wo, y, dy, relu, q0,
+                                                    list, count, dw, db);
         count_launches(2);
         e = cudaGetLastError();
     }
