@@ -533,11 +533,26 @@ __device__ __forceinline__ float dz_at(const float* dy, const float* y, int relu
 // equal to 0: NaN counts.)  The list is made and used in bands of up to kDzBand
 // pixels, as offsets from the band's first (q0), so that its entries have 32
 // bits and its memory is bounded whatever the map's size.
+// A product with a dz of 0 counts all the same where its other factor is not
+// finite (it is NaN): the first band's launch looks for such values, and dw
+// takes every pixel if x (nx values) has one, dx if w (nw) has one.
 constexpr int64_t kDzBand = (int64_t)1 << 28;
+constexpr int kDzAllX = 1, kDzAllW = 2;  // count[1]
+
+// Whether one of a[i], a[i + step], ... below n is not finite.
+__device__ __forceinline__ bool any_not_finite(const float* __restrict__ a, int64_t i, int64_t n,
+                                               int64_t step) {
+    float z = 0.f;
+#pragma unroll 8
+    for (; i < n; i += step) z = fmaf(a[i], 0.f, z);
+    return !(z == 0.f);
+}
 
 __global__ void __launch_bounds__(256) k_dz_pixels(const float* __restrict__ y,
                                                    const float* __restrict__ dy, int relu,
                                                    int Cout, int64_t npix, int64_t q0, int32_t nq,
+                                                   const float* __restrict__ x, int64_t nx,
+                                                   const float* __restrict__ w, int64_t nw,
                                                    uint8_t* __restrict__ map,
                                                    int32_t* __restrict__ list,
                                                    int32_t* __restrict__ count) {
@@ -554,12 +569,19 @@ __global__ void __launch_bounds__(256) k_dz_pixels(const float* __restrict__ y,
     if (lane == 0 && m) at = atomicAdd(count, __popc(m));
     at = __shfl_sync(0xffffffffu, at, 0) + __popc(m & ((1u << lane) - 1u));
     if (on) list[at] = (int32_t)at0;
+    if (q0 == 0) {
+        const int64_t step = (int64_t)gridDim.x * blockDim.x;
+        const int all = (any_not_finite(x, at0, nx, step) ? kDzAllX : 0) |
+                        (any_not_finite(w, at0, nw, step) ? kDzAllW : 0);
+        if (all) atomicOr(count + 1, all);
+    }
 }
 
 // Backward, data: dx[ci][iy][ix] = sum_{co, tap} w[co][ci][tap] dz[co][oy][ox]
 // over the outputs whose window covers (iy, ix).  One thread per input pixel
 // and 32 input channels, the weights in shared memory as [tap][co][ci]; a CTA
-// none of whose pixels is covered by a listed output stores zeros.  Bound by
+// none of whose pixels is covered by a listed output stores zeros (count[1]: see
+// k_dz_pixels).  Bound by
 // the store of dx.  Layer 2 of the proposer (32 -> 32, stride 2, 313 x 360):
 // one thread per dx value, every output read, took 443 us.
 constexpr int kBdCi = 32;
@@ -568,20 +590,22 @@ template <int S>
 __global__ void __launch_bounds__(256)
     k_conv3x3_bwd_data(const float* __restrict__ w, int Cin, int H, int W, int Cout, int Ho,
                        int Wo, const float* __restrict__ y, const float* __restrict__ dy,
-                       int relu, const uint8_t* __restrict__ map, float* __restrict__ dx) {
+                       int relu, const uint8_t* __restrict__ map,
+                       const int32_t* __restrict__ count, float* __restrict__ dx) {
     extern __shared__ __align__(16) float ws[];  // [9][Cout][32]
     const int64_t npix = (int64_t)H * W;
     const int64_t q = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
     const int ci0 = blockIdx.y * kBdCi, nci = min(kBdCi, Cin - ci0);
     const int ix = (int)(q % W), iy = (int)(q / W);
     // the outputs (oy, ox) = ((iy + 1 - ky) / S, ...) of each tap, where listed
+    const bool all = count[1] & kDzAllW;
     unsigned taps = 0;
     if (q < npix) {
 #pragma unroll
         for (int tap = 0; tap < 9; ++tap) {
             const int ty = iy + 1 - tap / 3, tx = ix + 1 - tap % 3;
             if (ty < 0 || tx < 0 || ty % S || tx % S || ty / S >= Ho || tx / S >= Wo) continue;
-            if (map[(int64_t)(ty / S) * Wo + tx / S]) taps |= 1u << tap;
+            if (all || map[(int64_t)(ty / S) * Wo + tx / S]) taps |= 1u << tap;
         }
     }
     float acc[kBdCi];
@@ -634,13 +658,15 @@ template <int S>
 __global__ void __launch_bounds__(256)
     k_conv3x3_bwd_weight(const float* __restrict__ x, int Cin, int H, int W, int Cout, int Ho,
                          int Wo, const float* __restrict__ y, const float* __restrict__ dy,
-                         int relu, int64_t q0, const int32_t* __restrict__ list,
+                         int relu, int64_t q0, int32_t nq, const int32_t* __restrict__ list,
                          const int32_t* __restrict__ count, float* __restrict__ dw,
                          float* __restrict__ db) {
     __shared__ float xs[kWgPix * 32 * 9];          // [pixel][ci][tap]
     __shared__ __align__(16) float dzs[kWgPix][32];  // [pixel][co]
     __shared__ int2 at[kWgPix];                      // input row, column of tap 0
-    const int n = *count;
+    const bool all = count[1] & kDzAllX;  // (see k_dz_pixels)
+    const int n = all ? nq : *count;
+    const auto pixel = [&](int p) { return q0 + (all ? p : list[p]); };
     const int ci0 = blockIdx.y * 32, co0 = blockIdx.z * 32;
     const int nci = min(32, Cin - ci0), nco = min(32, Cout - co0);
     const int per = 8 * nci, slices = 256 / per;
@@ -657,7 +683,7 @@ __global__ void __launch_bounds__(256)
         const int np = min(kWgPix, n - p0);
         __syncthreads();  // the previous batch is consumed
         if (threadIdx.x < np) {
-            const int64_t pix = q0 + list[p0 + threadIdx.x];
+            const int64_t pix = pixel(p0 + threadIdx.x);
             at[threadIdx.x] = make_int2((int)(pix / Wo) * S - 1, (int)(pix % Wo) * S - 1);
         }
         __syncthreads();
@@ -675,7 +701,7 @@ __global__ void __launch_bounds__(256)
         for (int q = threadIdx.x; q < np * 32; q += 256) {
             const int p = q >> 5, c = q & 31;
             dzs[p][c] = c < nco ? dz_at(dy, y, relu,
-                                        (int64_t)(co0 + c) * Ho * Wo + q0 + list[p0 + p])
+                                        (int64_t)(co0 + c) * Ho * Wo + pixel(p0 + p))
                                 : 0.f;
         }
         __syncthreads();
@@ -1068,12 +1094,13 @@ static cudaError_t conv_bwd_t(const float* x, int Cin, int H, int W, const float
     const dim3 gw(kWgCtas, blocks_for(Cin, 32), blocks_for(Cout, 32));
     for (int64_t q0 = 0; q0 < npix && e == cudaSuccess; q0 += band) {
         const int32_t nq = (int32_t)std::min(band, npix - q0);
-        e = cudaMemsetAsync(count, 0, 4, st);
+        e = cudaMemsetAsync(count, 0, q0 == 0 ? 8 : 4, st);
         if (e != cudaSuccess) break;
-        k_dz_pixels<<<blocks_for(nq, 256), 256, 0, st>>>(y, dy, relu, Cout, npix, q0, nq, map,
-                                                         list, count);
+        k_dz_pixels<<<blocks_for(nq, 256), 256, 0, st>>>(y, dy, relu, Cout, npix, q0, nq, x,
+                                                         (int64_t)Cin * H * W, w,
+                                                         (int64_t)Cout * Cin * 9, map, list, count);
         k_conv3x3_bwd_weight<S><<<gw, 256, 0, st>>>(x, Cin, H, W, Cout, Ho, Wo, y, dy, relu, q0,
-                                                    list, count, dw, db);
+                                                    nq, list, count, dw, db);
         count_launches(2);
         e = cudaGetLastError();
     }
@@ -1084,7 +1111,7 @@ static cudaError_t conv_bwd_t(const float* x, int Cin, int H, int W, const float
         if (e == cudaSuccess) {
             const dim3 gd(blocks_for((int64_t)H * W, 256), blocks_for(Cin, kBdCi));
             k_conv3x3_bwd_data<S><<<gd, 256, sm, st>>>(w, Cin, H, W, Cout, Ho, Wo, y, dy, relu,
-                                                       map, dx);
+                                                       map, count, dx);
             count_launches(1);
             e = cudaGetLastError();
         }

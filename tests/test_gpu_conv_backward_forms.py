@@ -9,6 +9,7 @@ torch = pytest.importorskip("torch")
 if not torch.cuda.is_available():  # pragma: no cover - CPU container
     pytest.skip("needs a CUDA device", allow_module_level=True)
 
+from oracle import cnn_oracle as CO  # noqa: E402
 from parflexdtw_b200 import _lib, plan  # noqa: E402
 
 
@@ -49,3 +50,38 @@ def test_more_than_2_31_pixels():
     assert dx.sum(dtype=torch.float64).item() == 18.0 * len(set(xh))
     del x, y, dy, dx
     torch.cuda.empty_cache()
+
+
+@pytest.mark.parametrize("where", ["x", "w", "both", "dy"])
+@pytest.mark.parametrize("cin,cout,stride,H,W", [(32, 32, 2, 41, 60), (1, 32, 4, 70, 61),
+                                                 (32, 1, 1, 19, 33), (40, 36, 1, 20, 17)])
+def test_values_that_are_not_finite(cin, cout, stride, H, W, where):
+    """An infinite or NaN weight or activation makes NaN of every product it is
+    in, those with a gradient of 0 among them, as a dense sum has it."""
+    rng = np.random.default_rng(cin + H)
+    Ho, Wo = (H - 1) // stride + 1, (W - 1) // stride + 1
+    x = rng.standard_normal((cin, H, W)).astype(np.float32)
+    w = rng.standard_normal((cout, cin, 3, 3)).astype(np.float32)
+    y = np.ones((cout, Ho, Wo), np.float32)
+    dy = (rng.standard_normal(y.shape) * (rng.random((1, Ho, Wo)) < 0.05)).astype(np.float32)
+    dy[:, 2:, :] = 0  # far from what follows
+    if where in ("x", "both"):
+        x[0, H - 3, W // 2], x[cin - 1, H - 2, 1] = np.inf, np.nan
+    if where in ("w", "both"):
+        w[0, 0, 1, 1], w[cout - 1, cin - 1, 2, 0] = -np.inf, np.nan
+    if where == "dy":
+        dy[0, Ho - 1, Wo - 1], dy[cout - 1, Ho // 2, 0] = np.inf, np.nan
+    d = [torch.from_numpy(a).cuda() for a in (x, w, y, dy)]
+    dx, dw = torch.full((cin, H, W), 7.0, device="cuda"), torch.zeros((cout, cin, 3, 3), device="cuda")
+    db = torch.zeros(cout, device="cuda")
+    backward(d[0], d[1], stride, d[2], 1, d[3], dx, dw, db)
+    with np.errstate(all="ignore"):
+        ref = CO.conv3x3_backward(x, w, stride, y, 1, dy)
+    assert any(np.isnan(r).any() for r in ref)
+    for got, want in zip((dx, dw, db), ref):
+        got = got.cpu().numpy()
+        assert np.array_equal(np.isnan(got), np.isnan(want))
+        assert np.array_equal(np.isinf(got), np.isinf(want))
+        ok = np.isfinite(want)
+        # sums of at most 9 cout or Ho Wo products of standard normals
+        assert np.allclose(got[ok], want[ok], rtol=1e-4, atol=1e-3)
