@@ -528,9 +528,12 @@ __device__ __forceinline__ float dz_at(const float* dy, const float* y, int relu
 // channel's dz is not 0.  In training they are few: a tile's score is one
 // logit, so dz of the last layer has one pixel per tile, the layer before it 9
 // per tile, and so on.  k_dz_pixels lists them (in no order) and marks them in
-// a map; dw and dx then skip everything else, and cost no more than a dense
-// pass where every pixel is listed.  (A listed pixel is one whose dz is not
-// equal to 0: NaN counts.)  The list is made and used in bands of up to kDzBand
+// a map; dw and dx then skip everything else.  (A listed pixel is one whose dz
+// is not equal to 0: NaN counts.)  Where most pixels are listed that is still
+// faster than the dense kernels were (32 -> 32 channels, stride 2, 626 x 720: 2.69
+// ms, now 0.22 with 1 % listed and 0.59 with all) but for few channels (1 -> 32,
+// stride 4, 1250 x 1438: 0.20, now 0.09 and 0.24; 32 -> 1 over 79 x 90, where the
+// two launches more count: 0.020, now 0.028 and 0.036).  The list is made and used in bands of up to kDzBand
 // pixels, as offsets from the band's first (q0), so that its entries have 32
 // bits and its memory is bounded whatever the map's size.
 // A product with a dz of 0 counts all the same where its other factor is not
@@ -579,23 +582,25 @@ __global__ void __launch_bounds__(256) k_dz_pixels(const float* __restrict__ y,
 
 // Backward, data: dx[ci][iy][ix] = sum_{co, tap} w[co][ci][tap] dz[co][oy][ox]
 // over the outputs whose window covers (iy, ix).  One thread per input pixel
-// and 32 input channels, the weights in shared memory as [tap][co][ci]; a CTA
-// none of whose pixels is covered by a listed output stores zeros (count[1]: see
-// k_dz_pixels).  Bound by
-// the store of dx.  Layer 2 of the proposer (32 -> 32, stride 2, 313 x 360):
-// one thread per dx value, every output read, took 443 us.
-constexpr int kBdCi = 32;
-
-template <int S>
+// and CI input channels (4 where there are no more, else 32), the weights in
+// shared memory as [tap][co][ci]; a CTA none of whose pixels is covered by a
+// listed output stores zeros (count[1]: see k_dz_pixels).
+// Bound by the CTAs with a listed output: each stages 36 KB of weights and runs
+// its pixels' chain of loads (the store of dx, 14.4 MB in 60 us, takes 4 % of
+// HBM). Layer 2 of the proposer (32 -> 32, stride 2, 313 x 360): one thread per
+// dx value, every output read, took 443 us. Layer 1 (one input channel, stride
+// 4, 1250 x 1438) with every output listed, dw included: 1.02 ms with 32
+// channels a thread, 0.24 with 4 and the batches below.
+template <int S, int CI>
 __global__ void __launch_bounds__(256)
     k_conv3x3_bwd_data(const float* __restrict__ w, int Cin, int H, int W, int Cout, int Ho,
                        int Wo, const float* __restrict__ y, const float* __restrict__ dy,
                        int relu, const uint8_t* __restrict__ map,
                        const int32_t* __restrict__ count, float* __restrict__ dx) {
-    extern __shared__ __align__(16) float ws[];  // [9][Cout][32]
+    extern __shared__ __align__(16) float ws[];  // [9][Cout][CI]
     const int64_t npix = (int64_t)H * W;
     const int64_t q = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-    const int ci0 = blockIdx.y * kBdCi, nci = min(kBdCi, Cin - ci0);
+    const int ci0 = blockIdx.y * CI, nci = min(CI, Cin - ci0);
     const int ix = (int)(q % W), iy = (int)(q / W);
     // the outputs (oy, ox) = ((iy + 1 - ky) / S, ...) of each tap, where listed
     const bool all = count[1] & kDzAllW;
@@ -608,12 +613,12 @@ __global__ void __launch_bounds__(256)
             if (all || map[(int64_t)(ty / S) * Wo + tx / S]) taps |= 1u << tap;
         }
     }
-    float acc[kBdCi];
+    float acc[CI];
 #pragma unroll
-    for (int c = 0; c < kBdCi; ++c) acc[c] = 0.f;
+    for (int c = 0; c < CI; ++c) acc[c] = 0.f;
     if (__syncthreads_or(taps != 0)) {
-        for (int i = threadIdx.x; i < 9 * Cout * kBdCi; i += blockDim.x) {
-            const int c = i % kBdCi, co = i / kBdCi % Cout, tap = i / kBdCi / Cout;
+        for (int i = threadIdx.x; i < 9 * Cout * CI; i += blockDim.x) {
+            const int c = i % CI, co = i / CI % Cout, tap = i / CI / Cout;
             ws[i] = c < nci ? w[((int64_t)co * Cin + ci0 + c) * 9 + tap] : 0.f;
         }
         __syncthreads();
@@ -624,9 +629,9 @@ __global__ void __launch_bounds__(256)
 #pragma unroll 8
             for (int co = 0; co < Cout; ++co) {
                 const float dz = dz_at(dy, y, relu, ((int64_t)co * Ho + oy) * Wo + ox);
-                const float4* w4 = reinterpret_cast<const float4*>(ws + (tap * Cout + co) * kBdCi);
+                const float4* w4 = reinterpret_cast<const float4*>(ws + (tap * Cout + co) * CI);
 #pragma unroll
-                for (int c4 = 0; c4 < kBdCi / 4; ++c4) {
+                for (int c4 = 0; c4 < CI / 4; ++c4) {
                     const float4 v = w4[c4];
                     acc[4 * c4 + 0] = fmaf(v.x, dz, acc[4 * c4 + 0]);
                     acc[4 * c4 + 1] = fmaf(v.y, dz, acc[4 * c4 + 1]);
@@ -638,7 +643,7 @@ __global__ void __launch_bounds__(256)
     }
     if (q >= npix) return;
 #pragma unroll
-    for (int c = 0; c < kBdCi; ++c)
+    for (int c = 0; c < CI; ++c)
         if (c < nci) dx[(int64_t)(ci0 + c) * npix + q] = acc[c];
 }
 
@@ -648,11 +653,16 @@ __global__ void __launch_bounds__(256)
 // channels and every gridDim.x-th batch of pixels, staged in shared memory; a
 // thread keeps 4 output channels x 9 taps of an input channel; with fewer
 // input channels the threads' slices of the batch are added up at the end.
-// Few CTAs, because each ends with an atomic per weight.  The proposer's
-// layers 2 and 1 (a CTA per 16 x 16 outputs and 8 input channels, every pixel):
-// 338 and 104 us.
-constexpr int kWgPix = 16;   // pixels per batch
+// Each CTA ends with an atomic per weight, so a few hundred pixels take
+// kWgCtas of them; more pixels take one per kWgPer, up to kWgMost (dx and dw of
+// 32 -> 32 channels over 300 x 300, every pixel listed: 0.72 ms with 64 CTAs, 0.37
+// with these). A CTA per 16 x 16 outputs and 8 input channels over every pixel
+// took 338 and 104 us in the proposer's layers 2 and 1.
+constexpr int kWgPix = 16;   // pixels per batch; with up to 8 input channels
+constexpr int kWgPixNarrow = 64;
 constexpr int kWgCtas = 64;
+constexpr int kWgPer = 32;
+constexpr int kWgMost = 592;
 
 template <int S>
 __global__ void __launch_bounds__(256)
@@ -661,15 +671,20 @@ __global__ void __launch_bounds__(256)
                          int relu, int64_t q0, int32_t nq, const int32_t* __restrict__ list,
                          const int32_t* __restrict__ count, float* __restrict__ dw,
                          float* __restrict__ db) {
-    __shared__ float xs[kWgPix * 32 * 9];          // [pixel][ci][tap]
-    __shared__ __align__(16) float dzs[kWgPix][32];  // [pixel][co]
-    __shared__ int2 at[kWgPix];                      // input row, column of tap 0
+    static_assert(kWgPixNarrow * 8 <= kWgPix * 32, "the narrow batch fits xs");
+    static_assert(4 * 128 <= kWgPix * 32, "the slices' sums fit xs");
+    __shared__ float xs[kWgPix * 32 * 9];                  // [pixel][ci][tap]
+    __shared__ __align__(16) float dzs[kWgPixNarrow][32];  // [pixel][co]
+    __shared__ int2 at[kWgPixNarrow];                      // input row, column of tap 0
     const bool all = count[1] & kDzAllX;  // (see k_dz_pixels)
     const int n = all ? nq : *count;
     const auto pixel = [&](int p) { return q0 + (all ? p : list[p]); };
+    const int ctas = max(kWgCtas, min((int)gridDim.x, (n + kWgPer - 1) / kWgPer));
+    if ((int)blockIdx.x >= ctas) return;
     const int ci0 = blockIdx.y * 32, co0 = blockIdx.z * 32;
     const int nci = min(32, Cin - ci0), nco = min(32, Cout - co0);
-    const int per = 8 * nci, slices = 256 / per;
+    const int npx = nci <= 8 ? kWgPixNarrow : kWgPix;
+    const int per = (nco + 3) / 4 * nci, slices = 256 / per;
     const int slice = threadIdx.x / per, cg = threadIdx.x % per / nci, ci = threadIdx.x % nci;
     const bool act = slice < slices;
     float acc[4][9], accb[4];
@@ -679,19 +694,22 @@ __global__ void __launch_bounds__(256)
 #pragma unroll
         for (int t = 0; t < 9; ++t) acc[c][t] = 0.f;
     }
-    for (int p0 = blockIdx.x * kWgPix; p0 < n; p0 += gridDim.x * kWgPix) {
-        const int np = min(kWgPix, n - p0);
+    for (int p0 = blockIdx.x * npx; p0 < n; p0 += ctas * npx) {
+        const int np = min(npx, n - p0);
         __syncthreads();  // the previous batch is consumed
         if (threadIdx.x < np) {
             const int64_t pix = pixel(p0 + threadIdx.x);
             at[threadIdx.x] = make_int2((int)(pix / Wo) * S - 1, (int)(pix % Wo) * S - 1);
         }
         __syncthreads();
-        for (int q = threadIdx.x; q < nci * 9; q += 256) {
+        // (with few input channels several pixels at a time)
+        const int row = nci * 9, pgs = row < 256 ? 256 / row : 1;
+        const int pg = row < 256 ? threadIdx.x / row : 0;
+        for (int q = threadIdx.x - pg * row; q < row && pg < pgs; q += 256) {
             const int c = q / 9, ky = q % 9 / 3, kx = q % 3;
             const float* xc = x + (int64_t)(ci0 + c) * H * W;
 #pragma unroll 8
-            for (int p = 0; p < np; ++p) {
+            for (int p = pg; p < np; p += pgs) {
                 const int iy = at[p].x + ky, ix = at[p].y + kx;
                 xs[p * nci * 9 + q] = (iy >= 0 && iy < H && ix >= 0 && ix < W)
                                           ? xc[(int64_t)iy * W + ix]
@@ -720,11 +738,12 @@ __global__ void __launch_bounds__(256)
             for (int c = 0; c < 4; ++c) accb[c] += d[c];
         }
     }
-    if (blockIdx.x * kWgPix >= n) return;
-    // the slices' sums, in shared memory where there are several
+    if (blockIdx.x * npx >= n) return;
+    // the slices' sums, in shared memory where there are several (two slices or
+    // more: per is at most 128, so nco nci is at most 512 and the sums fit xs)
     __syncthreads();
     if (slices > 1) {
-        for (int q = threadIdx.x; q < 32 * nci * 9; q += 256) xs[q] = 0.f;
+        for (int q = threadIdx.x; q < nco * nci * 9; q += 256) xs[q] = 0.f;
         for (int q = threadIdx.x; q < 32; q += 256) dzs[0][q] = 0.f;
         __syncthreads();
     }
@@ -1091,27 +1110,30 @@ static cudaError_t conv_bwd_t(const float* x, int Cin, int H, int W, const float
     int32_t* count = reinterpret_cast<int32_t*>(tmp);
     int32_t* list = reinterpret_cast<int32_t*>(tmp + 16);
     uint8_t* map = reinterpret_cast<uint8_t*>(list + band);
-    const dim3 gw(kWgCtas, blocks_for(Cin, 32), blocks_for(Cout, 32));
+    const int most = (int)std::min<int64_t>(kWgMost, (band + kWgPer - 1) / kWgPer);
+    const dim3 gw((unsigned)std::max(kWgCtas, most), blocks_for(Cin, 32), blocks_for(Cout, 32));
     for (int64_t q0 = 0; q0 < npix && e == cudaSuccess; q0 += band) {
         const int32_t nq = (int32_t)std::min(band, npix - q0);
         e = cudaMemsetAsync(count, 0, q0 == 0 ? 8 : 4, st);
         if (e != cudaSuccess) break;
-        k_dz_pixels<<<blocks_for(nq, 256), 256, 0, st>>>(y, dy, relu, Cout, npix, q0, nq, x,
-                                                         (int64_t)Cin * H * W, w,
-                                                         (int64_t)Cout * Cin * 9, map, list, count);
+        // (the first launch wide enough for eight values of x a thread)
+        const int64_t nx = (int64_t)Cin * H * W;
+        const unsigned wide = q0 == 0 ? blocks_for(std::min<int64_t>(nx, 1 << 23), 2048) : 0;
+        k_dz_pixels<<<std::max(blocks_for(nq, 256), wide), 256, 0, st>>>(
+            y, dy, relu, Cout, npix, q0, nq, x, nx, w, (int64_t)Cout * Cin * 9, map, list, count);
         k_conv3x3_bwd_weight<S><<<gw, 256, 0, st>>>(x, Cin, H, W, Cout, Ho, Wo, y, dy, relu, q0,
                                                     nq, list, count, dw, db);
         count_launches(2);
         e = cudaGetLastError();
     }
     if (e == cudaSuccess && dx) {
-        const size_t sm = sizeof(float) * 9 * Cout * kBdCi;
-        e = cudaFuncSetAttribute(k_conv3x3_bwd_data<S>,
-                                 cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
+        const int CI = Cin <= 4 ? 4 : 32;
+        auto kern = CI == 4 ? k_conv3x3_bwd_data<S, 4> : k_conv3x3_bwd_data<S, 32>;
+        const size_t sm = sizeof(float) * 9 * Cout * CI;
+        e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
         if (e == cudaSuccess) {
-            const dim3 gd(blocks_for((int64_t)H * W, 256), blocks_for(Cin, kBdCi));
-            k_conv3x3_bwd_data<S><<<gd, 256, sm, st>>>(w, Cin, H, W, Cout, Ho, Wo, y, dy, relu,
-                                                       map, count, dx);
+            const dim3 gd(blocks_for((int64_t)H * W, 256), blocks_for(Cin, CI));
+            kern<<<gd, 256, sm, st>>>(w, Cin, H, W, Cout, Ho, Wo, y, dy, relu, map, count, dx);
             count_launches(1);
             e = cudaGetLastError();
         }
