@@ -266,12 +266,9 @@ struct pfx_batch {
     std::vector<std::vector<int32_t>> mask_slots, mask_lists;
     std::vector<std::vector<uint8_t>> mask_host, done;
     bool ran = false;  // a run since pfx_batch_set_masks
-    // path checks and row-layout copies (allocated on first use)
-    PathRef* pref = nullptr;  // filled on first use
-    bool pref_ready = false;
-    S2Pair* s2tab = nullptr;  // every pair's stage 2, in wave order (NaN beta: stale)
-    double s2tab_beta = 0.0;
-    int32_t* rows = nullptr;  // lo | hi block-row scratch
+    PathRef* pref = nullptr;  // every pair's path
+    S2Pair* s2tab = nullptr;  // every pair's stage 2, in wave order
+    int32_t* rows = nullptr;  // lo | hi block-row scratch of path checks (on first use)
     size_t rows_cap = 0;
 };
 
@@ -311,6 +308,22 @@ static void batch_free(pfx_batch* b) {
 }
 
 extern "C" void pfx_batch_destroy(pfx_batch* b) { batch_free(b); }
+
+// Every pair's stage 2 in wave order: the table of the waves' launches. It
+// depends on the waves alone, so it is written with them (pfx_batch_create,
+// pfx_batch_set_masks) and a run only reads it.
+static void stage2_table(const pfx_batch* b, const std::vector<int>& wave_pairs, S2Pair* tab) {
+    for (size_t q = 0; q < wave_pairs.size(); ++q) {
+        const pfx_plan& p = b->plans[wave_pairs[q]];
+        // (with the in-kernel cost no slabs are kept: costs from the features)
+        const S2Src src = b->gen_cost
+                              ? S2Src{nullptr, nullptr, 0, p.feat,
+                                      p.feat + (int64_t)b->d * p.g.N, b->d, 0}
+                              : S2Src{nullptr, p.Csk, p.skew_stride, nullptr, nullptr, 0,
+                                      p.fp32 != 0};
+        tab[q] = S2Pair{p.g, p.s2, src};
+    }
+}
 
 #define BCK(call)                                                                          \
     do {                                                                                   \
@@ -594,11 +607,32 @@ extern "C" int pfx_batch_create(int32_t n, const int64_t* N, const int64_t* M, c
             e = cudaMemcpy(b->gpairs, gp.data(), gp.size() * sizeof(GPair),
                            cudaMemcpyHostToDevice);
     }
-    // (here, not in the first run: a cudaMalloc can take milliseconds)
+    // the tables of stage 2 and of the paths (here, not in the first run: a
+    // cudaMalloc can take milliseconds)
     if (e == cudaSuccess) e = cudaMalloc(&b->s2tab, (size_t)n * sizeof(S2Pair));
-    b->s2tab_beta = NAN;
+    if (e == cudaSuccess) {
+        std::vector<S2Pair> tab((size_t)n);
+        stage2_table(b, b->wave_pairs, tab.data());
+        e = cudaMemcpy(b->s2tab, tab.data(), tab.size() * sizeof(S2Pair), cudaMemcpyHostToDevice);
+    }
     if (e == cudaSuccess) e = cudaMalloc(&b->pref, (size_t)n * sizeof(PathRef));
+    if (e == cudaSuccess) {
+        std::vector<PathRef> h((size_t)n);
+        int64_t to = 0, ro = 0;
+        for (int i = 0; i < n; ++i) {
+            const pfx_plan& p = b->plans[i];
+            h[i] = PathRef{p.s2.wp, p.s2.wp_len, p.tile_mask, p.g.N, p.g.M, p.g.n1, p.g.n2, p.g.L,
+                           0, to, ro};
+            to += (int64_t)p.g.n1 * p.g.n2;
+            ro += p.g.N + 2;  // block rows for any block size >= 1
+        }
+        e = cudaMemcpy(b->pref, h.data(), h.size() * sizeof(PathRef), cudaMemcpyHostToDevice);
+    }
     if (e == cudaSuccess) e = cudaMemset(b->status, 0, 4);
+    // the copies and fills above ran on the default stream, and a copy from
+    // pageable memory may return before it has arrived: nothing else orders
+    // them before a run on the caller's stream or the batch's own
+    if (e == cudaSuccess) e = cudaStreamSynchronize(nullptr);
     if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&b->cap, cudaStreamNonBlocking);
     for (int k = 0; k < kSide && e == cudaSuccess; ++k) {
         e = cudaStreamCreateWithFlags(&b->side[k], cudaStreamNonBlocking);
@@ -684,7 +718,7 @@ extern "C" int pfx_batch_set_masks(pfx_batch* b, const uint8_t* masks, int32_t o
     }
     int64_t kept_total = 0;
     for (int i = 0; i < n; ++i) kept_total += kept_n[i];
-    need += al16((size_t)kept_total * sizeof(TileDesc));
+    need += al16((size_t)kept_total * sizeof(TileDesc)) + al16((size_t)n * sizeof(S2Pair));
     const size_t table_cap = (size_t)6 * n + (need >> 16) + 16;  // chunks of <= 64 KB
     need += table_cap * sizeof(CopySeg);
     BCK(cudaStreamSynchronize(s));  // the staging buffers may still feed earlier copies
@@ -774,6 +808,8 @@ extern "C" int pfx_batch_set_masks(pfx_batch* b, const uint8_t* masks, int32_t o
         for (const TileDesc* d : kv) qall[qo++] = *d;
         wt.push_back((int64_t)kv.size());
     }
+    stage2_table(b, wave_pairs, reinterpret_cast<S2Pair*>(
+                                    reserve(b->s2tab, (size_t)n * sizeof(S2Pair))));
     if (segs.size() > table_cap)
         return errf(PFX_ERR_TOO_LARGE, "copy table: %zu segments > %zu", segs.size(), table_cap);
     const size_t toff = so;
@@ -794,7 +830,6 @@ extern "C" int pfx_batch_set_masks(pfx_batch* b, const uint8_t* masks, int32_t o
     b->max_wave_tiles = 0;
     for (int64_t x : wt) b->max_wave_tiles = std::max(b->max_wave_tiles, x);
     b->masked = 1;
-    b->s2tab_beta = NAN;  // the waves changed
     if (b->exec) {
         cudaGraphExecDestroy(b->exec);
         b->exec = nullptr;
@@ -972,7 +1007,7 @@ extern "C" int pfx_batch_plan(pfx_batch* b, int32_t i, pfx_plan** plan) {
 
 // The launch sequence of one batch run, on stream s (captured or direct;
 // `timed` records the phase events, direct runs only).
-static int batch_enqueue(pfx_batch* b, cudaStream_t s, bool timed) {
+static int batch_enqueue(pfx_batch* b, double beta, cudaStream_t s, bool timed) {
     const int waves = (int)b->wave_first.size() - 1;
     BCK(cudaMemsetAsync(b->heads, 0, (size_t)waves * sizeof(int), s));
     if (timed && b->phase_ev.empty()) {
@@ -1073,7 +1108,7 @@ static int batch_enqueue(pfx_batch* b, cudaStream_t s, bool timed) {
         used_side = std::max(used_side, w % kSide + 1);
         BCK(cudaStreamWaitEvent(ss, b->fork_ev, 0));
         BCK(launch_stage2_prop(one, tab, q1 - q0, ss));
-        BCK(launch_sync_scan(one, tab, q1 - q0, ss));
+        BCK(launch_sync_scan(one, tab, q1 - q0, beta, ss));
         BCK(launch_stitch(one, tab, q1 - q0, ss, 1, 0, 0, 0, 0));
     }
     for (int k = 0; k < used_side; ++k) {
@@ -1092,26 +1127,7 @@ extern "C" int pfx_batch_run(pfx_batch* b, double beta, int32_t use_graph, void*
         b->done = b->mask_host;
         b->ran = true;
     }
-    if (b->s2tab_beta != beta) {
-        // every pair's stage 2 in wave order (waves and beta are fixed until
-        // the next pfx_batch_set_masks or another beta)
-        BCK(cudaStreamSynchronize(s));  // an earlier run may still read the table
-        std::vector<S2Pair> tab((size_t)b->n);
-        for (int q = 0; q < b->n; ++q) {
-            const pfx_plan& p = b->plans[b->wave_pairs[q]];
-            // (with the in-kernel cost no slabs are kept: costs from the features)
-            const S2Src src = b->gen_cost
-                                  ? S2Src{nullptr, nullptr, 0, p.feat,
-                                          p.feat + (int64_t)b->d * p.g.N, b->d, 0}
-                                  : S2Src{nullptr, p.Csk, p.skew_stride, nullptr, nullptr, 0,
-                                          p.fp32 != 0};
-            tab[q] = S2Pair{p.g, p.s2, buffer_global(p.g.N, p.g.M, beta), src};
-        }
-        BCK(cudaMemcpy(b->s2tab, tab.data(), tab.size() * sizeof(S2Pair),
-                       cudaMemcpyHostToDevice));
-        b->s2tab_beta = beta;
-    }
-    if (!use_graph) return batch_enqueue(b, s, true);
+    if (!use_graph) return batch_enqueue(b, beta, s, true);
     if (!b->exec || b->graph_beta != beta) {
         if (b->exec) {
             cudaGraphExecDestroy(b->exec);
@@ -1122,7 +1138,7 @@ extern "C" int pfx_batch_run(pfx_batch* b, double beta, int32_t use_graph, void*
         BCK(cudaStreamWaitEvent(b->cap, b->fork_ev, 0));
         BCK(cudaStreamBeginCapture(b->cap, cudaStreamCaptureModeRelaxed));
         const int64_t k0 = pfx_kernel_launches();
-        const int st = batch_enqueue(b, b->cap, false);
+        const int st = batch_enqueue(b, beta, b->cap, false);
         // recorded launches run at each replay: count them there, not here
         b->graph_kernels = pfx_kernel_launches() - k0;
         count_launches(-(int)b->graph_kernels);
@@ -1193,30 +1209,12 @@ extern "C" int pfx_batch_results(pfx_batch* b, void* stream, double* best_cost, 
     return PFX_OK;
 }
 
-static int ensure_pref(pfx_batch* b) {
-    if (b->pref_ready) return PFX_OK;
-    std::vector<PathRef> h((size_t)b->n);
-    int64_t to = 0, ro = 0;
-    for (int i = 0; i < b->n; ++i) {
-        const pfx_plan& p = b->plans[i];
-        h[i] = PathRef{p.s2.wp, p.s2.wp_len, p.tile_mask, p.g.N, p.g.M, p.g.n1, p.g.n2, p.g.L,
-                       0, to, ro};
-        to += (int64_t)p.g.n1 * p.g.n2;
-        ro += p.g.N + 2;  // block rows for any block size >= 1
-    }
-    BCK(cudaMemcpy(b->pref, h.data(), h.size() * sizeof(PathRef), cudaMemcpyHostToDevice));
-    b->pref_ready = true;
-    return PFX_OK;
-}
-
 extern "C" int pfx_batch_check_paths(pfx_batch* b, int32_t margin, uint8_t* near, int32_t* flags,
                                      void* stream) {
     if (!b || !near || !flags) return errf(PFX_ERR_ARG, "null argument");
     if (margin < 1) return errf(PFX_ERR_ARG, "margin %d", margin);
     if (!b->masked) return errf(PFX_ERR_ARG, "pfx_batch_check_paths needs a masked batch");
     cudaStream_t s = (cudaStream_t)stream;
-    int st = ensure_pref(b);
-    if (st) return st;
     size_t rows = 0;
     for (int i = 0; i < b->n; ++i) rows += (size_t)b->plans[i].g.N + 2;
     if (rows * 2 > b->rows_cap) {
@@ -1276,8 +1274,6 @@ extern "C" int pfx_batch_copy_paths_rows(pfx_batch* b, void* stream, int64_t* ho
                         (long long)lens[i], (long long)offsets[i], (long long)cap);
         total = std::max(total, offsets[i] + lens[i]);
     }
-    int st = ensure_pref(b);
-    if (st) return st;
     PathStage ps(s);
     BCK(ps.alloc(total, b->n));
     std::vector<int64_t> ol((size_t)2 * b->n);
@@ -1324,8 +1320,6 @@ extern "C" int pfx_batch_copy_paths(pfx_batch* b, void* stream, int64_t* wp_host
                 BCK(cudaMemcpyAsync(wp_host + 2 * offsets[i], b->plans[i].s2.wp,
                                     (size_t)ol[n + i] * 16, cudaMemcpyDeviceToHost, s));
     } else if (total > 0) {
-        int st = ensure_pref(b);
-        if (st) return st;
         PathStage ps(s);
         BCK(ps.alloc(total, n));
         BCK(cudaMemcpyAsync(ps.off, ol.data(), ol.size() * 8, cudaMemcpyHostToDevice, s));

@@ -621,20 +621,20 @@ extern "C" int pfx_stage2_edges(pfx_plan* p, const double* C, int64_t ldc, void*
         // the overlap costs come from the normalised features
         const S2Src src{nullptr, nullptr, 0, p->feat, p->feat + (int64_t)p->feat_d * g.N,
                         p->feat_d, 0};
-        CK(launch_stage2_edges(S2Pair{g, p->s2, 0, src}, nullptr, 1, (cudaStream_t)stream));
+        CK(launch_stage2_edges(S2Pair{g, p->s2, src}, nullptr, 1, (cudaStream_t)stream));
         return PFX_OK;
     }
     // the FP32 form reads overlap costs from its own FP32 slabs (the values
     // its DP used), never from an FP64 C
     const S2Src src{p->fp32 ? nullptr : C, p->Csk, p->skew_stride, nullptr, nullptr, 0,
                     p->fp32 != 0};
-    CK(launch_stage2_edges(S2Pair{g, p->s2, 0, src}, nullptr, 1, (cudaStream_t)stream));
+    CK(launch_stage2_edges(S2Pair{g, p->s2, src}, nullptr, 1, (cudaStream_t)stream));
     return PFX_OK;
 }
 
 extern "C" int pfx_stage2_prop(pfx_plan* p, void* stream) {
     if (!p) return fail(PFX_ERR_ARG, "null plan");
-    CK(launch_stage2_prop(S2Pair{p->g, p->s2, 0}, nullptr, 1, (cudaStream_t)stream));
+    CK(launch_stage2_prop(S2Pair{p->g, p->s2, {}}, nullptr, 1, (cudaStream_t)stream));
     return PFX_OK;
 }
 
@@ -652,24 +652,16 @@ extern "C" int pfx_snapshot_prop(pfx_plan* p, void* stream) {
     return PFX_OK;
 }
 
-int64_t pfx::buffer_global(int64_t N, int64_t M, double beta) {
-    // Parflex.py:1520, evaluated in the same order
-    const double mn = (double)(N < M ? N : M), mx = (double)(N < M ? M : N);
-    const double bg = mn * (1 - (1 - beta) * mn / mx);
-    return (int64_t)bg;
-}
-
 extern "C" int pfx_stage2_scan(pfx_plan* p, double beta, void* stream) {
     if (!p) return fail(PFX_ERR_ARG, "null plan");
-    CK(launch_sync_scan(S2Pair{p->g, p->s2, buffer_global(p->g.N, p->g.M, beta)}, nullptr, 1,
-                        (cudaStream_t)stream));
+    CK(launch_sync_scan(S2Pair{p->g, p->s2, {}}, nullptr, 1, beta, (cudaStream_t)stream));
     return PFX_OK;
 }
 
 extern "C" int pfx_stage2_stitch(pfx_plan* p, int from_best, int64_t i, int64_t j, int64_t edge,
                                  int64_t idx, void* stream) {
     if (!p) return fail(PFX_ERR_ARG, "null plan");
-    CK(launch_stitch(S2Pair{p->g, p->s2, 0}, nullptr, 1, (cudaStream_t)stream, from_best, i, j,
+    CK(launch_stitch(S2Pair{p->g, p->s2, {}}, nullptr, 1, (cudaStream_t)stream, from_best, i, j,
                      edge, idx));
     return PFX_OK;
 }

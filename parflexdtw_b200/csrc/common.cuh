@@ -343,11 +343,10 @@ struct S2Src {
     const double *An, *Bn;
     int32_t d, f32;
 };
-// One alignment of a stage-2 launch (buf: the scan's global buffer).
+// One alignment of a stage-2 launch.
 struct S2Pair {
     Geo g;
     S2Buf b;
-    int64_t buf;
     S2Src src;
 };
 // Stage 2 of one alignment (tab null) or of the npairs in the device table tab;
@@ -356,7 +355,8 @@ struct S2Pair {
 // slabs); propagation; overlap sync and edge scan; stitched backtrace.
 cudaError_t launch_stage2_edges(const S2Pair& one, const S2Pair* tab, int npairs, cudaStream_t st);
 cudaError_t launch_stage2_prop(const S2Pair& one, const S2Pair* tab, int npairs, cudaStream_t st);
-cudaError_t launch_sync_scan(const S2Pair& one, const S2Pair* tab, int npairs, cudaStream_t st);
+cudaError_t launch_sync_scan(const S2Pair& one, const S2Pair* tab, int npairs, double beta,
+                             cudaStream_t st);
 cudaError_t launch_stitch(const S2Pair& one, const S2Pair* tab, int npairs, cudaStream_t st,
                           int from_best, int64_t si, int64_t sj, int64_t se, int64_t sx);
 // The tile chain of the stitched backtrace alone (b.chain, b.chain_len): it

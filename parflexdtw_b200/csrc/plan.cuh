@@ -76,6 +76,4 @@ inline int64_t plan_slab_bytes(const pfx_plan* p) {
     return slabs * p->skew_stride * (p->fp32 ? 4 : 8);
 }
 int num_sms_cur();
-// The scan's global buffer (Parflex.py:1520).
-int64_t buffer_global(int64_t N, int64_t M, double beta);
 }  // namespace pfx

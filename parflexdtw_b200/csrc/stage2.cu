@@ -423,15 +423,25 @@ __device__ __forceinline__ void block_first_min(double& n, int64_t& i, double* s
 // (Parflex.py:1167-1168).
 constexpr int kScanThreads = 1024;
 
+// buffer_global (Parflex.py:1520), every operation rounded in its order; one
+// that is no int64 excludes nothing.
+__device__ __forceinline__ int64_t buffer_global(int64_t N, int64_t M, double beta) {
+    const double mn = (double)(N < M ? N : M), mx = (double)(N < M ? M : N);
+    const double part = __ddiv_rn(__dmul_rn(__dsub_rn(1.0, beta), mn), mx);
+    const double bg = __dmul_rn(mn, __dsub_rn(1.0, part));
+    return fabs(bg) < 0x1p63 ? (int64_t)bg : 0;
+}
+
 __global__ void __launch_bounds__(kScanThreads) k_scan(const S2Pair one,
-                                                       const S2Pair* __restrict__ tab) {
+                                                       const S2Pair* __restrict__ tab,
+                                                       const double beta) {
     __shared__ double sn[32];
     __shared__ int64_t si[32];
     cg::cluster_group cl = cg::this_cluster();
     const S2Pair& p = tab ? tab[blockIdx.y] : one;
     const Geo g = p.g;
     const S2Buf b = p.b;
-    const int64_t buf = p.buf;
+    const int64_t buf = buffer_global(g.N, g.M, beta);
     const int nb = (int)cl.num_blocks(), rank = (int)cl.block_rank();
     const int nthr = nb * kScanThreads, tid = rank * kScanThreads + (int)threadIdx.x;
     const int nt = g.n1 * g.n2;
@@ -795,9 +805,9 @@ cudaError_t launch_stage2_edges(const S2Pair& one, const S2Pair* tab, int npairs
 }
 
 // A kernel on clusters of cn CTAs, one cluster per alignment.
-template <typename K>
-static cudaError_t launch_clusters(K kern, int cn, int npairs, int threads, const S2Pair& one,
-                                   const S2Pair* tab, cudaStream_t st) {
+template <typename K, typename... More>
+static cudaError_t launch_clusters(K kern, int cn, int npairs, int threads, cudaStream_t st,
+                                   const S2Pair& one, const S2Pair* tab, More... more) {
     cudaLaunchConfig_t cfg = {};
     cudaLaunchAttribute attr[1];
     attr[0].id = cudaLaunchAttributeClusterDimension;
@@ -809,7 +819,7 @@ static cudaError_t launch_clusters(K kern, int cn, int npairs, int threads, cons
     cfg.stream = st;
     cfg.attrs = attr;
     cfg.numAttrs = 1;
-    const cudaError_t e = cudaLaunchKernelEx(&cfg, kern, one, tab);
+    const cudaError_t e = cudaLaunchKernelEx(&cfg, kern, one, tab, more...);
     count_launches(1);
     return e;
 }
@@ -831,14 +841,16 @@ cudaError_t launch_stage2_prop(const S2Pair& one, const S2Pair* tab, int npairs,
     if (e != cudaSuccess) return e;
     // about one slot in eight is valid; a cluster takes 512 to 4096 at once
     return launch_clusters(k_propagate, cluster_for((int64_t)std::min(g.n1, g.n2) * g.L),
-                           npairs, kPropThreads, one, tab, st);
+                           npairs, kPropThreads, st, one, tab);
 }
 
-cudaError_t launch_sync_scan(const S2Pair& one, const S2Pair* tab, int npairs, cudaStream_t st) {
+cudaError_t launch_sync_scan(const S2Pair& one, const S2Pair* tab, int npairs, double beta,
+                             cudaStream_t st) {
     // a CTA per two segments, up to 8
     const int64_t segs = 2 * std::max((one.g.N + one.g.L - 1) / one.g.L,
                                       (one.g.M + one.g.L - 1) / one.g.L);
-    return launch_clusters(k_scan, cluster_for(segs * 1024), npairs, kScanThreads, one, tab, st);
+    return launch_clusters(k_scan, cluster_for(segs * 1024), npairs, kScanThreads, st, one, tab,
+                           beta);
 }
 
 cudaError_t launch_stitch_chain(const Geo& g, const S2Buf& b, cudaStream_t st, int from_best,
