@@ -1323,9 +1323,12 @@ extern "C" int pfx_batch_copy_paths(pfx_batch* b, void* stream, int64_t* wp_host
         PathStage ps(s);
         BCK(ps.alloc(total, n));
         BCK(cudaMemcpyAsync(ps.off, ol.data(), ol.size() * 8, cudaMemcpyHostToDevice, s));
-        k_path_pack<<<dim3(16, n), 256, 0, s>>>(b->pref, ps.off, ps.len, ps.rows);
-        count_launches(1);
-        BCK(cudaGetLastError());
+        BCK(for_pairs(n, [&](int q, int m) {
+            k_path_pack<<<dim3(16, (unsigned)m), 256, 0, s>>>(b->pref + q, ps.off + q, ps.len + q,
+                                                             ps.rows);
+            count_launches(1);
+            return cudaGetLastError();
+        }));
         BCK(cudaMemcpyAsync(wp_host + 2 * offsets[0], ps.rows, (size_t)total * 16,
                             cudaMemcpyDeviceToHost, s));
     }

@@ -349,6 +349,16 @@ struct S2Pair {
     S2Buf b;
     S2Src src;
 };
+// Grids hold at most 65535 pairs in y: f(first, count) for every run of a
+// table's pairs that one launch takes.
+constexpr int kPairsPerLaunch = 65535;
+template <typename F>
+cudaError_t for_pairs(int npairs, F f) {
+    cudaError_t e = cudaSuccess;
+    for (int q = 0; q < npairs && e == cudaSuccess; q += kPairsPerLaunch)
+        e = f(q, npairs - q < kPairsPerLaunch ? npairs - q : kPairsPerLaunch);
+    return e;
+}
 // Stage 2 of one alignment (tab null) or of the npairs in the device table tab;
 // `one` then holds the largest n1, n2, L, N and M of the table, which size the
 // launches.  The edge tensors and valid marks (the only part that reads the cost

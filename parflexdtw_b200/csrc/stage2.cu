@@ -791,17 +791,21 @@ cudaError_t launch_fill(double* p, int64_t n, double v, cudaStream_t st) {
 cudaError_t launch_stage2_edges(const S2Pair& one, const S2Pair* tab, int npairs,
                                 cudaStream_t st) {
     const int64_t nslots = (int64_t)one.g.n1 * one.g.n2 * 2 * one.g.L;
-    const dim3 grid((unsigned)std::min<int64_t>((nslots + 255) / 256, 8192), (unsigned)npairs);
-    if (tab) {
-        k_clear_valid<<<dim3((grid.x + 15) / 16, grid.y), 256, 0, st>>>(tab);
-        count_launches(1);
-    } else {
+    const unsigned blocks = (unsigned)std::min<int64_t>((nslots + 255) / 256, 8192);
+    if (!tab) {
         const cudaError_t e = cudaMemsetAsync(one.b.valid, 0, (size_t)nslots, st);
         if (e != cudaSuccess) return e;
     }
-    k_edges<<<grid, 256, 0, st>>>(one, tab);
-    count_launches(1);
-    return cudaGetLastError();
+    return for_pairs(npairs, [&](int q, int n) {
+        const S2Pair* t = tab ? tab + q : nullptr;
+        if (t) {
+            k_clear_valid<<<dim3((blocks + 15) / 16, (unsigned)n), 256, 0, st>>>(t);
+            count_launches(1);
+        }
+        k_edges<<<dim3(blocks, (unsigned)n), 256, 0, st>>>(one, t);
+        count_launches(1);
+        return cudaGetLastError();
+    });
 }
 
 // A kernel on clusters of cn CTAs, one cluster per alignment.
@@ -814,14 +818,15 @@ static cudaError_t launch_clusters(K kern, int cn, int npairs, int threads, cuda
     attr[0].val.clusterDim.x = (unsigned)cn;
     attr[0].val.clusterDim.y = 1;
     attr[0].val.clusterDim.z = 1;
-    cfg.gridDim = dim3((unsigned)cn, (unsigned)npairs);
     cfg.blockDim = dim3((unsigned)threads);
     cfg.stream = st;
     cfg.attrs = attr;
     cfg.numAttrs = 1;
-    const cudaError_t e = cudaLaunchKernelEx(&cfg, kern, one, tab, more...);
-    count_launches(1);
-    return e;
+    return for_pairs(npairs, [&](int q, int n) {
+        cfg.gridDim = dim3((unsigned)cn, (unsigned)n);
+        count_launches(1);
+        return cudaLaunchKernelEx(&cfg, kern, one, tab ? tab + q : nullptr, more...);
+    });
 }
 
 // CTAs per alignment for `work` items: one per 2048, 1 to 8, a power of two.
@@ -835,9 +840,12 @@ cudaError_t launch_stage2_prop(const S2Pair& one, const S2Pair* tab, int npairs,
     const Geo& g = one.g;
     const int64_t nslots = (int64_t)g.n1 * g.n2 * 2 * g.L;
     const int64_t blocks = std::min<int64_t>((nslots + 255) / 256, 8192);
-    k_valid_lists<<<dim3((unsigned)blocks, (unsigned)npairs), 256, 0, st>>>(one, tab);
-    count_launches(1);
-    cudaError_t e = cudaGetLastError();
+    const cudaError_t e = for_pairs(npairs, [&](int q, int n) {
+        k_valid_lists<<<dim3((unsigned)blocks, (unsigned)n), 256, 0, st>>>(one,
+                                                                          tab ? tab + q : nullptr);
+        count_launches(1);
+        return cudaGetLastError();
+    });
     if (e != cudaSuccess) return e;
     // about one slot in eight is valid; a cluster takes 512 to 4096 at once
     return launch_clusters(k_propagate, cluster_for((int64_t)std::min(g.n1, g.n2) * g.L),
@@ -864,14 +872,14 @@ cudaError_t launch_stitch(const S2Pair& one, const S2Pair* tab, int npairs, cuda
                           int from_best, int64_t si, int64_t sj, int64_t se, int64_t sx) {
     // a path crosses at most n1 + n2 - 1 tiles, and the stitch follows 101
     const int most = std::min(kChainMax, one.g.n1 + one.g.n2);
-    k_walk<<<dim3((unsigned)most, (unsigned)npairs), 32, 0, st>>>(
-        one, tab, ChainStart{si, sj, se, sx, from_best});
-    count_launches(1);
-    cudaError_t e = cudaGetLastError();
-    if (e != cudaSuccess) return e;
-    k_concat<<<dim3((unsigned)most, (unsigned)npairs), 256, 0, st>>>(one, tab);
-    count_launches(1);
-    return cudaGetLastError();
+    return for_pairs(npairs, [&](int q, int n) {
+        const dim3 grid((unsigned)most, (unsigned)n);
+        const S2Pair* t = tab ? tab + q : nullptr;
+        k_walk<<<grid, 32, 0, st>>>(one, t, ChainStart{si, sj, se, sx, from_best});
+        k_concat<<<grid, 256, 0, st>>>(one, t);
+        count_launches(2);
+        return cudaGetLastError();
+    });
 }
 
 }  // namespace pfx
