@@ -113,8 +113,7 @@ class Batch:
         if len(pairs) != self.n:
             raise ValueError(f"{len(pairs)} pairs for a batch of {self.n}")
         here = torch.cuda.current_device() == self.device
-        ptrs = (ct.c_void_p * (2 * self.n))()
-        keep, rest = [], []  # keep: alive until the copies are submitted
+        items = []  # (pair, 0 or 1, tensor, whether one launch may take it)
         for i, pair in enumerate(pairs):
             F1, F2 = pair
             for k, src in ((0, F1), (1, F2)):
@@ -123,18 +122,30 @@ class Batch:
                 want = (self.d, self.shapes[i][k])
                 if tuple(t.shape) != want:
                     raise ValueError(f"pair {i}: features {tuple(t.shape)} for a buffer {want}")
-                if (here and type(t) is torch.Tensor and t.is_cuda
-                        and t.get_device() == self.device and t.dtype == torch.float64
-                        and t.layout == torch.strided and t.is_contiguous()
-                        and not t.requires_grad and not t.is_neg()):
+                items.append((i, k, t, here and type(t) is torch.Tensor and t.is_cuda
+                              and t.get_device() == self.device and t.dtype == torch.float64
+                              and t.layout == torch.strided and t.is_contiguous()
+                              and not t.requires_grad and not t.is_neg()))
+        # in the order given, as a source may be one of the batch's own buffers;
+        # device arrays as they are, up to 128 of a run of them in one launch
+        views, at = (-1, None), 0
+        while at < len(items):
+            end = at
+            while end < len(items) and items[end][3]:
+                end += 1
+            if end > at:
+                ptrs = (ct.c_void_p * (2 * self.n))()
+                for i, k, t, _ in items[at:end]:
                     ptrs[2 * i + k] = t.data_ptr()
-                    keep.append(t)
-                else:
-                    rest.append((i, k, t))
-        if keep:  # device arrays as they are: one launch for up to 128 of them
-            _lib.check(_lib.load().pfx_batch_load_device(self._h, ptrs, current_stream_ptr()))
-        for i, k, t in rest:
-            self.feature_views(i)[k].copy_(t, non_blocking=non_blocking)
+                _lib.check(_lib.load().pfx_batch_load_device(self._h, ptrs,
+                                                             current_stream_ptr()))
+                at = end
+                continue
+            i, k, t, _ = items[at]
+            if views[0] != i:
+                views = i, self.feature_views(i)
+            views[1][k].copy_(t, non_blocking=non_blocking)
+            at += 1
 
     def set_masks(self, masks, stream=None):
         """Restrict each pair to its tile mask (a CUDA uint8 tensor holding
