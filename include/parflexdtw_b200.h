@@ -63,6 +63,11 @@ int pfx_version(void);
  * benchmarks. */
 int64_t pfx_kernel_launches(void);
 
+/* Gives back the scratch memory that the library keeps between calls (up to 256
+ * MB per device); what a call in flight still uses stays.  No reference
+ * counterpart. */
+int pfx_scratch_trim(void);
+
 /* ---------------------------------------------------------------------------
  * Plans.  A plan fixes (N, M, L, steps, weights) and owns the device
  * workspace of one alignment: stage-1 edge tensors and packed backpointers

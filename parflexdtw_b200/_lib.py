@@ -45,6 +45,7 @@ SIGNATURES = [
     ("pfx_last_error", ct.c_char_p, []),
     ("pfx_version", ct.c_int, []),
     ("pfx_kernel_launches", ct.c_int64, []),
+    ("pfx_scratch_trim", ct.c_int, []),
     ("pfx_plan_create", ct.c_int, [_i64, _i64, _i32, _i64p, _f64p, _i32, ct.POINTER(_vp)]),
     ("pfx_plan_create_ex", ct.c_int, [_i64, _i64, _i32, _i64p, _f64p, _i32, _i32,
                                       ct.POINTER(_vp)]),

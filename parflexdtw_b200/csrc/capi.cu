@@ -365,17 +365,19 @@ extern "C" int pfx_plan_buffer(pfx_plan* p, int which, void** ptr, int64_t* nbyt
     return PFX_OK;
 }
 
+constexpr int kScratchDevices = 64;
+static std::mutex scratch_mutex;
+static cudaMemPool_t scratch_pools[kScratchDevices] = {};  // by device, made on first use
+
 cudaError_t pfx::scratch_alloc(void** p, size_t bytes, cudaStream_t st) {
-    static std::mutex mu;
-    static cudaMemPool_t pools[64] = {};
     int dev = 0;
     cudaError_t e = cudaGetDevice(&dev);
     if (e != cudaSuccess) return e;
-    if (dev < 0 || dev >= 64) return cudaMallocAsync(p, bytes, st);
+    if (dev < 0 || dev >= kScratchDevices) return cudaMallocAsync(p, bytes, st);
     cudaMemPool_t pool;
     {
-        std::lock_guard<std::mutex> lock(mu);
-        if (!pools[dev]) {
+        std::lock_guard<std::mutex> lock(scratch_mutex);
+        if (!scratch_pools[dev]) {
             cudaMemPoolProps props = {};
             props.allocType = cudaMemAllocationTypePinned;
             props.location.type = cudaMemLocationTypeDevice;
@@ -383,11 +385,18 @@ cudaError_t pfx::scratch_alloc(void** p, size_t bytes, cudaStream_t st) {
             uint64_t keep = 256ull << 20;
             if ((e = cudaMemPoolCreate(&pool, &props)) != cudaSuccess) return e;
             cudaMemPoolSetAttribute(pool, cudaMemPoolAttrReleaseThreshold, &keep);
-            pools[dev] = pool;
+            scratch_pools[dev] = pool;
         }
-        pool = pools[dev];
+        pool = scratch_pools[dev];
     }
     return cudaMallocFromPoolAsync(p, bytes, pool, st);
+}
+
+extern "C" int pfx_scratch_trim(void) {
+    std::lock_guard<std::mutex> lock(scratch_mutex);
+    for (cudaMemPool_t pool : scratch_pools)
+        if (pool) CK(cudaMemPoolTrimTo(pool, 0));
+    return PFX_OK;
 }
 
 static int check_ldc(const pfx_plan* p, const double* C, int64_t ldc) {

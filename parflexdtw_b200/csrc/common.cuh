@@ -208,9 +208,9 @@ int report_status(int status, const char* msg);
 int parse_step_kinds(const int64_t* steps, const double* weights, int32_t n, Geo* g);
 
 // Stream-ordered scratch of a call (freed with cudaFreeAsync on its stream),
-// from a pool of the library's own that keeps up to 256 MB between calls: the
-// default pool gives its memory back at every synchronisation, and taking it
-// again costs more than the kernels that use it.
+// from a pool of the library's own that keeps up to 256 MB between calls (until
+// pfx_scratch_trim): the default pool gives its memory back at every
+// synchronisation, and taking it again costs more than the kernels that use it.
 cudaError_t scratch_alloc(void** p, size_t bytes, cudaStream_t st);
 
 // Count of kernels this library has launched (process-wide).

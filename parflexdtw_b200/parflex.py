@@ -492,11 +492,14 @@ def _lease_plan(N, M, Lb, steps, weights, owner) -> Plan:
 
 
 def clear_plan_cache():
-    """Release every pooled plan's device memory."""
+    """Release every pooled plan's device memory, and the scratch memory the
+    library keeps between calls."""
     for pool in _PLAN_POOL.values():
         for p in pool:
             p.close()
     _PLAN_POOL.clear()
+    if L._lib is not None:
+        L.check(L.load().pfx_scratch_trim())
 
 
 def _buffer_global(L1, L2, beta):
