@@ -268,6 +268,8 @@ struct pfx_batch {
     bool ran = false;  // a run since pfx_batch_set_masks
     PathRef* pref = nullptr;  // every pair's path
     S2Pair* s2tab = nullptr;  // every pair's stage 2, in wave order
+    int64_t* stage_pts = nullptr;  // staging of the path copies: stage_cap points and
+    int64_t stage_cap = 0;         // 2 n words
     int32_t* rows = nullptr;  // lo | hi block-row scratch of path checks (on first use)
     size_t rows_cap = 0;
 };
@@ -419,7 +421,11 @@ extern "C" int pfx_batch_create(int32_t n, const int64_t* N, const int64_t* M, c
         for (int i = 0; i < n; ++i) s += round256((size_t)d * (N[i] + M[i]) * 8);
         return s;
     }();
-    const size_t fixed = arena + fin_total + round256(b->total_tiles * sizeof(TileDesc)) + (1 << 20);
+    // a path's points: at most one per row and column, and a start per tile walk
+    int64_t stage_cap = 0;
+    for (int i = 0; i < n; ++i) stage_cap += N[i] + M[i] + 101;
+    const size_t path_bytes = round256(((size_t)2 * stage_cap + 2 * (size_t)n) * 8);
+    const size_t fixed = arena + fin_total + path_bytes + round256(b->total_tiles * sizeof(TileDesc)) + (1 << 20);
     int64_t budget = wave_bytes;
     // default: 70 % of the memory the batch's other buffers leave free
     if (budget <= 0) budget = (int64_t)((freeb > fixed ? freeb - fixed : 0) / 10 * 7);
@@ -494,6 +500,8 @@ extern "C" int pfx_batch_create(int32_t n, const int64_t* N, const int64_t* M, c
     arena += round256((size_t)n * sizeof(PairOut));
     const size_t off_res = arena;
     arena += round256((size_t)n * 9 * 8);
+    const size_t off_stage = arena;
+    arena += path_bytes;
     cudaError_t e = cudaMalloc(&b->arena, arena);
     if (e == cudaSuccess) e = cudaMemset(b->arena, 0, arena);
     if (e == cudaSuccess) e = cudaMalloc(&b->slabs, (size_t)pool);
@@ -511,6 +519,8 @@ extern "C" int pfx_batch_create(int32_t n, const int64_t* N, const int64_t* M, c
     b->status = reinterpret_cast<int32_t*>(b->arena + off_status);
     b->pout = reinterpret_cast<PairOut*>(b->arena + off_pout);
     b->res = reinterpret_cast<int64_t*>(b->arena + off_res);
+    b->stage_pts = reinterpret_cast<int64_t*>(b->arena + off_stage);
+    b->stage_cap = stage_cap;
     // pass 2: carve the plans
     b->fin_off.resize(n);
     std::vector<PairOut> po(n);
@@ -1236,28 +1246,34 @@ extern "C" int pfx_batch_check_paths(pfx_batch* b, int32_t margin, uint8_t* near
     return PFX_OK;
 }
 
-// Device staging of a call, in stream order: `total` path points, then every
-// pair's offset and length.
+// Device staging of `total` path points, then every pair's offset and length: the
+// batch's own, or scratch of the call where the caller's offsets ask for more
+// than the paths can need.
 struct PathStage {
     int64_t* rows = nullptr;
     int64_t* off = nullptr;
     int64_t* len = nullptr;
+    void* scratch = nullptr;
     cudaStream_t st;
     explicit PathStage(cudaStream_t s) : st(s) {}
     PathStage(const PathStage&) = delete;
     PathStage& operator=(const PathStage&) = delete;
     ~PathStage() {
-        if (rows) cudaFreeAsync(rows, st);
+        if (scratch) cudaFreeAsync(scratch, st);
     }
-    cudaError_t alloc(int64_t total, int n) {
-        const cudaError_t e =
-            scratch_alloc((void**)&rows, ((size_t)2 * total + 2 * (size_t)n) * 8, st);
-        if (e != cudaSuccess) {
-            rows = nullptr;
-            return e;
+    cudaError_t take(const pfx_batch* b, int64_t total) {
+        rows = b->stage_pts;
+        if (total > b->stage_cap) {
+            const cudaError_t e =
+                scratch_alloc(&scratch, ((size_t)2 * total + 2 * (size_t)b->n) * 8, st);
+            if (e != cudaSuccess) {
+                scratch = nullptr;
+                return e;
+            }
+            rows = static_cast<int64_t*>(scratch);
         }
-        off = rows + 2 * total;
-        len = off + n;
+        off = rows + 2 * std::max(total, (int64_t)0);
+        len = off + b->n;
         return cudaSuccess;
     }
 };
@@ -1275,7 +1291,7 @@ extern "C" int pfx_batch_copy_paths_rows(pfx_batch* b, void* stream, int64_t* ho
         total = std::max(total, offsets[i] + lens[i]);
     }
     PathStage ps(s);
-    BCK(ps.alloc(total, b->n));
+    BCK(ps.take(b, total));
     std::vector<int64_t> ol((size_t)2 * b->n);
     std::copy(offsets, offsets + b->n, ol.begin());
     std::copy(lens, lens + b->n, ol.begin() + b->n);
@@ -1314,14 +1330,14 @@ extern "C" int pfx_batch_copy_paths(pfx_batch* b, void* stream, int64_t* wp_host
         ol[n + i] = len;
         total += len;
     }
-    if (!dense) {
+    if (!dense || total > b->stage_cap) {
         for (int i = 0; i < n; ++i)
             if (ol[n + i] > 0)
                 BCK(cudaMemcpyAsync(wp_host + 2 * offsets[i], b->plans[i].s2.wp,
                                     (size_t)ol[n + i] * 16, cudaMemcpyDeviceToHost, s));
     } else if (total > 0) {
         PathStage ps(s);
-        BCK(ps.alloc(total, n));
+        BCK(ps.take(b, total));
         BCK(cudaMemcpyAsync(ps.off, ol.data(), ol.size() * 8, cudaMemcpyHostToDevice, s));
         BCK(for_pairs(n, [&](int q, int m) {
             k_path_pack<<<dim3(16, (unsigned)m), 256, 0, s>>>(b->pref + q, ps.off + q, ps.len + q,
