@@ -13,6 +13,7 @@
 
 #include "plan.cuh"
 #include "prop_list.cuh"
+#include "tile_shape.cuh"
 
 
 
@@ -814,17 +815,6 @@ extern "C" int pfx_cost_matrix_f64(const double* F1, const double* F2, int32_t d
     return PFX_OK;
 }
 
-// Whether a single tile goes through launch_tile_full: from the size where its
-// cluster pays for the two extra passes (one CTA against the cluster, with the
-// call's scratch allocation: 63 x 65 0.33 and 0.33 ms, 64 x 64 0.32 and 0.31,
-// 100 x 100 0.38 and 0.35, 300 x 300 0.70 and 0.50, 1500 x 1801 10.1 and 1.9,
-// 8000 x 9000 327 and 14), and not where the tile is a ribbon and the cluster has
-// one strip of a few rows or columns to share (3000 x 2: 1.79 and 1.87; 30 x
-// 3000: 2.26 and 1.72).
-static bool full_tile_on_cluster(int32_t R, int32_t W) {
-    return std::min(R, W) >= 16 && (int64_t)R * W >= 4096;
-}
-
 extern "C" int pfx_flexdtw_tile(const double* C, int64_t ldc, int32_t R, int32_t W,
                                 const int64_t* steps, const double* weights, int32_t n_steps,
                                 double* D, int32_t* P, int8_t* B, void* stream) {
@@ -846,7 +836,8 @@ extern "C" int pfx_flexdtw_tile(const double* C, int64_t ldc, int32_t R, int32_t
     g.b_words = tile_b_words(g.L);
     if ((st = check_smem(g.L, 8))) return st;
     cudaStream_t s = (cudaStream_t)stream;
-    if (full_tile_on_cluster(R, W)) {
+    const bool std_steps = g.S == 3 && g.kind[0] == 0 && g.kind[1] == 1 && g.kind[2] == 2;
+    if (full_tile_on_cluster(R, W, g.S, std_steps, stage1_model_steps(R, W, 32))) {
         bool done = false;
         CK(launch_tile_full(C, g, D, P, B, s, &done));
         if (done) return PFX_OK;
