@@ -26,6 +26,7 @@
 #include <vector>
 
 #include "stage1_dp.cuh"
+#include "tile_shape.cuh"
 
 namespace pfx {
 
@@ -226,17 +227,17 @@ static cudaError_t cl_config(const S1Mem& m, int cn, int nclusters, ClConfig* c)
     return cudaSuccess;
 }
 
-// max != null: only the number of clusters that can run at once.
+// max != null: only the number of clusters that can run at once; fit > 0: that
+// number, where the caller has it.
 template <int CW, bool STD, typename T, int QD, bool FULL>
 static cudaError_t cl_launch(const S1Mem& m, int cn, const TileDesc* descs, int ntiles, int* head,
                              const Geo& g, int32_t* status, cudaStream_t st, int* max,
-                             int2* Psk = nullptr) {
+                             int2* Psk = nullptr, int fit = 0) {
     auto kern = k_stage1_cl<CW, STD, T, QD, FULL>;
     ClConfig c;
     cudaError_t e = cl_config<CW, STD, T, QD, FULL>(m, cn, 1, &c);
     if (e != cudaSuccess) return e;
-    int fit = 0;
-    e = cudaOccupancyMaxActiveClusters(&fit, kern, &c.cfg);
+    if (fit <= 0) e = cudaOccupancyMaxActiveClusters(&fit, kern, &c.cfg);
     if (e != cudaSuccess) return e;
     if (max) {
         *max = fit;
@@ -331,14 +332,33 @@ cudaError_t launch_tile_full(const double* C, const Geo& g, double* D, int32_t* 
     *done = false;
     const int R = (int)g.N, W = (int)g.M;
     const int nS = ceil_div32(R, kStripRows);
+    const bool std_steps = g.S == 3 && g.kind[0] == 0 && g.kind[1] == 1 && g.kind[2] == 2;
     // as many warps as strips, four per SM up to 8 SMs, then eight
     const int cw = nS > 48 ? 8 : 4;
-    int cn = 1;
-    while (cn < 8 && cn * cw < nS) cn *= 2;
-    Geo gt = g;
-    const Sched2 s = make_sched2(g.L, g.L, cn * cw);
-    const S1Mem m = stage1_mem(s.lag, cw, cta_budget(16), 8, 4);
-    if (m.rb == 0 || m.qd == 0) return cudaSuccess;
+    S1Mem m;
+    TileDesc* dd = nullptr;
+    int* head = nullptr;
+    int2* Psk = nullptr;
+    int fit = 0;
+    // max: only how many clusters of cn CTAs can be resident
+    const auto cluster = [&](int cn, int* max) -> cudaError_t {
+#define PFX_FULL(CW)                                                                          \
+    (std_steps ? cl_launch<CW, true, double, 4, true>(m, cn, dd, 1, head, g, head + 1, st,    \
+                                                      max, Psk, fit)                          \
+               : cl_launch<CW, false, double, 4, true>(m, cn, dd, 1, head, g, head + 1, st,   \
+                                                       max, Psk, fit))
+        return cw == 8 ? PFX_FULL(8) : PFX_FULL(4);
+#undef PFX_FULL
+    };
+    const int cn = full_tile_ctas(nS, cw, [&](int n) {
+        m = stage1_mem(make_sched2(g.L, g.L, n * cw).lag, cw, cta_budget(16), 8, 4);
+        fit = 0;
+        if (m.rb == 0 || m.qd == 0) return false;
+        if (cluster(n, &fit) == cudaSuccess) return fit > 0;
+        cudaGetLastError();  // a shape that cannot be resident is no error of the caller's
+        return false;
+    });
+    if (cn == 0) return cudaSuccess;
     // scratch: slab and P (large: from the library's own pool, taking 60 MB from
     // the default one costs about 1.5 ms), and backpointers, edges, descriptor,
     // queue head and status
@@ -353,7 +373,7 @@ cudaError_t launch_tile_full(const double* C, const Geo& g, double* D, int32_t* 
         return cudaSuccess;
     }
     double* Dsk = reinterpret_cast<double*>(big);
-    int2* Psk = reinterpret_cast<int2*>(big + slab);
+    Psk = reinterpret_cast<int2*>(big + slab);
     TileDesc d;
     memset(&d, 0, sizeof(d));
     d.Csk = Dsk;
@@ -364,20 +384,13 @@ cudaError_t launch_tile_full(const double* C, const Geo& g, double* D, int32_t* 
     d.W = W;
     d.L = g.L;
     char* misc = tmp + bw + ed;
-    TileDesc* dd = reinterpret_cast<TileDesc*>(misc + 256);
-    int* head = reinterpret_cast<int*>(misc);
+    dd = reinterpret_cast<TileDesc*>(misc + 256);
+    head = reinterpret_cast<int*>(misc);
     k_one_tile<<<1, 1, 0, st>>>(d, dd, head);
     count_launches(1);
     cudaError_t e = cudaGetLastError();
-    if (e == cudaSuccess) e = launch_relayout_skew(C, g.ldc, gt, Dsk, 0, st);
-    const bool std_steps = g.S == 3 && g.kind[0] == 0 && g.kind[1] == 1 && g.kind[2] == 2;
-#define PFX_FULL(CW)                                                                           \
-    (std_steps ? cl_launch<CW, true, double, 4, true>(m, cn, dd, 1, head, g, head + 1, st,     \
-                                                      nullptr, Psk)                            \
-               : cl_launch<CW, false, double, 4, true>(m, cn, dd, 1, head, g, head + 1, st,    \
-                                                       nullptr, Psk))
-    if (e == cudaSuccess) e = cw == 8 ? PFX_FULL(8) : PFX_FULL(4);
-#undef PFX_FULL
+    if (e == cudaSuccess) e = launch_relayout_skew(C, g.ldc, g, Dsk, 0, st);
+    if (e == cudaSuccess) e = cluster(cn, nullptr);
     if (e == cudaSuccess) {
         k_unskew<<<dim3((unsigned)ceil_div32(W, 64), (unsigned)(2 * nS)), 256, 0, st>>>(
             Dsk, reinterpret_cast<const int*>(Psk), d.Bw, head + 1, R, W, D, P, B);

@@ -33,4 +33,15 @@ inline bool full_tile_on_cluster(int32_t R, int32_t W, int steps, bool std_steps
     return one >= (steps == 1 ? 1.1 : 1.6) * cluster_steps;
 }
 
+// CTAs of cw warps for a tile of `strips` strips: a warp per strip up to 8
+// CTAs, or as many (a power of two) as can be resident together here: fits(n)
+// says whether a cluster of n can. 0: none can.
+template <typename F>
+inline int full_tile_ctas(int strips, int cw, F fits) {
+    int cn = 1;
+    while (cn < 8 && cn * cw < strips) cn *= 2;
+    while (cn > 0 && !fits(cn)) cn /= 2;
+    return cn;
+}
+
 }  // namespace pfx

@@ -12,6 +12,9 @@ SRC = r"""
 extern "C" int on_cluster(int32_t R, int32_t W, int steps, int std_steps, double n) {
     return pfx::full_tile_on_cluster(R, W, steps, std_steps != 0, n);
 }
+extern "C" int ctas(int strips, int cw, int most) {
+    return pfx::full_tile_ctas(strips, cw, [&](int n) { return n <= most; });
+}
 """
 
 
@@ -53,3 +56,14 @@ def test_the_faster_kernel(host, R, W):
     for steps, std, want in zip((1, 2, 3, 3), (0, 0, 0, 1), FASTER[R, W]):
         if want is not None:
             assert host.on_cluster(R, W, steps, std, n) == want
+
+
+@pytest.mark.parametrize("strips,cw,want", [(1, 4, 1), (4, 4, 1), (5, 4, 2), (16, 4, 4), (17, 4, 8),
+                                            (48, 4, 8), (49, 8, 8), (500, 8, 8)])
+def test_ctas(host, strips, cw, want):
+    """As many CTAs as the strips ask for, or what can be resident at once; 0
+    (the other kernel) where no cluster can."""
+    for most in (0, 1, 2, 3, 4, 7, 8, 16):
+        got = host.ctas(strips, cw, most)
+        fits = [n for n in (1, 2, 4, 8) if n <= min(want, most)]
+        assert got == (max(fits) if fits else 0)
