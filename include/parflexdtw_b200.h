@@ -255,9 +255,12 @@ int pfx_cost_matrix_f64(const double *F1, const double *F2, int32_t d,
 /* FlexDTW.flexdtw's DP on one R x W tile of C with full outputs
  * (FlexDTW.py:326-370; flexdtw_chunk_from_global_C, gpu_flexdtw.py:288-402):
  * D (f64), P (int32 start encoding) and B (int8 step index, -1 when no step
- * won), each R x W row-major on the device.  Tiles of 4096 cells or more take 12
- * bytes per cell of scratch in stream order where there is room (a slower
- * kernel without it where there is not). */
+ * won), each R x W row-major on the device.  Tiles of 4096 cells or more and
+ * 16 rows and columns or more may run on a cluster of CTAs, which takes scratch
+ * in stream order: 12.25 bytes per cell of the tile padded to 64 ceil(R / 64) rows
+ * of 16 ceil((W + 63) / 16) cells, and 24 bytes per row or column of the longer
+ * side.  Where there is no room for it, and for other tiles, a slower kernel
+ * takes 0.25 bytes per cell of a square of the longer side. */
 int pfx_flexdtw_tile(const double *C, int64_t ldc, int32_t R, int32_t W,
                      const int64_t *steps, const double *weights,
                      int32_t n_steps, double *D, int32_t *P, int8_t *B,

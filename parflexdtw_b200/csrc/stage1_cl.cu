@@ -363,8 +363,10 @@ cudaError_t launch_tile_full(const double* C, const Geo& g, double* D, int32_t* 
     // the default one costs about 1.5 ms), and backpointers, edges, descriptor,
     // queue head and status
     auto up = [](size_t b) { return (b + 255) & ~(size_t)255; };
-    const size_t slab = up((size_t)nS * ceil_div32(W + kStripRows - 1, kBlk) * kBlk * 64 * 8);
-    const size_t bw = up((size_t)tile_b_words2(g.L) * 4), ed = up((size_t)2 * g.L * 12);
+    // (the tile's own strips and periods, not those of an L x L tile)
+    const size_t words = (size_t)nS * ceil_div32(W + kStripRows - 1, kBlk) * kStripRows;
+    const size_t slab = up(words * kBlk * 8);
+    const size_t bw = up(words * 4), ed = up((size_t)2 * g.L * 12);
     char *big = nullptr, *tmp = nullptr;
     if (scratch_alloc((void**)&big, slab + slab / 2, st) != cudaSuccess ||
         cudaMallocAsync((void**)&tmp, bw + ed + 512, st) != cudaSuccess) {
