@@ -86,10 +86,20 @@ int pfx_plan_create_ex(int64_t N, int64_t M, int32_t L, const int64_t *steps,
                        pfx_plan **out);
 void pfx_plan_destroy(pfx_plan *plan);
 
-/* Stage-1 warps per tile CTA (4, 8 or 16; the plan picks one from its tile
- * count).  A masked run with few tiles is faster with 16.  No reference
- * counterpart. */
+/* Stage-1 warps per tile.  Without this call the plan picks them, and where it
+ * has few tiles spreads each over a cluster of CTAs.  4 or 8: one CTA of that
+ * many warps per tile, whatever the plan would take; 16: one CTA of 16 warps, or
+ * clusters where the plan would take those.  A masked run with few tiles is
+ * faster with 16.  No reference counterpart. */
 int pfx_plan_set_warps(pfx_plan *plan, int32_t nw);
+/* Undoes pfx_plan_set_warps. */
+int pfx_plan_default_warps(pfx_plan *plan);
+
+/* How the next pfx_stage1 without a mask runs the plan's tiles.  shape[0]: 0,
+ * every tile on one CTA of shape[1] warps; else the shape[2] largest tiles each
+ * on a cluster of shape[0] CTAs of shape[1] warps, the others on one CTA of 16
+ * warps.  No reference counterpart. */
+int pfx_plan_stage1_shape(pfx_plan *plan, int32_t *shape);
 
 /* info[0..7] = n1, n2, L, hop, n_steps, b_words_per_tile, device_bytes,
  * stage-1 warps per CTA. */

@@ -314,8 +314,37 @@ extern "C" int pfx_plan_set_warps(pfx_plan* p, int32_t nw) {
     if (!stage1_queue_fits(p->g.L, nw))
         return fail(PFX_ERR_TOO_LARGE, "L=%d: rings of %d warps do not fit", p->g.L, nw);
     p->nw = nw;
-    p->nw_set = nw != p->nw_default;
+    p->nw_set = 1;
     p->s1_planned = 0;
+    return PFX_OK;
+}
+
+extern "C" int pfx_plan_default_warps(pfx_plan* p) {
+    if (!p) return fail(PFX_ERR_ARG, "null plan");
+    p->nw = p->nw_default;
+    p->nw_set = 0;
+    p->s1_planned = 0;
+    return PFX_OK;
+}
+
+// How stage 1 runs p's tiles, decided once: it asks the driver what fits.
+static const S1Plan& stage1_shape(pfx_plan* p) {
+    if (!p->s1_planned) {
+        p->s1_plan = p->arena_mode == 0 && (!p->nw_set || p->nw == 16)
+                         ? stage1_plan(p->g, p->g.n1 * p->g.n2, p->fp32 != 0, num_sms_cur())
+                         : S1Plan{0, p->nw, 0};
+        if (p->s1_plan.cn == 0) p->s1_plan.cw = p->nw;
+        p->s1_planned = 1;
+    }
+    return p->s1_plan;
+}
+
+extern "C" int pfx_plan_stage1_shape(pfx_plan* p, int32_t* shape) {
+    if (!p || !shape) return fail(PFX_ERR_ARG, "null argument");
+    const S1Plan& s = stage1_shape(p);
+    shape[0] = s.cn;
+    shape[1] = s.cw;
+    shape[2] = s.big;
     return PFX_OK;
 }
 
@@ -577,15 +606,7 @@ extern "C" int pfx_stage1(pfx_plan* p, const double* C, int64_t ldc, void* strea
                                p->s1.status, p->nw, p->fp32 != 0, s));
     } else {
         const int nt = p->g.n1 * p->g.n2;
-        // (decided once per plan: it asks the driver what fits)
-        if (!p->s1_planned) {
-            p->s1_plan = p->arena_mode == 0 && (!p->nw_set || p->nw == 16)
-                             ? stage1_plan(p->g, nt, p->fp32 != 0, num_sms_cur())
-                             : S1Plan{0, p->nw, 0};
-            if (p->s1_plan.cn == 0) p->s1_plan.cw = p->nw;
-            p->s1_planned = 1;
-        }
-        const S1Plan& sp = p->s1_plan;
+        const S1Plan& sp = stage1_shape(p);
         if (sp.cn > 0) {
             // few tiles: the largest (the queue is ordered largest first) on
             // clusters, the others at the same time on a second stream

@@ -7,7 +7,7 @@
 struct pfx_plan {
     pfx::Geo g;
     int nw;      // warps per tile CTA of the stage-1 queue kernel
-    int nw_default, nw_set;  // the rule's choice; 1: the caller chose another
+    int nw_default, nw_set;  // the rule's choice; 1: the caller chose nw
     pfx::S1Plan s1_plan;     // how stage 1 runs the tiles (pfx_stage1 fills it in)
     int s1_planned;
     int device;

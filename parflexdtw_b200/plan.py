@@ -55,6 +55,8 @@ def _free_plan(handle):
 class Plan:
     """Geometry + device workspace for an N x M cost matrix with tile length L."""
 
+    warps_chosen = None  # what set_warps was called with, if it was
+
     def __init__(self, N, M, Lb, steps, weights, precision="fp64"):
         lib = L.load()
         if precision not in ("fp64", "fp32"):
@@ -196,9 +198,24 @@ class Plan:
             int(F1_dev.shape[0]), stream or current_stream_ptr()))
 
     def set_warps(self, nw):
-        """Stage-1 warps per tile CTA (4, 8 or 16)."""
+        """Stage-1 warps per tile: 4 or 8 in one CTA, or 16 (one CTA, or
+        clusters of CTAs where the plan would take those)."""
         L.check(L.load().pfx_plan_set_warps(self._h, int(nw)))
-        self.warps = int(nw)
+        self.warps = self.warps_chosen = int(nw)
+
+    def default_warps(self):
+        """Undo ``set_warps``: the plan's own choice, clusters included."""
+        L.check(L.load().pfx_plan_default_warps(self._h))
+        info = (ct.c_int64 * 8)()
+        L.check(L.load().pfx_plan_info(self._h, info))
+        self.warps, self.warps_chosen = int(info[7]), None
+
+    def stage1_shape(self):
+        """(CTAs of a tile's cluster, warps of a CTA, tiles on clusters) of the
+        next stage 1 without a mask; (0, warps, 0): one CTA per tile."""
+        out = (ct.c_int32 * 3)()
+        L.check(L.load().pfx_plan_stage1_shape(self._h, out))
+        return tuple(out)
 
     def set_tile_mask(self, mask=None, stream=None):
         """Restrict cost building and stage 1 to the tiles set in ``mask``

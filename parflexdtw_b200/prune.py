@@ -335,6 +335,13 @@ def _needs_fallback(wp, mask, N, M, L, margin=FALLBACK_MARGIN):
     return bool(_pruned_near_path(wp, mask, N, M, L, margin).any())
 
 
+def _restore_warps(plan, chosen):
+    if chosen is None:
+        plan.default_warps()
+    else:
+        plan.set_warps(chosen)
+
+
 def parflex_pruned(F1, F2, steps, weights, beta, L, proposer=None, threshold=None,
                    dilation=1, precision="fp64", plan=None, warps=None):
     """ParFlex from features with learned tile pruning.
@@ -358,7 +365,7 @@ def parflex_pruned(F1, F2, steps, weights, beta, L, proposer=None, threshold=Non
     total = plan.n1 * plan.n2
     info = {"tiles_total": total, "tiles_run": kept, "skipped_fraction": 1 - kept / total,
             "fallback": False, "reason": None}
-    full_warps = plan.warps
+    chosen = plan.warps_chosen
     best = wp = None
     if kept:
         plan.set_tile_mask(mask)
@@ -377,7 +384,7 @@ def parflex_pruned(F1, F2, steps, weights, beta, L, proposer=None, threshold=Non
         info.update(fallback=True, reason="no tile proposed")
     if info["fallback"]:
         plan.set_tile_mask(None)
-        plan.set_warps(full_warps)
+        _restore_warps(plan, chosen)
         plan.load_features(f1, f2)
         plan.run(None, beta)
         best, end, found, n = plan.result()
@@ -385,7 +392,7 @@ def parflex_pruned(F1, F2, steps, weights, beta, L, proposer=None, threshold=Non
         info["tiles_run"] = kept + total
     else:
         plan.set_tile_mask(None)
-        plan.set_warps(full_warps)
+        _restore_warps(plan, chosen)
     return best, np.ascontiguousarray(wp.T), info
 
 
