@@ -7,11 +7,7 @@
 #pragma once
 #include <stdint.h>
 
-#ifdef __CUDACC__
-#define PFX_HD __host__ __device__ __forceinline__
-#else
-#define PFX_HD inline
-#endif
+#include "host_device.cuh"
 
 namespace pfx {
 
