@@ -304,22 +304,20 @@ struct Wave {
 // of kBlk, and per-warp exchange entries, [NW][kXch].  At the start of its
 // step T (counted from the tile's start) every lane stores the pair {B one
 // step ago, A two steps ago} and loads its neighbour lane i-1's, which the
-// next step uses as x1 and x3.  Lanes 0..30 store into an exchange entry
-// (exchange.cuh; a step done again by the careful loop stores the same pair
-// again); lane 31 stores into ring slot (T - 64) mod RB, which then holds rows
-// 64k+63 and 64k+62 of column j = tau - 64; lane 0 loads ring slot (T' - lag) mod
-// RB of the previous strip, its column tau'.  So one address per lane takes the
+// next step uses as x1 and x3.  Lanes 0..30 store into their exchange entry
+// (exchange.cuh: one barrier of the warp per step, and another after even
+// ones); lane 31 stores into ring slot (T - 64) mod RB, which then holds rows
+// 64k+63 and 64k+62 of column j = tau - 64; lane 0 loads ring slot (T' - lag) mod RB
+// of the previous strip, its column tau'.  So one address per lane takes the
 // place of shuffles, of the ring's own loads and stores and of the selects
-// between the two; all of them move one place per step.  Both ring windows of a
-// block start on a multiple of kBlk: no address inside a block wraps, and a
-// ring slot lies in the bank that lane 31's (lane 0's) own entry leaves free.
-// D is one {B, A} vector, the start encodings one {B, A} int2.
+// between the two.  Both ring windows of a block start on a multiple of
+// kBlk: no address inside a block wraps.  D is one {B, A} vector, the start
+// encodings one {B, A} int2.
 template <typename T>
 struct Rings {
     typename Vec2<T>::type *D, *xD;
     int2 *P, *xP;
 };
-static_assert(kXchSteps == kBlk, "a block's steps");
 template <typename T>
 __host__ __device__ constexpr int ring_slot_bytes() {
     return (int)(sizeof(typename Vec2<T>::type) + sizeof(int2));
@@ -377,11 +375,13 @@ __device__ __forceinline__ typename Vec2<T>::type make_v2(T x, T y) {
 template <typename T>
 struct Block {
     const typename Vec2<T>::type* Cs;  // the strip's cost, at this lane
-    uint32_t w, r, wD, rD;             // this lane's store and load addresses, P and D
+    uint32_t w, r;                     // this lane's store and load addresses (P; the
+    uint32_t kd;                       // D address is that times 2 (FP32 form: 1), + kd)
     typename Vec2<T>::type* pD;        // PUSH: the ring slot in a cluster peer's
     int2* pP;                          // shared memory, or null
     typename Vec2<T>::type* oD;        // FULL: D and P of every cell at step tau0, this
     int2* oP;                          // lane, in the cost's layout (oD may be the cost)
+    uint32_t incW, incR;               // and their moves per two steps (ring lanes)
     int span, tau0, k, R, W, lane, nP;
 };
 
@@ -443,13 +443,13 @@ __device__ __forceinline__ bool fast_step(Wave<T, QD>& st, const Block<T>& b,
     const typename Vec2<T>::type cc = queue_take<QD, T>(st.q, u, t);
     T x1n, x3n;
     int p1n, p3n;
-    st_pair(b.wD + u * SD, b.w + u * SP, st.bD1, st.aD2, st.bP1, st.aP2);
+    st_pair(d_address<T>(b.w, b.kd) + u * SD, b.w + u * SP, st.bD1, st.aD2, st.bP1, st.aP2);
     if (PUSH && b.pD && lane == 31) {
         b.pD[u] = make_v2<T>(st.bD1, st.aD2);
         b.pP[u] = make_int2(st.bP1, st.aP2);
     }
     __syncwarp();
-    ld_pair(b.rD + u * SD, b.r + u * SP, x1n, x3n, p1n, p3n);
+    ld_pair(d_address<T>(b.r, b.kd) + u * SD, b.r + u * SP, x1n, x3n, p1n, p3n);
     T m0A = addr(rc, -fabs((T)st.x1P));
     T m2A = addr(rc, -fabs((T)st.x3P));
     T m0B = addr(rc, -fabs((T)st.aP2));
@@ -572,16 +572,15 @@ __device__ __forceinline__ int fast_steps(Wave<T, QD>& st, Block<T>& b, const Ti
             return t;
         queue_next<QD, T>(st.q, 0, t, cp, !rimmed || t < ahead);
         rc = addr(rc, (T)1);
+        __syncwarp();  // (exchange.cuh)
         if (!fast_step<KIND, PUSH, FULL, T, QD>(st, b, td, 1, t + 1, rc, w0, w1, w2, eD, eP, bitsA,
                                                 bitsB))
             return t + 1;
         queue_next<QD, T>(st.q, 1, t + 1, cp + 32, !rimmed || t + 1 < ahead);
         rc = addr(rc, (T)1);
         cp += 64;
-        b.w += 2 * sizeof(int2);
-        b.r += 2 * sizeof(int2);
-        b.wD += 4 * sizeof(T);
-        b.rD += 4 * sizeof(T);
+        b.w += b.incW;
+        b.r += b.incR;
         if (PUSH && b.pD) {
             b.pD += 2;
             b.pP += 2;
@@ -608,13 +607,13 @@ __device__ __forceinline__ void careful_step(const Geo& g, Wave<T, QD>& st, cons
     const int cA = b.tau0 + t - 2 * lane, cB = cA - 1;
     T x1n, x3n;
     int p1n, p3n;
-    st_pair(b.wD + u * SD, b.w + u * SP, st.bD1, st.aD2, st.bP1, st.aP2);
+    st_pair(d_address<T>(b.w, b.kd) + u * SD, b.w + u * SP, st.bD1, st.aD2, st.bP1, st.aP2);
     if (PUSH && b.pD && lane == 31) {
         b.pD[u] = make_v2<T>(st.bD1, st.aD2);
         b.pP[u] = make_int2(st.bP1, st.aP2);
     }
     __syncwarp();
-    ld_pair(b.rD + u * SD, b.r + u * SP, x1n, x3n, p1n, p3n);
+    ld_pair(d_address<T>(b.r, b.kd) + u * SD, b.r + u * SP, x1n, x3n, p1n, p3n);
     T m0A = addr(rc, -fabs((T)st.x1P));
     T m2A = addr(rc, -fabs((T)st.x3P));
     T m0B = addr(rc, -fabs((T)st.aP2));
@@ -683,6 +682,7 @@ __device__ __forceinline__ void careful_steps(const Geo& g, Wave<T, QD>& st, Blo
         }
     }
     if (t & 1) cp += 32;
+    __syncwarp();  // (the step that left the fast loop stores its pair again)
 #pragma unroll 1
     for (; t < kBlk; ++t) {
         const V2 cc = queue_take<QD, T>(st.q, 0, t);
@@ -692,13 +692,12 @@ __device__ __forceinline__ void careful_steps(const Geo& g, Wave<T, QD>& st, Blo
         careful_step<STD, PUSH, FULL, T, QD>(g, st, b, td, t & 1, t, rim, mask, rc, cc, bitsA,
                                              bitsB);
         if constexpr (QD > 0) queue_next<QD, T>(st.q, 1, t, cp, t < ahead);
+        __syncwarp();  // (exchange.cuh)
         cp += 32;
         rc = addr(rc, (T)1);
         if (t & 1) {
-            b.w += 2 * sizeof(int2);
-            b.r += 2 * sizeof(int2);
-            b.wD += 4 * sizeof(T);
-            b.rD += 4 * sizeof(T);
+            b.w += b.incW;
+            b.r += b.incR;
             if (PUSH && b.pD) {
                 b.pD += 2;
                 b.pP += 2;
@@ -795,10 +794,10 @@ __device__ __forceinline__ void zero_wave(Wave<T, QD>& st) {
 __device__ __forceinline__ int ring_start(int off, int RB) { return (RB - off % RB) % RB; }
 __device__ __forceinline__ int ring_next(int s, int RB) { return s + kBlk == RB ? 0 : s + kBlk; }
 
-// Lane addresses of a block's first step: exchange entries, but lane 31 stores
-// into the ring slot `wslot` (< 0: nobody reads the strip, its entry instead;
-// then a ring another strip still reads is not overwritten) and lane 0 loads
-// slot `rslot` (< 0: strip 0, which has no producer; its own entry).
+// Lane addresses of a block: exchange entries, but lane 31 stores into the
+// ring slot `wslot` (< 0: nobody reads the strip, its entry instead; then a
+// ring another strip still reads is not overwritten) and lane 0 loads slot
+// `rslot` (< 0: strip 0, which has no producer).
 template <typename T>
 __device__ __forceinline__ void lane_addresses(Block<T>& b, const Rings<T>& rg, int warp,
                                                int wslot, int rslot) {
@@ -807,10 +806,10 @@ __device__ __forceinline__ void lane_addresses(Block<T>& b, const Rings<T>& rg, 
     const int y = warp * kXch + exchange_load(b.lane, 0);
     b.w = (uint32_t)__cvta_generic_to_shared(w ? rg.P + wslot : rg.xP + x);
     b.r = (uint32_t)__cvta_generic_to_shared(r ? rg.P + rslot : rg.xP + y);
-    const uint32_t kd = (uint32_t)__cvta_generic_to_shared(rg.D) -
-                        d_address<T>((uint32_t)__cvta_generic_to_shared(rg.P), 0u);
-    b.wD = d_address<T>(b.w, kd);
-    b.rD = d_address<T>(b.r, kd);
+    b.kd = (uint32_t)__cvta_generic_to_shared(rg.D) -
+           d_address<T>((uint32_t)__cvta_generic_to_shared(rg.P), 0u);
+    b.incW = w ? 2 * (int)sizeof(int2) : 0;
+    b.incR = r ? 2 * (int)sizeof(int2) : 0;
 }
 
 // Bounded wait until progress word *p reaches target; gives up early when
@@ -842,7 +841,7 @@ inline int ring_len(int lag, int nw, int smem_limit, int vbytes, int queue) {
 }
 // Shared memory of a CTA of nw warps for tiles of up to L x L whose strips
 // are `lag` steps apart.  qd is the depth asked for; 0 is taken instead where
-// the queue would leave the rings less than 48 slots of slack.
+// the queue would leave the rings less than 64 slots of slack.
 struct S1Mem {
     int rb, qd;    // ring slots (0: does not fit), queue depth
     size_t bytes;
@@ -852,7 +851,7 @@ inline S1Mem stage1_mem(int lag, int nw, int smem_limit, int vbytes, int qd) {
     S1Mem m{0, 0, 0, 0};
     const int queue = nw * qd * 32 * 2 * vbytes;
     int rb = qd ? ring_len(lag, nw, smem_limit, vbytes, queue) : 0;
-    m.qd = rb >= lag + 48 ? qd : 0;
+    m.qd = rb >= lag + 64 ? qd : 0;
     m.rb = m.qd ? rb : ring_len(lag, nw, smem_limit, vbytes, 0);
     if (m.rb == 0) return m;
     const size_t ring = vbytes == 8 ? ring_bytes<double>(nw, m.rb, nw + 2)
@@ -876,10 +875,9 @@ inline int smem_per_sm() {
     return v;
 }
 
-// Shared memory budget per CTA when 16/NW CTAs share an SM, each with 1024 bytes
-// that the driver reserves and up to 256 of static shared memory.
+// Shared memory budget per CTA when 16/NW CTAs share an SM.
 inline int cta_budget(int nw) {
-    const int per_cta = smem_per_sm() / (16 / nw) - 1024 - 256;
+    const int per_cta = smem_per_sm() / (16 / nw) - 2048;  // static smem and reserve
     const int optin = smem_optin();
     return per_cta < optin ? per_cta : optin;
 }
