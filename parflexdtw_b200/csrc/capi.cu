@@ -239,6 +239,10 @@ int pfx::plan_init(pfx_plan* p, int64_t N, int64_t M, int32_t L, const int64_t* 
     // backpointer words stage 1 never writes (past a tile's rows or steps)
     // read as 0, so that two plans' arrays compare equal
     CK(cudaMemset(p->s1.Bw, 0, (size_t)nt * g.b_words * sizeof(uint32_t)));
+    // (the fills are on the default stream; nothing else orders them before
+    // the plan's first work on another one, which counts on diag_count and status
+    // and writes Bw)
+    CK(cudaStreamSynchronize(nullptr));
     return PFX_OK;
 }
 
@@ -446,6 +450,7 @@ static int ensure_cost_buffer(pfx_plan* p) {
     std::vector<TileDesc> d((size_t)p->g.n1 * p->g.n2);
     plan_tile_descs(p, p->Csk, d.data());
     CK(cudaMemcpy(p->descs, d.data(), d.size() * sizeof(TileDesc), cudaMemcpyHostToDevice));
+    CK(cudaStreamSynchronize(nullptr));  // (a copy from pageable memory returns before it arrives)
     return PFX_OK;
 }
 
