@@ -2,12 +2,13 @@
 // tensor cores, written straight into the FP32 tile-skewed slabs that the
 // FP32 stage-1 kernel reads.
 //
-// One CTA (4 warps) produces the skewed rows tau in [128 cb, 128 cb + 128) of
-// the two 64-row strips 2 kk, 2 kk + 1 of one tile.  Those rows hold the cells
+// A block is the skewed rows tau in [128 cb, 128 cb + 128) of the two 64-row
+// strips 2 kk, 2 kk + 1 of one tile; one CTA of 16 warps per SM takes blocks in
+// turn (roles: see k_gemm_cost_skew).  Those rows hold the cells
 // (rho, tau - rho), rho < 64, i.e. rows 128 kk + [0, 128) and columns
 // 128 cb - 64 + [1, 192) of the tile: a 128 x 192 block of C (the 64 extra
-// columns overlap the neighbouring CTA; tensor-core work is cheap next to
-// the slab write, which bounds this kernel).
+// columns overlap the neighbouring block; tensor-core work is cheap next to
+// the slab write and the operands' way from L2).
 //
 //   TMA (SWIZZLE_128B, K-major boxes of 64 bf16 x rows; rows outside the
 //   sequences, e.g. the negative column offset of the first block, arrive as
@@ -15,8 +16,8 @@
 //   FP32 accumulate, M = 128, N = 192, K = 16 per instruction) into a TMEM
 //   accumulator of 192 columns -> tcgen05.ld (32 lanes x 32 columns per warp
 //   and step) -> 1 - acc, masked to 0 outside the tile -> shared memory in
-//   skewed order (address 65 rho + const: conflict-free) -> 256-byte rows of
-//   float2 per warp to global (streaming stores).
+//   skewed order (address 65 rho + const: conflict-free) -> global, each strip's
+//   rows of 256 bytes with one cp.async.bulk copy.
 //
 // Every wait is bounded: a wait that runs out sets the status word, waits
 // (bounded) for the CTA's own copies or MMAs still in flight, frees its TMEM
@@ -593,9 +594,10 @@ __global__ void __launch_bounds__(kGThreads, 1)
 // takes 32 frames into shared memory (rows of 256 bytes, all loads in flight
 // at once): one thread per frame sums its squares (fixed order), then all
 // threads produce the block's rows -- contiguous in `out` -- one word (two bf16)
-// per thread and step. Bound by the read of F. 64 pairs of 1000 to 8000 frames,
-// 128 features (0.56 GB): 0.44 -> 0.27 ms against reading F twice, the second
-// time across its rows.
+// per thread and step. A block's phases follow one another (its loads, the sums
+// of squares on one warp, the rows), which bounds it: 64 pairs of 1000 to 8000
+// frames, 128 features (0.56 GB read, 0.16 GB written) 0.27 ms, 41 % of HBM; 0.44
+// with F read twice, the second time across its rows.
 constexpr int kFbFrames = 32;
 constexpr int kFbStride = kFbFrames + 1;
 constexpr int kFbThreads = 256;

@@ -16,7 +16,7 @@ constexpr int kSpinLimit = 1 << 22;
 
 // Pulls the cost of a strip's next block of steps (kBlk steps x 32 lanes,
 // contiguous in the skewed slab) into L2 with one bulk prefetch, so that the
-// DP's own loads, two steps ahead, hit L2 instead of HBM.  Issued by one lane;
+// DP's own loads, two to four steps ahead, hit L2 instead of HBM.  Issued by one lane;
 // the range must lie inside the strip (the caller checks).
 template <typename V2>
 __device__ __forceinline__ void prefetch_next_block(const V2* strip, int tau_next) {
@@ -307,12 +307,12 @@ struct Wave {
 // next step uses as x1 and x3.  Lanes 0..30 store into their exchange entry
 // (exchange.cuh: one barrier of the warp per step, and another after even
 // ones); lane 31 stores into ring slot (T - 64) mod RB, which then holds rows
-// 64k+63 and 64k+62 of column j = tau - 64; lane 0 loads ring slot (T' - lag) mod RB
-// of the previous strip, its column tau'.  So one address per lane takes the
+// 64k+63 and 64k+62 of column j = tau - 64; lane 0 loads ring slot (T' - lag) mod
+// RB of the previous strip, its column tau'.  So one address per lane takes the
 // place of shuffles, of the ring's own loads and stores and of the selects
-// between the two.  Both ring windows of a block start on a multiple of
-// kBlk: no address inside a block wraps.  D is one {B, A} vector, the start
-// encodings one {B, A} int2.
+// between the two.  Both ring windows of a block start on a multiple of kBlk: no
+// address inside a block wraps.  D is one {B, A} vector, the start encodings one
+// {B, A} int2.
 template <typename T>
 struct Rings {
     typename Vec2<T>::type *D, *xD;
@@ -426,7 +426,7 @@ __device__ __forceinline__ uint32_t d_address(uint32_t p, uint32_t kd) {
 enum StripKind { kInner, kTop, kBottom, kRim, kCorner };
 
 // One step of the fast loop: standard steps, every cell of the strip's rows
-// inside the tile has c >= 18 and is off the last column.  Returns false, with
+// inside the tile has c >= 17 and is off the last column.  Returns false, with
 // the wave unchanged, when some lane's cell needs the exact routine.  u: the
 // step's parity.  kTop: strip 0 of several (row 0 is the cost itself, rows 1
 // and 2 have predecessors on it); kBottom: the last strip of several, whose
@@ -713,7 +713,7 @@ constexpr int kCornerWidth = 800;  // see run_block
 // The fast loop (standard steps) has no divisions and one branch per step, out
 // of the loop when some cell is too close to call. It has a copy for each kind
 // of block: inner ones, every cell of which has all its predecessors in the
-// tile and off its rim (columns from 18 to the last but one), need no tests at
+// tile and off its rim (columns from 17 to the last but one), need no tests at
 // all; strip 0 and the last strip a few, because the strips after strip 0
 // follow at its pace and a tile ends with its last strip; blocks at the tile's
 // first and last columns selects around the selection, because a strip starts
